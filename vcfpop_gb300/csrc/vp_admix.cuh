@@ -1,0 +1,316 @@
+// Per-copy label draws of the admixture model on 2-bit biallelic diploid data
+// (UpdateZAdmix, src/structure.cpp:1350-1487) with counter streams.
+#pragma once
+#include "vp_kernels.cuh"
+
+namespace vp {
+
+// ---------------------------------------------------------------------------
+// Genotypes by slice: word [s][i] holds individual i's 2-bit codes at the
+// PZ_LC loci of slice s (locus 16 s + j at bits 2j, 2j + 1; 3 past the last
+// locus and past the last individual), so that a lane that walks the loci of
+// one individual reads 16 calls with one coalesced load. Built once per
+// context, for chains that draw labels per copy.
+constexpr int PZ_LC = 16;
+static_assert(PZ_LC == ZA_LC, "the Philox streams are per slice of ZA_LC loci");
+__global__ void __launch_bounds__(256) k_build_slices(const DevData D, uint32_t* gt, int Npad) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= Npad) return;
+    const int w = i >> 4, sh = (i & 15) * 2;
+    for (int64_t s = blockIdx.y; s * PZ_LC < D.L; s += gridDim.y) {
+        uint32_t v = 0;
+#pragma unroll
+        for (int j = 0; j < PZ_LC; ++j) {
+            const int64_t l = s * PZ_LC + j;
+            const uint32_t c = l < D.L && i < D.N ? (__ldg(D.g2 + l * D.Nw + w) >> sh) & 3u : 3u;
+            v |= c << (2 * j);
+        }
+        gt[s * Npad + i] = v;
+    }
+}
+
+// two FP32 values in one 64-bit register pair, and the packed operations on
+// them (each half rounds as the scalar instruction does)
+typedef unsigned long long f2x;
+__device__ __forceinline__ f2x f2_pack(float a, float b) {
+    f2x r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f2_unpack(f2x v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f2x f2_fma(f2x a, f2x b, f2x c) {
+    f2x r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f2x f2_mul(f2x a, f2x b) {
+    f2x r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2x f2_add(f2x a, f2x b) {
+    f2x r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// transpose of a 32 x 32 bit matrix held as one word a lane: bit p of lane n
+// becomes bit n of lane p
+struct BitTranspose {
+    uint32_t s16, s8, k4, k2, k1;   // byte selectors of the two outer steps, kept bits of the inner ones
+    int r4, r2, r1;                 // left rotations of the partner's word
+    __device__ __forceinline__ explicit BitTranspose(int lane) {
+        s16 = lane & 16 ? 0x3276u : 0x5410u;
+        s8 = lane & 8 ? 0x3715u : 0x6240u;
+        k4 = lane & 4 ? 0xF0F0F0F0u : 0x0F0F0F0Fu;
+        k2 = lane & 2 ? 0xCCCCCCCCu : 0x33333333u;
+        k1 = lane & 1 ? 0xAAAAAAAAu : 0x55555555u;
+        r4 = lane & 4 ? 28 : 4;
+        r2 = lane & 2 ? 30 : 2;
+        r1 = lane & 1 ? 31 : 1;
+    }
+    __device__ __forceinline__ uint32_t operator()(uint32_t x) const {
+        x = __byte_perm(x, __shfl_xor_sync(0xffffffffu, x, 16), s16);
+        x = __byte_perm(x, __shfl_xor_sync(0xffffffffu, x, 8), s8);
+        uint32_t y = __shfl_xor_sync(0xffffffffu, x, 4);
+        x = (x & k4) | (__funnelshift_l(y, y, r4) & ~k4);
+        y = __shfl_xor_sync(0xffffffffu, x, 2);
+        x = (x & k2) | (__funnelshift_l(y, y, r2) & ~k2);
+        y = __shfl_xor_sync(0xffffffffu, x, 1);
+        return (x & k1) | (__funnelshift_l(y, y, r1) & ~k1);
+    }
+};
+
+// the words with label k among the bit planes p[0..3] of 32 labels
+template <int KM>
+__device__ __forceinline__ uint32_t label_mask(const uint32_t* p, int k) {
+    uint32_t m = k & 1 ? p[0] : ~p[0];
+    if (KM > 2) m &= k & 2 ? p[1] : ~p[1];
+    if (KM > 4) m &= k & 4 ? p[2] : ~p[2];
+    if (KM > 8) m &= k & 8 ? p[3] : ~p[3];
+    return m;
+}
+
+// 16-byte chunks (two clusters' frequency pairs) of a table row, an odd count:
+// the four codes' rows of a locus then start in different banks
+template <int KM>
+__host__ __device__ constexpr int pz_chunks() { return ((KM + 1) / 2) | 1; }
+
+// Label draws of every copy, one lane per individual, a warp of 32
+// individuals walking the slices of the CTA's locus range (grid.y).
+//
+// The same draws as k_update_z_admix_ctr, bit for bit: one Philox stream per
+// (individual, slice), two draws per locus, prefix sums of q_k p_k by fused
+// multiply-adds in cluster order, and the first cluster whose cumulative
+// weight exceeds the uniform times the total. The prefix sums do not
+// decrease, so that cluster is the number of clusters (but the last) whose
+// threshold the uniform reaches.
+//
+// What bounds it is instruction issue, so the work per copy is cut down to
+// the draw itself:
+//  - the staged table holds, for each code of a locus, the pair (frequency of
+//    the first copy's allele, of the second's) of every cluster, so that one
+//    16-byte load brings two clusters of both copies and packed FP32
+//    instructions serve both copies at once;
+//  - labels go four bits each into a word (eight copies), the words become
+//    bit planes of a slice's 32 copies, and a lane's copies per cluster are
+//    one population count a cluster and slice;
+//  - for the counts per locus the planes are transposed across the warp (bit
+//    n = lane n), lane p then holds one copy slot of one locus for the 32
+//    individuals, and copies of an allele with label k are one population
+//    count against the genotype words' own bit planes (lane n is individual
+//    n / 2 of the first genotype word or of the second, by n's last bit, so
+//    that the planes interleave as the words do).
+// Counts of both alleles share a word of the CTA's histogram (16 bits each: a
+// CTA adds at most 2 x 256 per slice), which goes to Ni as 64-bit additions of
+// the two neighbouring counts. One barrier a slice: table and histogram are
+// double-buffered.
+//
+// Measured (one GB300, launch): see the dispatch in launch_zadm_ctr.
+constexpr int PZ_MAXK = 16;
+constexpr int PZ_MAXT = 256;
+template <int KM, bool EXACT>
+__global__ void __launch_bounds__(PZ_MAXT, KM <= 6 ? 3 : 2) k_z_admix_pk(const DevChain* chains, int force,
+                                                                        const int4* map = nullptr) {
+    constexpr int CH = pz_chunks<KM>();
+    constexpr int NPL = KM <= 2 ? 1 : KM <= 4 ? 2 : KM <= 8 ? 3 : 4;      // bit planes of a label
+    constexpr int NF = (PZ_LC * KM + 127) / 128;                          // staged frequencies a thread (128 threads or more)
+    __shared__ __align__(16) float2 sF[2][PZ_LC][4][CH * 2];
+    __shared__ uint32_t hs[2][KM][PZ_LC];
+    __shared__ double sh[32];
+    const VBlock vb = vblock(map);
+    const DevChain& c = chains[vb.z];
+    if (map && run_over(c)) return;
+    const DevData& D = c.D;
+    const int K = EXACT ? KM : c.K, m = c.ctl->m;
+    if (!force && binaryq_at(c, m)) return;
+    const int lane = threadIdx.x & 31, T = blockDim.x;
+    const int ib = vb.x * T + (threadIdx.x & ~31);
+    const int i = ib + (lane >> 1) + 16 * (lane & 1);
+    const bool live = i < D.N;
+    const uint32_t lives = __ballot_sync(0xffffffffu, live);
+    const int nsl = (int)((D.L + PZ_LC - 1) / PZ_LC);
+    const int s0 = vb.y * c.pz_slices, s1 = min(nsl, s0 + c.pz_slices);
+    const int Npad = (D.N + 31) & ~31;
+    f2x q[KM];
+    int32_t mi[KM];
+#pragma unroll
+    for (int k = 0; k < KM; ++k) {
+        const float v = (live && (EXACT || k < K)) ? c.Q[(int64_t)i * K + k] : 0.f;
+        q[k] = f2_pack(v, v);
+        mi[k] = 0;
+    }
+    // this lane's copy slot after the transpose: copy j of the group of four
+    // loci g sits in nibble 7 - j of the group's word and at bit 3 - g of the
+    // nibble once the four groups' planes are merged
+    const int slot = 7 - (lane >> 2), pl = 4 * (3 - (lane & 3)) + (slot >> 1);
+    const bool second = slot & 1;
+    const BitTranspose tr(lane);
+    const bool rec = force || record_at(c, m);
+    float ls = 0.f, lc = 0.f;                       // Kahan sum of ln(sum_k q_k p)
+    const float minf = (float)VP_MIN_FREQ;
+    const f2x kmin = f2_pack((float)(VP_MIN_FREQ * K), (float)(VP_MIN_FREQ * K));
+    const uint2 key = make_uint2((uint32_t)c.seed, (uint32_t)(c.seed >> 32));
+    const uint32_t ca = ST_ZSLICE | ((uint32_t)m << 4);
+    const float2* F2 = reinterpret_cast<const float2*>(c.Freq);
+    float2 fn[NF];
+    auto load_f = [&](int s) {
+#pragma unroll
+        for (int u = 0; u < NF; ++u) {
+            const int j = threadIdx.x + u * T, k = j >> 4;
+            const int64_t l = (int64_t)s * PZ_LC + (j & 15);
+            fn[u] = j < PZ_LC * K && l < D.L ? __ldg(F2 + (int64_t)k * D.L + l) : make_float2(0.f, 0.f);
+        }
+    };
+    auto store_f = [&](int buf) {
+#pragma unroll
+        for (int u = 0; u < NF; ++u) {
+            const int j = threadIdx.x + u * T;
+            if (j < PZ_LC * KM) {
+                float2(*r)[CH * 2] = sF[buf][j & 15];
+                const int k = j >> 4;
+                r[0][k] = make_float2(fn[u].x, fn[u].x);
+                r[1][k] = fn[u];
+                r[2][k] = make_float2(fn[u].y, fn[u].y);
+            }
+        }
+    };
+    if (s0 >= s1) return;
+    for (int j = threadIdx.x; j < 2 * PZ_LC * CH * 2; j += T)
+        sF[j / (PZ_LC * CH * 2)][j / (CH * 2) % PZ_LC][3][j % (CH * 2)] = make_float2(0.f, 0.f);
+    for (int j = threadIdx.x; j < 2 * KM * PZ_LC; j += T) (&hs[0][0][0])[j] = 0;
+    load_f(s0);
+    store_f(0);
+    uint32_t gn = ib < Npad ? __ldg(D.gt + (int64_t)s0 * Npad + i) : 0xFFFFFFFFu;
+    __syncthreads();
+    int buf = 0;
+    for (int s = s0; s < s1; ++s, buf ^= 1) {
+        uint32_t gw = gn;
+        // this lane's locus for the counts: its two genotype words
+        uint32_t w0 = 0xFFFFFFFFu, w1 = 0xFFFFFFFFu;
+        {
+            const int64_t l = (int64_t)s * PZ_LC + pl;
+            const int w = ib >> 4;
+            if (l < D.L) {
+                if (w < D.Nw) w0 = __ldg(D.g2 + l * D.Nw + w);
+                if (w + 1 < D.Nw) w1 = __ldg(D.g2 + l * D.Nw + w + 1);
+            }
+        }
+        if (s + 1 < s1) {
+            if (ib < Npad) gn = __ldg(D.gt + (int64_t)(s + 1) * Npad + i);
+            load_f(s + 1);
+        }
+        uint32_t P[NPL];
+#pragma unroll
+        for (int b = 0; b < NPL; ++b) P[b] = 0;
+#pragma unroll 1
+        for (int g = 0; g < 4; ++g) {
+            uint32_t Z = 0;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint4 rb = Philox::round10(make_uint4(ca, (uint32_t)s, (uint32_t)i, (uint32_t)(2 * g + h)), key);
+#pragma unroll
+                for (int v = 0; v < 2; ++v) {
+                    const uint32_t code = gw & 3u;
+                    gw >>= 2;
+                    const float4* row = reinterpret_cast<const float4*>(&sF[buf][4 * g + 2 * h + v][code][0]);
+                    f2x pre[KM], sx = 0;
+#pragma unroll
+                    for (int k = 0; k < KM; k += 2) {
+                        const float4 f = row[k >> 1];
+                        sx = f2_fma(q[k], f2_pack(f.x, f.y), sx);
+                        pre[k] = sx;
+                        if (k + 1 < KM) {
+                            sx = f2_fma(q[k + 1], f2_pack(f.z, f.w), sx);
+                            pre[k + 1] = sx;
+                        }
+                    }
+                    // uniforms ((x >> 8) + 1) / 2^24: every step exact
+                    const float ua = fmaf((float)((v ? rb.z : rb.x) >> 8), 1.f / 16777216.f, 1.f / 16777216.f);
+                    const float ub = fmaf((float)((v ? rb.w : rb.y) >> 8), 1.f / 16777216.f, 1.f / 16777216.f);
+                    float ta, tb;
+                    f2_unpack(f2_mul(f2_pack(ua, ub), f2_add(sx, kmin)), ta, tb);
+                    uint32_t za = 0, zb = 0;
+#pragma unroll
+                    for (int k = 0; k < KM - 1; ++k) {
+                        if (!EXACT && k >= K - 1) break;
+                        float pa, pb;
+                        f2_unpack(pre[k], pa, pb);
+                        if (!(ta < __fmaf_rn((float)(k + 1), minf, pa))) ++za;
+                        if (!(tb < __fmaf_rn((float)(k + 1), minf, pb))) ++zb;
+                    }
+                    Z = (((Z << 4) | za) << 4) | zb;
+                    if (rec && code != 3u) {
+                        float xa, xb;
+                        f2_unpack(sx, xa, xb);
+                        const float y = (logf(xa) + logf(xb)) - lc, t = ls + y;
+                        lc = (t - ls) - y;
+                        ls = t;
+                    }
+                }
+            }
+#pragma unroll
+            for (int b = 0; b < NPL; ++b) P[b] = (P[b] << 1) | ((Z >> b) & 0x11111111u);
+        }
+        // the genotype words' planes, bit n = lane n's individual
+        const uint32_t LO = (w0 & 0x55555555u) | ((w1 << 1) & 0xAAAAAAAAu);
+        const uint32_t HI = ((w0 >> 1) & 0x55555555u) | (w1 & 0xAAAAAAAAu);
+        const uint32_t MS = (LO & HI) | ~lives;
+        const uint32_t A1 = (second ? LO ^ HI : HI & ~LO) & ~MS, A0 = ~(A1 | MS);
+        const uint32_t typed = ~tr(MS);                  // this lane's typed copies
+#pragma unroll
+        for (int k = 0; k < KM; ++k)
+            if (EXACT || k < K) mi[k] += __popc(label_mask<KM>(P, k) & typed);
+        uint32_t R[NPL];
+#pragma unroll
+        for (int b = 0; b < NPL; ++b) R[b] = tr(P[b]);
+#pragma unroll
+        for (int k = 0; k < KM; ++k) {
+            if (!EXACT && k >= K) break;
+            const uint32_t mk = label_mask<KM>(R, k);
+            const uint32_t n = (uint32_t)__popc(mk & A0) | ((uint32_t)__popc(mk & A1) << 16);
+            atomicAdd(&hs[buf][k][pl], n);
+        }
+        if (s + 1 < s1) store_f(buf ^ 1);
+        __syncthreads();
+        unsigned long long* N2 = reinterpret_cast<unsigned long long*>(c.Ni);
+        for (int j = threadIdx.x; j < PZ_LC * K; j += T) {
+            uint32_t* h = &hs[buf][j >> 4][j & 15];
+            const uint32_t n = *h;
+            if (!n) continue;
+            *h = 0;
+            atomicAdd(N2 + (int64_t)(j >> 4) * D.L + (int64_t)s * PZ_LC + (j & 15),
+                      (unsigned long long)(n & 0xFFFFu) | ((unsigned long long)(n >> 16) << 32));
+        }
+    }
+    if (live)
+#pragma unroll
+        for (int k = 0; k < KM; ++k)
+            if ((EXACT || k < K) && mi[k]) atomicAdd(&c.Mi[(int64_t)i * K + k], mi[k]);
+    const double t = block_sum((double)ls - (double)lc, sh);
+    if (threadIdx.x == 0) c.lnlp[vb.y * vb.gx + vb.x] = t;
+}
+
+}  // namespace vp

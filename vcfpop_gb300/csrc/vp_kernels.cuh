@@ -19,6 +19,7 @@ struct DevData {
     int32_t popcontig;    // every population's individuals are consecutive
     int64_t L, KT, coprime;
     const uint32_t* g2;   // [L][Nw]
+    const uint32_t* gt;   // the same calls by slice of 16 loci and individual (k_build_slices), or null
     const uint8_t* gb;    // [L][N][vmax]
     const int32_t* k;
     const int64_t* off;
@@ -41,7 +42,7 @@ struct DevChain {
     DevData D;
     int32_t K, admix, locpriori, fmodel, nburnin, nreps, nthinning, nadmburnin, writelnl;
     int32_t metrofreq, inferalpha, diffalpha, uniformalpha, fsame, difflambda, rlen, rng, nchunk, lchunk;
-    int32_t zadm_tn, nlnlp, kp, nsampblk, zadm_lc;
+    int32_t pz_slices, nlnlp, kp, nsampblk, zadm_lc;
     int32_t ntrace;       // capacity of lnlTrace in records
     double lambda, alpha, stdalpha, maxalpha, alphapriora, alphapriorb, maxr, epsr, epseta, epsgamma;
     double pmeanf, pstdf, stdf;

@@ -9,6 +9,7 @@
 
 #include "vp_internal.h"
 #include "vp_kernels.cuh"
+#include "vp_admix.cuh"
 #include "vp_tc.cuh"
 
 using namespace vp;
@@ -368,8 +369,28 @@ size_t zadm_smem(const vp_chain* c) {
 #define VP_ZADM_EXACT(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12)
 #define VP_ZADM_PADDED(X) X(16) X(32) X(64)
 
+// chains whose per-copy draws run on the sliced 2-bit genotypes (k_z_admix_pk)
+bool pz_form(bool packed2, const vp_params& P) {
+    return packed2 && P.rng == VP_RNG_COUNTER && P.K <= PZ_MAXK;
+}
+// individuals per CTA of k_z_admix_pk: 256 share a staged table when that
+// leaves few idle lanes, 128 on small samples
+int pz_threads(int32_t N) { return N <= 1024 ? 128 : PZ_MAXT; }
+
 int launch_zadm_ctr(vp_chain* c, int force) {
     vp_ctx* x = c->ctx;
+    if (pz_form(x->packed2, c->P)) {
+        const int T = pz_threads(x->N), K = c->P.K;
+        const dim3 g(cdiv(x->N, T), cdiv(cdiv(x->L, PZ_LC), c->h.pz_slices), 1);
+        prof_mark(x, true);
+        struct End { vp_ctx* x; ~End() { prof_mark(x, false); } } end_{x};
+#define VP_ZE(n) \
+    if (K == n) { SL(c, (k_z_admix_pk<n, true>), (g), (T), 0, 1, force); return VP_OK; }
+        VP_ZADM_EXACT(VP_ZE)
+#undef VP_ZE
+        SL(c, (k_z_admix_pk<PZ_MAXK, false>), (g), (T), 0, 1, force);
+        return VP_OK;
+    }
     dim3 g(cdiv(x->N, ZA_WARPS * 32), cdiv(x->L, c->h.zadm_lc), 1);
     size_t sm = zadm_smem(c);
     prof_mark(x, true);
@@ -779,6 +800,15 @@ int chain_plan(const vp_ctx* x, const vp_params* P, vp_chain* c, size_t* bytes) 
     }
     h.nlnlp = (int32_t)std::max<int64_t>(std::max<int64_t>(cdiv(L, 128), (int64_t)cdiv(N, ZA_WARPS * 32) * cdiv(L, h.zadm_lc)),
                                          std::max<int64_t>(h.nsampblk, cdiv(N, tc::TS_TILE)));
+    {
+        // slices per CTA of the sliced label kernel: about 64 CTAs' worth of
+        // 128 threads per SM, as above
+        const int T = pz_threads(N);
+        const int64_t nsl = cdiv(L, PZ_LC), nx = cdiv(N, T), want = (int64_t)x->nsm * 64 * 128 / T;
+        h.pz_slices = (int32_t)std::max<int64_t>(1, cdiv(nsl * nx, want));
+        if (pz_form(x->packed2, *P))
+            h.nlnlp = (int32_t)std::max<int64_t>(h.nlnlp, nx * cdiv(nsl, h.pz_slices));
+    }
     c->plain_lazy = tc_batchable(x, P, h);
     Carve probe{nullptr};
     chain_layout(probe, c, x);
@@ -786,6 +816,29 @@ int chain_plan(const vp_ctx* x, const vp_params* P, vp_chain* c, size_t* bytes) 
     return VP_OK;
 }
 }  // namespace
+
+// chains that draw a label per allele copy: admixture, or its burn-in
+static bool per_copy(const DevChain& h) { return h.admix || h.nadmburnin > 0; }
+static size_t slices_bytes(const vp_ctx* x) {
+    return (size_t)cdiv(x->L, PZ_LC) * ((x->N + 31) & ~31) * sizeof(uint32_t);
+}
+// the context's genotypes by slice, built on the first chain that needs them
+static int ensure_slices(vp_ctx* x) {
+    if (x->D.gt) return VP_OK;
+    void* p = nullptr;
+    const cudaError_t e = dev_alloc(&p, slices_bytes(x), x->device, x->stream);
+    if (e != cudaSuccess) {
+        vp_set_error("device allocation of %zu bytes for the sliced genotypes failed: %s", slices_bytes(x), cudaGetErrorString(e));
+        return VP_E_MEM;
+    }
+    x->allocs.push_back(p);
+    const int Npad = (x->N + 31) & ~31;
+    k_build_slices<<<dim3(cdiv(Npad, 256), (unsigned)std::min<int64_t>(cdiv(x->L, PZ_LC), 32768), 1), 256, 0, x->stream>>>(
+        x->D, (uint32_t*)p, Npad);
+    if (int rc = check_launch(x, "k_build_slices")) return rc;
+    x->D.gt = (const uint32_t*)p;
+    return VP_OK;
+}
 
 int64_t vp_request_bytes(const vp_dataset* ds, const vp_params* P, int nsm) {
     vp_ctx g;
@@ -800,6 +853,7 @@ int64_t vp_request_bytes(const vp_dataset* ds, const vp_params* P, int nsm) {
     data += r(ds->k.size() * 4) + r(ds->off.size() * 8) + r(ds->vt.size() * 8) + r(ds->popid.size() * 4) +
             r(ds->pop_ind0.size() * 4) + r(ds->pop_nind.size() * 4) + r(ds->totfreq.size() * 4) +
             r(ds->nhaplo.size() * 4) + (ds->perm.empty() ? 0 : r(ds->perm.size() * 4));
+    if (per_copy(c.h) && pz_form(ds->packed2, *P)) data += r(slices_bytes(&g));
     return data + (int64_t)chain;
 }
 
@@ -815,6 +869,10 @@ extern "C" int vp_chain_create(vp_ctx* x, const vp_params* P, vp_chain** out) {
     const int K = P->K, N = x->N;
     const int64_t L = x->L;
     DevChain& h = c->h;
+    if (per_copy(h) && pz_form(x->packed2, *P)) {
+        if ((prc = ensure_slices(x))) { delete c; return prc; }
+        h.D.gt = x->D.gt;
+    }
     cudaError_t e = dev_alloc(&c->mem, bytes, x->device, x->stream);
     if (e != cudaSuccess) {
         vp_set_error("device allocation of %zu bytes for chain state failed: %s", bytes, cudaGetErrorString(e));
