@@ -51,3 +51,44 @@ def test_admixture_burn_in():
     d = synth.fmodel(9, 90, 100, 3, 0.1, 0.05)
     kw = dict(admix=0, nadmburnin=3)
     _same(_run(d, True, 3, 3, **kw), _run(d, False, 3, 3, **kw))
+
+
+def _philox(c, key):
+    """Philox-4x32-10 of uint32 counters c [4, n] (Salmon et al., SC'11)."""
+    c = [x.astype(np.uint64) for x in c]
+    k = [int(key) & 0xFFFFFFFF, int(key) >> 32]
+    m = np.uint64(0xFFFFFFFF)
+    for _ in range(10):
+        p0, p1 = c[0] * np.uint64(0xD2511F53), c[2] * np.uint64(0xCD9E8D57)
+        c = [(p1 >> np.uint64(32)) ^ c[1] ^ np.uint64(k[0]), p1 & m, (p0 >> np.uint64(32)) ^ c[3] ^ np.uint64(k[1]), p0 & m]
+        k = [(k[0] + 0x9E3779B9) & 0xFFFFFFFF, (k[1] + 0xBB67AE85) & 0xFFFFFFFF]
+    return np.stack(c)
+
+
+# the initial labels of every copy: one stream per (locus, individual), its
+# draws modulo K, over CTA and slice edges, both layouts and mixed ploidy
+@pytest.mark.parametrize("N,L,K,poly", [(15, 17, 1, 0), (257, 33, 5, 0), (256, 16, 3, 1), (300, 70, 16, 0), (90, 41, 7, 1)])
+def test_initial_labels(N, L, K, poly):
+    rng = np.random.default_rng(N)
+    kw = dict(ploidy=rng.choice([1, 2, 4, 6], N), n_alleles=rng.integers(2, 6, L)) if poly else {}
+    d = synth.fmodel(N, N, L, 3, 0.1, 0.1, admix_alpha=0.5, **kw)
+    ds = S.Dataset.from_synth(d)
+    ctx = S.Context(ds)
+    seed = 1234567890123 + K
+    c = S.Chain(ctx, S.params(K, seed, admix=1))
+    order = ds.order()
+    G, k = d["G"][order], d["k"][order]
+    off = np.concatenate([[0], np.cumsum(k)])
+    ll, ii = (x.reshape(-1) for x in np.meshgrid(np.arange(len(order)), np.arange(N), indexing="ij"))
+    draws = [_philox([np.full(ll.size, 8, np.uint32), ll, ii, np.full(ll.size, b, np.uint32)], seed) for b in range(2)]
+    draws = np.concatenate(draws).reshape(8, len(order), N).astype(np.int64) % K
+    Mi, Ni = np.zeros((N, K), int), np.zeros((K, ds.KT), int)
+    for a in range(G.shape[2]):
+        l, i = np.nonzero(G[:, :, a] >= 0)
+        z = draws[a, l, i]
+        np.add.at(Mi, (i, z), 1)
+        np.add.at(Ni, (z, off[l] + G[l, i, a]), 1)
+    assert np.array_equal(c.get("MI").reshape(N, K), Mi)
+    assert np.array_equal(c.get("NI").reshape(K, -1), Ni)
+    c.close()
+    ctx.close()

@@ -202,29 +202,82 @@ __device__ __forceinline__ void load_copies(const DevData& D, int64_t l, int i, 
     cp.n = n;
 }
 
-// InitAdmix, per-copy form: per locus RNG(seed + l, SALT_INITADM), one draw per
-// typed copy (src/structure.cpp:617-645)
-__global__ void k_init_admix(const DevChain* chains) {
+// InitAdmix, per-copy form (src/structure.cpp:617-645), reference streams: per
+// locus RNG(seed + l, SALT_INITADM), one draw per typed copy in order
+__global__ void k_init_admix_ref(const DevChain* chains) {
     const DevChain& c = chains[blockIdx.z];
     const DevData& D = c.D;
     const int K = c.K;
     int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (l >= D.L) return;
     Rng64 r;
-    if (c.rng == 0) r.init(c.seed + l, VP_SALT_INITADM);
+    r.init(c.seed + l, VP_SALT_INITADM);
     int64_t o = D.off[l];
     for (int i = 0; i < D.N; ++i) {
         Copies cp;
         load_copies(D, l, i, cp);
-        if (!cp.n) continue;
-        Philox ph;
-        if (c.rng) ph.init(c.seed, ST_INITADM, (uint32_t)l, (uint32_t)i);
         for (int a = 0; a < cp.n; ++a) {
-            int k2 = c.rng == 0 ? (int)r.nextn(K) : (int)(ph.next() % (uint32_t)K);
+            int k2 = (int)r.nextn(K);
             atomicAdd(&c.Mi[i * K + k2], 1);
             atomicAdd(&c.Ni[k2 * D.KT + o + cp.a[a]], 1);
         }
     }
+}
+
+// The same with counter streams: one Philox stream per call, so calls are
+// independent. CTA = 256 individuals (one per thread) walking a range of loci
+// in groups of IA_LC: the copies go to a shared histogram of the group's
+// (locus, cluster, allele) bins and to the thread's own shared column of
+// cluster counts, and only non-zero sums reach Ni and Mi. Issue-bound (a
+// Philox block per call). One thread per locus walking every individual, with
+// two global atomics per copy, left most of the chip idle: N = 2,000 x
+// L = 50,000, K = 5 took 4.10 ms, N = 1,500 x L = 8,000 of mixed ploidy, K = 8
+// 5.93 ms; now 0.80 and
+// 0.24 ms.
+constexpr int IA_LC = 16, IA_T = 256;
+__global__ void __launch_bounds__(IA_T) k_init_admix_ctr(const DevChain* chains, int lc) {
+    extern __shared__ int32_t ia_sm[];
+    const DevChain& c = chains[blockIdx.z];
+    const DevData& D = c.D;
+    const int K = c.K, MK = D.maxK, nb = K * MK, t = threadIdx.x;
+    int32_t* hs = ia_sm;                      // [IA_LC][K][MK]
+    int32_t* ms = ia_sm + IA_LC * nb;         // [K][IA_T]
+    const int i = blockIdx.x * IA_T + t;
+    const bool live = i < D.N;
+    const int64_t lb0 = (int64_t)blockIdx.y * lc, lb1 = min(D.L, lb0 + lc);
+    for (int k = 0; k < K; ++k) ms[k * IA_T + t] = 0;
+    for (int64_t l0 = lb0; l0 < lb1; l0 += IA_LC) {
+        const int nl = (int)min((int64_t)IA_LC, lb1 - l0);
+        __syncthreads();
+        for (int j = t; j < IA_LC * nb; j += IA_T) hs[j] = 0;
+        __syncthreads();
+        if (live)
+            for (int ll = 0; ll < nl; ++ll) {
+                const int64_t l = l0 + ll;
+                Copies cp;
+                load_copies(D, l, i, cp);
+                if (!cp.n) continue;
+                Philox ph;
+                ph.init(c.seed, ST_INITADM, (uint32_t)l, (uint32_t)i);
+                for (int a = 0; a < cp.n; ++a) {
+                    const int k2 = (int)(ph.next() % (uint32_t)K);
+                    ms[k2 * IA_T + t]++;
+                    atomicAdd(&hs[ll * nb + k2 * MK + cp.a[a]], 1);
+                }
+            }
+        __syncthreads();
+        for (int j = t; j < nl * nb; j += IA_T) {
+            const int v = hs[j];
+            if (!v) continue;
+            const int a = j % MK, k = (j / MK) % K, ll = j / nb;
+            atomicAdd(&c.Ni[(int64_t)k * D.KT + D.off[l0 + ll] + a], v);
+        }
+    }
+    if (live)
+        for (int k = 0; k < K; ++k) {
+            const int v = ms[k * IA_T + t];
+            if (v) atomicAdd(&c.Mi[(int64_t)i * K + k], v);
+        }
 }
 
 // ---------------------------------------------------------------------------

@@ -364,6 +364,7 @@ size_t zadm_smem(const vp_chain* c) {
     const int K = c->P.K, MK = c->ctx->maxK;
     return (size_t)ZA_LC * MK * (K | 1) * 4 + (size_t)ZA_LC * K * MK * 4;
 }
+size_t init_smem(const vp_chain* c) { return (size_t)c->P.K * (IA_LC * c->ctx->maxK + IA_T) * sizeof(int32_t); }
 // instantiations of the per-copy label kernel: exact cluster counts up to
 // 12, then padded sizes
 #define VP_ZADM_EXACT(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12)
@@ -442,6 +443,7 @@ void set_smem_limits(int device) {
     if (!first_on_device(mu, seen, device)) return;
     const int big = 200 * 1024;
     cudaFuncSetAttribute(k_count_noadmix, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+    cudaFuncSetAttribute(k_init_admix_ctr, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     cudaFuncSetAttribute(k_count_packed<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     cudaFuncSetAttribute(k_count_packed<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     cudaFuncSetAttribute(k_count_packed<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
@@ -906,8 +908,16 @@ extern "C" int vp_chain_create(vp_ctx* x, const vp_params* P, vp_chain** out) {
             }
             if ((rc = launch_count(c, 1))) break;
         } else {
-            k_init_admix<<<cdiv(L, 128), 128, 0, s>>>(c->d);
-            if ((rc = check_launch(x, "k_init_admix"))) break;
+            if (P->rng == VP_RNG_REFERENCE) {
+                k_init_admix_ref<<<cdiv(L, 128), 128, 0, s>>>(c->d);
+                if ((rc = check_launch(x, "k_init_admix_ref"))) break;
+            } else {
+                // about 16 CTAs' worth of locus ranges per SM
+                const int64_t nx = cdiv(N, IA_T), ny = std::max<int64_t>(1, (int64_t)x->nsm * 16 / nx);
+                const int lc = (int)(cdiv(cdiv(L, ny), IA_LC) * IA_LC);
+                k_init_admix_ctr<<<dim3(nx, cdiv(L, lc), 1), IA_T, init_smem(c), s>>>(c->d, lc);
+                if ((rc = check_launch(x, "k_init_admix_ctr"))) break;
+            }
         }
     } while (0);
     if (rc) { dev_free(c->mem, x->stream); delete c; return rc; }
