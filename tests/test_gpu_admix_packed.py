@@ -17,7 +17,8 @@ def _run(d, packed, K, sweeps, **kw):
     ctx = S.Context(ds)
     c = S.Chain(ctx, S.params(K, 77 + K, nburnin=2, nreps=max(1, sweeps - 2), nthinning=2, writelnl=1, **kw))
     c.run(sweeps)
-    out = {f: c.get(f) for f in ("NI", "MI", "Q", "FREQ", "ALPHA")}
+    out = {f: c.get(f) for f in ("NI", "MI", "Q", "FREQ", "ALPHA", "METRO")}
+    out["L"] = ds.L
     out["lnl"] = c.result()["lnl"]
     c.close()
     ctx.close()
@@ -30,6 +31,9 @@ def _same(a, b):
     # the copies' ln(sum q p) are added in another grouping (FP32 Kahan sums per
     # lane and range, FP64 across): within a few FP32 ulps of a lane's sum
     assert np.allclose(a["lnl"], b["lnl"], rtol=1e-7, atol=0)
+    # Metropolis log ratios: the byte layout's FP32 sums over 64 copies round
+    # at up to 64 x 5 x 2^-24 a copy
+    assert np.allclose(a["METRO"], b["METRO"], rtol=0, atol=2 * 64 * 5 * 2.0 ** -24 * a["L"])
 
 
 # sizes around the warp, the CTA and the 16-locus slice

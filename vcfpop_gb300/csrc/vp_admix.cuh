@@ -128,7 +128,11 @@ __host__ __device__ constexpr int pz_chunks() { return ((KM + 1) / 2) | 1; }
 // the two neighbouring counts. One barrier a slice: table and histogram are
 // double-buffered.
 //
-// Measured (one GB300, launch): see the dispatch in launch_zadm_ctr.
+// Measured, us a launch against k_update_z_admix_ctr on the same calls: N = 2,000 x
+// L = 50,000, K = 5 1,030 -> 375; N = 4,999 x L = 40,009, K = 11 3,700 -> 1,160;
+// N = 300 x L = 3,000, K = 4 32 -> 17. At K = 5 issue is 75% active, the ALU
+// pipe 61%, the multiplier pipe (Philox) 64%. Round keys read from shared
+// memory instead of added up gave 1.7%, 2 or 4 CTAs per SM instead of 3 lost 1%.
 constexpr int PZ_MAXK = 16;
 constexpr int PZ_MAXT = 256;
 template <int KM, bool EXACT>
@@ -311,6 +315,116 @@ __global__ void __launch_bounds__(PZ_MAXT, KM <= 6 ? 3 : 2) k_z_admix_pk(const D
             if ((EXACT || k < K) && mi[k]) atomicAdd(&c.Mi[(int64_t)i * K + k], mi[k]);
     const double t = block_sum((double)ls - (double)lc, sh);
     if (threadIdx.x == 0) c.lnlp[vb.y * vb.gx + vb.x] = t;
+}
+
+// The Metropolis log ratios (UpdateQMetro, src/structure.cpp:1006-1086) on the
+// sliced 2-bit genotypes: per individual the sum over its copies of
+// ln(sum_k q'_k p / sum_k q_k p), one partial per locus range (grid.y) in
+// metrop. The staged table and packed FP32 operations of k_z_admix_pk give the
+// four weighted sums of a call. Their logarithms are not taken one by one: the
+// products of the numerators and of the denominators are carried as a mantissa
+// in [1, 2) and an integer exponent each, and one logarithm of the mantissas'
+// ratio closes a range, which rounds less than a sum of FP32 logarithms (two
+// roundings of 2^-24 a copy against a rounding at the running sum's size). A
+// call with a product below 2^-100 adds its logarithms singly, so that zeros
+// and infinities come out as they do from the terms.
+// Issue-bound: N = 2,000 x L = 50,000, K = 5 593 -> 149 us a launch, N = 4,999 x
+// L = 40,009, K = 11 1,586 -> 535 us (against k_metro_ratio on the same calls).
+template <int KM, bool EXACT>
+__global__ void __launch_bounds__(PZ_MAXT, 2) k_metro_pk(const DevChain* chains, int force, const int4* map = nullptr) {
+    constexpr int CH = pz_chunks<KM>();
+    constexpr int NF = (PZ_LC * KM + 127) / 128;
+    __shared__ __align__(16) float2 sF[2][PZ_LC][4][CH * 2];
+    const VBlock vb = vblock(map);
+    const DevChain& c = chains[vb.z];
+    if (map && run_over(c)) return;
+    const DevData& D = c.D;
+    const int K = EXACT ? KM : c.K, m = c.ctl->m;
+    if (!force && !metro_turn(c, m)) return;
+    const int T = blockDim.x, i = vb.x * T + threadIdx.x;
+    const bool live = i < D.N;
+    const int Npad = (D.N + 31) & ~31;
+    const int nsl = (int)((D.L + PZ_LC - 1) / PZ_LC);
+    const int s0 = vb.y * c.pz_slices, s1 = min(nsl, s0 + c.pz_slices);
+    if (s0 >= s1) return;
+    f2x q1[KM], q0[KM];
+#pragma unroll
+    for (int k = 0; k < KM; ++k) {
+        const bool on = live && (EXACT || k < K);
+        const float a = on ? c.Qprop[(int64_t)i * K + k] : 0.f, b = on ? c.Q[(int64_t)i * K + k] : 0.f;
+        q1[k] = f2_pack(a, a);
+        q0[k] = f2_pack(b, b);
+    }
+    const float2* F2 = reinterpret_cast<const float2*>(c.Freq);
+    auto stage = [&](int s, int buf) {
+#pragma unroll
+        for (int u = 0; u < NF; ++u) {
+            const int j = threadIdx.x + u * T, k = j >> 4;
+            if (j >= PZ_LC * KM) break;
+            const int64_t l = (int64_t)s * PZ_LC + (j & 15);
+            const float2 f = k < K && l < D.L ? __ldg(F2 + (int64_t)k * D.L + l) : make_float2(0.f, 0.f);
+            float2(*r)[CH * 2] = sF[buf][j & 15];
+            r[0][k] = make_float2(f.x, f.x);
+            r[1][k] = f;
+            r[2][k] = make_float2(f.y, f.y);
+        }
+    };
+    // an odd cluster count leaves one column unwritten, read and not used;
+    // the missing code's rows are read and not used too
+    float R1 = 1.f, R0 = 1.f, single = 0.f;
+    int ex = 0;
+    auto normalise = [](float& r) {
+        const uint32_t b = __float_as_uint(r);
+        r = __uint_as_float((b & 0x007FFFFFu) | 0x3F800000u);
+        return (int)(b >> 23) - 127;
+    };
+    stage(s0, 0);
+    uint32_t gn = i < Npad ? __ldg(D.gt + (int64_t)s0 * Npad + i) : 0xFFFFFFFFu;
+    __syncthreads();
+    int buf = 0;
+    for (int s = s0; s < s1; ++s, buf ^= 1) {
+        uint32_t gw = gn;
+        if (s + 1 < s1) {
+            if (i < Npad) gn = __ldg(D.gt + (int64_t)(s + 1) * Npad + i);
+            stage(s + 1, buf ^ 1);
+        }
+#pragma unroll 4
+        for (int ll = 0; ll < PZ_LC; ++ll) {
+            const uint32_t code = gw & 3u;
+            gw >>= 2;
+            const float4* row = reinterpret_cast<const float4*>(&sF[buf][ll][code][0]);
+            f2x x1 = 0, x0 = 0;
+#pragma unroll
+            for (int k = 0; k < KM; k += 2) {
+                const float4 f = row[k >> 1];
+                const f2x fa = f2_pack(f.x, f.y), fb = f2_pack(f.z, f.w);
+                x1 = f2_fma(q1[k], fa, x1);
+                x0 = f2_fma(q0[k], fa, x0);
+                if (k + 1 < KM) {
+                    x1 = f2_fma(q1[k + 1], fb, x1);
+                    x0 = f2_fma(q0[k + 1], fb, x0);
+                }
+            }
+            float a1, b1, a0, b0;
+            f2_unpack(x1, a1, b1);
+            f2_unpack(x0, a0, b0);
+            const float p1 = a1 * b1, p0 = a0 * b0;
+            const bool fine = p1 > 7.888609e-31f && p0 > 7.888609e-31f;   // 2^-100
+            if (code != 3u) {
+                if (fine) {
+                    R1 *= p1;
+                    R0 *= p0;
+                    ex += normalise(R1) - normalise(R0);
+                } else {
+                    single += logf(a1 / a0);
+                    single += logf(b1 / b0);
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (live)
+        c.metrop[(int64_t)vb.y * D.N + i] = (double)ex * 0.693147180559945309 + (double)logf(R1 / R0) + (double)single;
 }
 
 }  // namespace vp

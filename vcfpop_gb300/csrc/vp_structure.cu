@@ -412,6 +412,16 @@ int launch_zadm_ctr(vp_chain* c, int force) {
 // the Metropolis ratio kernel on the same K instantiations as the label kernel
 int launch_metro_ratio(vp_chain* c, int force) {
     vp_ctx* x = c->ctx;
+    if (pz_form(x->packed2, c->P)) {
+        const int T = pz_threads(x->N), K = c->P.K;
+        const dim3 g(cdiv(x->N, T), c->h.nmetro, 1);
+#define VP_ME(n) \
+    if (K == n) { SL(c, (k_metro_pk<n, true>), (g), (T), 0, 1, force); return VP_OK; }
+        VP_ZADM_EXACT(VP_ME)
+#undef VP_ME
+        SL(c, (k_metro_pk<PZ_MAXK, false>), (g), (T), 0, 1, force);
+        return VP_OK;
+    }
     const dim3 g(cdiv(x->N, 256), cdiv(x->L, c->h.zadm_lc), 1);
     const size_t sm = (size_t)ZA_LC * x->maxK * (c->P.K | 1) * 4;
     const int K = c->P.K;
@@ -513,7 +523,7 @@ int launch_step(vp_chain* c, int step, int force) {
                 if (P.metrofreq > 0) {
                     SL(c, k_metro_propose, (ref ? 1 : gi, 1, 1), (ref ? 32 : 256), 0, 1, 0);
                     if (int rc = launch_metro_ratio(c, 0)) return rc;
-                    SL(c, k_metro_accept, (ref ? 1 : gi, 1, 1), (ref ? 32 : 256), 0, 1, 0);
+                    SL(c, k_metro_accept, (ref ? 1 : cdiv(x->N, MA_I), 1, 1), (ref ? 32 : MA_T), 0, 1, 0);
                 }
             }
             return VP_OK;
@@ -727,7 +737,7 @@ void chain_layout(Carve& cv, vp_chain* c, const vp_ctx* x) {
     h.LL = cv.take<double>((int64_t)N * K);
     h.metro = cv.take<double>(N);
     // Metropolis partials: one per locus range of the per-copy kernels
-    h.metrop = cv.take<double>((int64_t)cdiv(L, h.zadm_lc) * N);
+    h.metrop = cv.take<double>((int64_t)h.nmetro * N);
     h.Alpha = cv.take<double>(K);
     h.Lambda = cv.take<double>(K);
     h.f = cv.take<double>(K);
@@ -808,8 +818,11 @@ int chain_plan(const vp_ctx* x, const vp_params* P, vp_chain* c, size_t* bytes) 
         const int T = pz_threads(N);
         const int64_t nsl = cdiv(L, PZ_LC), nx = cdiv(N, T), want = (int64_t)x->nsm * 64 * 128 / T;
         h.pz_slices = (int32_t)std::max<int64_t>(1, cdiv(nsl * nx, want));
-        if (pz_form(x->packed2, *P))
+        h.nmetro = (int32_t)cdiv(L, h.zadm_lc);
+        if (pz_form(x->packed2, *P)) {
             h.nlnlp = (int32_t)std::max<int64_t>(h.nlnlp, nx * cdiv(nsl, h.pz_slices));
+            h.nmetro = (int32_t)cdiv(nsl, h.pz_slices);
+        }
     }
     c->plain_lazy = tc_batchable(x, P, h);
     Carve probe{nullptr};
