@@ -36,6 +36,7 @@ struct Ctl {
     int32_t m, nr, nlnl, done;     // done: blocks finished, for last-block reductions
     double r;
     double lnl;           // likelihood of the last sampled labels (no-admixture form)
+    double fprop;         // UpdateF's proposal for the next cluster
 };
 
 struct DevChain {
@@ -53,7 +54,7 @@ struct DevChain {
     int32_t *Mi, *Ni;
     int64_t* MiSum;
     double *LLp, *LL, *metro, *metrop, *Alpha, *Lambda, *f, *F, *Eta, *Gamma, *AlphaLocal, *SumAlpha;
-    double *rout, *lnlTrace, *red, *lnlp;
+    double *rout, *lnlTrace, *red, *lnlp, *fpart;
     Rng64* rstate;
 };
 
@@ -1766,7 +1767,7 @@ __global__ void k_update_locpriori(const DevChain* chains, const int4* map = nul
 
 // UpdateA1 (src/structure.cpp:1646-1695): independent Dirichlet proposal of the
 // ancestral frequencies at each locus. Reference streams: 32 block streams.
-__device__ void update_a1_locus(const DevChain& c, int64_t l, Rng64* r, Philox* ph, float* pb, float* pc) {
+__device__ void update_a1_locus(const DevChain& c, int64_t l, Rng64& r, float* pb, float* pc) {
     const DevData& D = c.D;
     const int K = c.K;
     int k2 = D.k[l];
@@ -1780,7 +1781,7 @@ __device__ void update_a1_locus(const DevChain& c, int64_t l, Rng64* r, Philox* 
     }
     double s = 0;
     for (int a = 0; a < k2; ++a) {
-        double v = r ? r->gamma((double)pb[a] * 1.0) : (double)ph->gammaf(pb[a]);
+        double v = r.gamma((double)pb[a] * 1.0);
         pc[a] = (float)v;
         s += v;
     }
@@ -1794,7 +1795,7 @@ __device__ void update_a1_locus(const DevChain& c, int64_t l, Rng64* r, Philox* 
         for (int a = 0; a < k2; ++a)
             dlnL += lgamma(fr * pa[a]) - lgamma(fr * pc[a]) + fr * (pc[a] - pa[a]) * ref_mylog(pk[a]);
     }
-    double u = dlnL >= VP_NZERO ? 0 : (r ? r->uniform() : ph->uniformd());
+    double u = dlnL >= VP_NZERO ? 0 : r.uniform();
     if (dlnL >= VP_NZERO || u < exp(dlnL))
         for (int a = 0; a < k2; ++a) pa[a] = pc[a];
 }
@@ -1802,24 +1803,16 @@ __device__ void update_a1_locus(const DevChain& c, int64_t l, Rng64* r, Philox* 
 // UpdateA2 (src/structure.cpp:1745-1804): move mass delta between two alleles.
 // The reference does not advance its frequency pointer on a rejected-bounds
 // locus, so later loci of the same block read shifted frequencies; `pshift`
-// carries that offset for the reference-stream form.
-__device__ void update_a2_locus(const DevChain& c, int64_t l, int64_t pshift, Rng64* r, Philox* ph, bool* skipped) {
+// carries that offset.
+__device__ void update_a2_locus(const DevChain& c, int64_t l, int64_t pshift, Rng64& r, bool* skipped) {
     const DevData& D = c.D;
     const int K = c.K;
     int k2 = D.k[l];
     float* pa = c.FreqA + D.off[l];
     const float* p = c.Freq + D.off[l] - pshift;
     double lam = c.Lambda[0];
-    int m1, n1;
-    double delta;
-    if (r) {
-        m1 = (int)r->nextn(k2); n1 = (int)r->next_avoid(k2, m1);
-        delta = r->uniform(0, pow((double)D.N, -0.5));
-    } else {
-        m1 = (int)(ph->next() % (uint32_t)k2);
-        n1 = (int)(ph->next() % (uint32_t)(k2 - 1)); if (n1 >= m1) n1++;
-        delta = ph->uniformd() * pow((double)D.N, -0.5);
-    }
+    const int m1 = (int)r.nextn(k2), n1 = (int)r.next_avoid(k2, m1);
+    const double delta = r.uniform(0, pow((double)D.N, -0.5));
     double pm0 = pa[m1], pm1 = pm0 + delta, pn0 = pa[n1], pn1 = pn0 - delta;
     *skipped = pm1 >= 1 || pn1 <= 0;
     if (*skipped) return;
@@ -1829,11 +1822,88 @@ __device__ void update_a2_locus(const DevChain& c, int64_t l, int64_t pshift, Rn
         dlnL += lgamma(fr * pm0) + lgamma(fr * pn0) - lgamma(fr * pm1) - lgamma(fr * pn1) +
                 (fr * delta) * ref_mylog(p[k * D.KT + m1] / p[k * D.KT + n1]);
     }
-    double u = dlnL >= VP_NZERO ? 0 : (r ? r->uniform() : ph->uniformd());
+    double u = dlnL >= VP_NZERO ? 0 : r.uniform();
     if (dlnL >= VP_NZERO || u < exp(dlnL)) { pa[m1] = (float)pm1; pa[n1] = (float)pn1; }
 }
 
-__global__ void k_update_a(const DevChain* chains, const int4* map = nullptr) {
+// The same two steps with counter streams, UA_G lanes a locus: the terms of
+// the log ratio (an lgamma pair and a logarithm per cluster and allele, or four
+// and one per cluster) are formed one a lane and added in the serial order, so
+// the decision is the one a thread of its own would take. Each lane draws the
+// locus's stream for itself. FP64-bound; a thread per locus left 47 CTAs of
+// long serial chains at L = 6,000, K = 4 (108-123 us, now 45-61).
+constexpr int UA_G = 8, UA_T = 128;
+struct LaneGroup {
+    uint32_t mask;
+    int j;    // lane in the group
+    // s + the terms t(0), t(1), ..., t(n - 1), in that order
+    template <class F>
+    __device__ __forceinline__ double add(double s, int n, F t) const {
+        for (int b = 0; b < n; b += UA_G) {
+            const double v = b + j < n ? t(b + j) : 0.0;
+            for (int u = 0; u < UA_G && b + u < n; ++u) s += __shfl_sync(mask, v, u, UA_G);
+        }
+        return s;
+    }
+};
+__device__ void update_a1_group(const DevChain& c, int64_t l, Philox& ph, float* pb, float* pc, const LaneGroup& g) {
+    const DevData& D = c.D;
+    const int K = c.K, k2 = D.k[l];
+    float* pa = c.FreqA + D.off[l];
+    const double lam = c.Lambda[0];
+    for (int a = g.j; a < k2; a += UA_G) {
+        float v = (float)lam;
+        for (int k = 0; k < K; ++k) v += c.Freq[k * D.KT + D.off[l] + a] * (float)c.f[k];
+        pb[a] = v;
+    }
+    __syncwarp(g.mask);
+    double s = 0;
+    float mine[64 / UA_G];
+    for (int a = 0; a < k2; ++a) {
+        const float v = ph.gammaf(pb[a]);
+        if (a % UA_G == g.j) mine[a / UA_G] = v;
+        s += (double)v;
+    }
+    const float inv = (float)(1.0 / s);
+    for (int a = g.j; a < k2; a += UA_G) pc[a] = mine[a / UA_G] * inv;
+    __syncwarp(g.mask);
+    double dlnL = g.add(0, k2, [&](int a) { return (pb[a] - lam) * (ref_mylog(pa[a] / pc[a])); });
+    dlnL = g.add(dlnL, K * k2, [&](int t) {
+        const int k = t / k2, a = t - k * k2;
+        const double fr = c.f[k];
+        return lgamma(fr * pa[a]) - lgamma(fr * pc[a]) + fr * (pc[a] - pa[a]) * ref_mylog(c.Freq[k * D.KT + D.off[l] + a]);
+    });
+    const double u = dlnL >= VP_NZERO ? 0 : ph.uniformd();
+    __syncwarp(g.mask);
+    if (dlnL >= VP_NZERO || u < exp(dlnL))
+        for (int a = g.j; a < k2; a += UA_G) pa[a] = pc[a];
+}
+__device__ void update_a2_group(const DevChain& c, int64_t l, Philox& ph, const LaneGroup& g) {
+    const DevData& D = c.D;
+    const int K = c.K, k2 = D.k[l];
+    float* pa = c.FreqA + D.off[l];
+    const float* p = c.Freq + D.off[l];
+    const double lam = c.Lambda[0];
+    const int m1 = (int)(ph.next() % (uint32_t)k2);
+    int n1 = (int)(ph.next() % (uint32_t)(k2 - 1));
+    if (n1 >= m1) n1++;
+    const double delta = ph.uniformd() * pow((double)D.N, -0.5);
+    const double pm0 = pa[m1], pm1 = pm0 + delta, pn0 = pa[n1], pn1 = pn0 - delta;
+    if (pm1 >= 1 || pn1 <= 0) return;
+    double dlnL = (lam - 1) * ref_mylog(pm1 * pn1 / pm0 / pn0);
+    dlnL = g.add(dlnL, K, [&](int k) {
+        const double fr = c.f[k];
+        return lgamma(fr * pm0) + lgamma(fr * pn0) - lgamma(fr * pm1) - lgamma(fr * pn1) +
+               (fr * delta) * ref_mylog(p[k * D.KT + m1] / p[k * D.KT + n1]);
+    });
+    const double u = dlnL >= VP_NZERO ? 0 : ph.uniformd();
+    if (dlnL >= VP_NZERO || u < exp(dlnL)) {
+        __syncwarp(g.mask);
+        if (g.j == 0) { pa[m1] = (float)pm1; pa[n1] = (float)pn1; }
+    }
+}
+
+__global__ void __launch_bounds__(UA_T) k_update_a(const DevChain* chains, const int4* map = nullptr) {
     const VBlock vb = vblock(map);
     const DevChain& c = chains[vb.z];
     if (map && run_over(c)) return;
@@ -1850,27 +1920,42 @@ __global__ void k_update_a(const DevChain* chains, const int4* map = nullptr) {
         float* pc = pb + D.maxK + 16;
         int64_t pshift = 0;
         for (int64_t l = l0; l < l1; ++l) {
-            if (one) update_a1_locus(c, l, &r, nullptr, pb, pc);
+            if (one) update_a1_locus(c, l, r, pb, pc);
             else {
                 bool sk;
-                update_a2_locus(c, l, pshift, &r, nullptr, &sk);
+                update_a2_locus(c, l, pshift, r, &sk);
                 if (sk) pshift += D.k[l];
             }
         }
         return;
     }
-    int64_t l = vb.x * (int64_t)blockDim.x + threadIdx.x;
+    __shared__ float buf[UA_T / UA_G][2][64];
+    const int gi = threadIdx.x / UA_G, j = threadIdx.x % UA_G;
+    const int64_t l = vb.x * (int64_t)(UA_T / UA_G) + gi;
     if (l >= D.L) return;
-    Philox ph; ph.init(c.seed, ST_A | ((uint32_t)m << 4), (uint32_t)l, 0);
-    float pb[64], pc[64];
-    if (one) update_a1_locus(c, l, nullptr, &ph, pb, pc);
-    else { bool sk; update_a2_locus(c, l, 0, nullptr, &ph, &sk); }
+    const LaneGroup g{((1u << UA_G) - 1u) << (threadIdx.x & 31 & ~(UA_G - 1)), j};
+    Philox ph;
+    ph.init(c.seed, ST_A | ((uint32_t)m << 4), (uint32_t)l, 0);
+    if (one) update_a1_group(c, l, ph, buf[gi][0], buf[gi][1], g);
+    else update_a2_group(c, l, ph, g);
 }
 
 // UpdateF (src/structure.cpp:1806-1858): per-cluster F with a Normal random
-// walk. One block per chain: thread 0 owns the stream, the block reduces the
-// sum over all alleles for each proposal.
-__global__ void k_update_f(const DevChain* chains, const int4* map = nullptr) {
+// walk, one launch per cluster (one in all with a single F), since a proposal
+// depends on the draws the decisions before it took. A launch's blocks share
+// the sum over alleles of the proposal's log ratio; the last one to finish adds
+// the blocks' sums in order, decides and draws the next cluster's proposal.
+// The stream is one xorshift sequence per sweep, whose state waits in rstate
+// between launches. Bound by the latency of the FP64 chains (two lgammas and a
+// logarithm an allele, then the decision's on one thread); one block for all of
+// it took 2,000 us at KT = 12,000, K = 4, now 12-32 us a launch (two lanes an
+// allele, an lgamma each: 12-31).
+constexpr int UF_T = 128;
+__device__ __forceinline__ void f_propose(const DevChain& c, Rng64& rng, int k) {
+    c.ctl->fprop = rng.normal(c.F[k], c.stdf);
+    *c.rstate = rng;
+}
+__global__ void __launch_bounds__(UF_T) k_update_f(const DevChain* chains, int k, const int4* map = nullptr) {
     const VBlock vb = vblock(map);
     const DevChain& c = chains[vb.z];
     if (map && run_over(c)) return;
@@ -1878,48 +1963,47 @@ __global__ void k_update_f(const DevChain* chains, const int4* map = nullptr) {
     const DevData& D = c.D;
     const int K = c.K, m = c.ctl->m;
     __shared__ double sh[32];
-    __shared__ double s_fm, s_fo, s_Fm;
-    __shared__ int s_go;
+    __shared__ double s_Fm;
     Rng64 rng;
-    if (threadIdx.x == 0) rng.init(c.seed + (uint64_t)m, VP_SALT_UPDATEF);
-    for (int k = 0; k < K; ++k) {
-        if (threadIdx.x == 0) {
-            double Fo = c.F[k];
-            double Fm = rng.normal(Fo, c.stdf);
-            s_go = !(Fm < 0 || Fm > 1);
-            s_Fm = Fm; s_fo = c.f[k]; s_fm = (1 - Fm) / Fm;
+    if (threadIdx.x == 0) {
+        if (k == 0) {   // every block draws the first proposal for itself
+            rng.init(c.seed + (uint64_t)m, VP_SALT_UPDATEF);
+            s_Fm = rng.normal(c.F[0], c.stdf);
+        } else {
+            s_Fm = c.ctl->fprop;
         }
-        __syncthreads();
-        if (!s_go) {
-            if (c.fsame) return;
-            __syncthreads();
-            continue;
-        }
-        double fm = s_fm, fo = s_fo;
-        double part = 0;
-        for (int k2 = k; k2 < K; ++k2) {
-            const float* p = c.Freq + k2 * D.KT;
-            for (int64_t a = threadIdx.x; a < D.KT; a += blockDim.x) {
-                float pa2 = c.FreqA[a];
-                part += pa2 * (fm - fo) * ref_mylog(p[a]) + lgamma(fo * pa2) - lgamma(fm * pa2);
-            }
-            if (!c.fsame) break;
-        }
-        double tot = block_sum(part, sh);
-        if (threadIdx.x == 0) {
-            double Fo = c.F[k], Fm = s_Fm;
-            double dlnL = c.pmeanf * (Fo - Fm) / (c.pstdf * c.pstdf) +
-                          (c.pmeanf * c.pmeanf / (c.pstdf * c.pstdf) - 1) * ref_mylog(Fm / Fo) +
-                          (c.fsame ? K : 1) * D.L * (lgamma(fm) - lgamma(fo));
-            dlnL += tot;
-            if (dlnL >= VP_NZERO || rng.uniform() < exp(dlnL)) {
-                if (c.fsame) for (int j = 0; j < K; ++j) { c.F[j] = Fm; c.f[j] = fm; }
-                else { c.F[k] = Fm; c.f[k] = fm; }
-            }
-        }
-        __syncthreads();
-        if (c.fsame) return;
     }
+    __syncthreads();
+    const double Fm = s_Fm, fm = (1 - Fm) / Fm, fo = c.f[k];
+    const bool go = !(Fm < 0 || Fm > 1);
+    double part = 0;
+    if (go) {
+        const int64_t n = (c.fsame ? K : 1) * D.KT;
+        const float* p = c.Freq + k * D.KT;
+        for (int64_t e = vb.x * (int64_t)UF_T + threadIdx.x; e < n; e += (int64_t)vb.gx * UF_T) {
+            const float pa2 = c.FreqA[e % D.KT];
+            part += pa2 * (fm - fo) * ref_mylog(p[e]) + lgamma(fo * pa2) - lgamma(fm * pa2);
+        }
+    }
+    part = block_sum(part, sh);
+    if (threadIdx.x == 0) c.fpart[vb.x] = part;
+    if (!last_block_done(c.ctl, vb.gx)) return;
+    const double tot = block_sum_partials(c.fpart, vb.gx, sh);
+    if (threadIdx.x) return;
+    c.ctl->done = 0;
+    if (k) rng = *c.rstate;
+    if (go) {
+        const double Fo = c.F[k];
+        double dlnL = c.pmeanf * (Fo - Fm) / (c.pstdf * c.pstdf) +
+                      (c.pmeanf * c.pmeanf / (c.pstdf * c.pstdf) - 1) * ref_mylog(Fm / Fo) +
+                      (c.fsame ? K : 1) * D.L * (lgamma(fm) - lgamma(fo));
+        dlnL += tot;
+        if (dlnL >= VP_NZERO || rng.uniform() < exp(dlnL)) {
+            if (c.fsame) for (int j = 0; j < K; ++j) { c.F[j] = Fm; c.f[j] = fm; }
+            else { c.F[k] = Fm; c.f[k] = fm; }
+        }
+    }
+    if (!c.fsame && k + 1 < K) f_propose(c, rng, k + 1);
 }
 
 // Record (src/structure.cpp:1941-2045): likelihood trace, running sums of the

@@ -495,6 +495,11 @@ int launch_count(vp_chain* c, int force) {
     return VP_OK;
 }
 
+// blocks of an UpdateF launch: one allele a thread up to 8 blocks per SM
+unsigned f_blocks(const vp_ctx* x, const vp_params& P) {
+    return (unsigned)std::min<int64_t>(cdiv((P.fsame ? P.K : 1) * x->KT, UF_T), (int64_t)x->nsm * 8);
+}
+
 int launch_step(vp_chain* c, int step, int force) {
     vp_ctx* x = c->ctx;
     const vp_params& P = c->P;
@@ -549,11 +554,13 @@ int launch_step(vp_chain* c, int step, int force) {
         case VP_STEP_UPDATEA:
             if (P.fmodel) {
                 if (ref) SL(c, k_update_a, (1, 1, 1), (32), 0, 0);
-                else SL(c, k_update_a, (cdiv(x->L, 128), 1, 1), (128), 0, 0);
+                else SL(c, k_update_a, (cdiv(x->L, UA_T / UA_G), 1, 1), (UA_T), 0, 0);
             }
             return VP_OK;
         case VP_STEP_UPDATEF:
-            if (P.fmodel) SL(c, k_update_f, (1, 1, 1), (256), 0, 0);
+            if (P.fmodel)
+                for (int k = 0; k < (P.fsame ? 1 : K); ++k)
+                    SL(c, k_update_f, (f_blocks(x, P), 1, 1), (UF_T), 0, 1, k);
             return VP_OK;
         case VP_STEP_RECORD:
             // single steps (parity tests): Record alone, without the advance
@@ -750,6 +757,7 @@ void chain_layout(Carve& cv, vp_chain* c, const vp_ctx* x) {
     h.lnlTrace = cv.take<double>(ntrace);
     h.red = cv.take<double>(((int64_t)S * K + K + 1) * (1 + LPQ_BLOCKS));
     h.lnlp = cv.take<double>(h.nlnlp);
+    h.fpart = cv.take<double>(P->fmodel ? f_blocks(x, *P) : 1);
     c->ancestry = cv.take<double>((int64_t)N * K);
     c->d = cv.take<DevChain>(1);
 }
