@@ -754,14 +754,19 @@ __device__ double sample_warp(const DevChain& c, int i, int m, int lane) {
     const int k0 = lane, k1 = lane + 32;
     const bool h0 = k0 < K, h1 = k1 < K;
     double v0 = 0, v1 = 0;
-    // unrolled so that the partials' loads are in flight together; the adds
-    // keep chunk order
+    // Few clusters leave most lanes idle, so the chunk partials are shared by
+    // 32 / 2^ceil(log2 K) groups of lanes (lane k of group g adds cluster k's
+    // chunks g, g + groups, ...) and the groups' sums are added by shuffles;
+    // unrolled so that the loads are in flight together.
+    const int lg = K <= 1 ? 0 : 32 - __clz(K - 1), step = lg < 5 ? 32 >> lg : 1;
+    const int kk = lg < 5 ? lane & ((1 << lg) - 1) : lane;
 #pragma unroll 8
-    for (int ch = 0; ch < c.nchunk; ++ch) {
+    for (int ch = lg < 5 ? lane >> lg : 0; ch < c.nchunk; ch += step) {
         const double* p = c.LLp + ((int64_t)ch * N + i) * K;
-        if (h0) v0 += p[k0];
+        if (kk < K) v0 += p[kk];
         if (h1) v1 += p[k1];
     }
+    for (int o = 1 << lg; o < 32; o <<= 1) v0 += __shfl_xor_sync(0xffffffffu, v0, o);
     double* LL = c.LL + (int64_t)i * K;
     float* Q = c.Q + (int64_t)i * K;
     int32_t* Mi = c.Mi + (int64_t)i * K;
@@ -852,11 +857,29 @@ __global__ void __launch_bounds__(SAMPLE_BLOCK) k_sample_noadmix(const DevChain*
     }
     if (c.locpriori) {
         __syncthreads();
-        for (int j = threadIdx.x; j < D.S * K; j += blockDim.x) c.Di[j] = 0.f;
+        // Q is one-hot, so Di's float sums are exact small integers: counted in
+        // shared memory where they fit (global float atomics on a few hundred
+        // addresses were most of this kernel's 75 us at N = 3,001)
+        constexpr int DI_SH = 2048;
+        __shared__ int di[DI_SH];
+        const int nd = D.S * K;
+        const bool in_sh = nd <= DI_SH;
+        for (int j = threadIdx.x; j < nd; j += blockDim.x) {
+            if (in_sh) di[j] = 0;
+            else c.Di[j] = 0.f;
+        }
         __syncthreads();
-        // Q is one-hot, so these float sums are exact small integers
+#pragma unroll 4
         for (int i = threadIdx.x; i < N; i += blockDim.x)
-            if (D.vt[i]) atomicAdd(&c.Di[D.popid[i] * K + c.Z[i]], 1.f);
+            if (D.vt[i]) {
+                const int j = D.popid[i] * K + c.Z[i];
+                if (in_sh) atomicAdd(&di[j], 1);
+                else atomicAdd(&c.Di[j], 1.f);
+            }
+        if (in_sh) {
+            __syncthreads();
+            for (int j = threadIdx.x; j < nd; j += blockDim.x) c.Di[j] = (float)di[j];
+        }
     }
 }
 
@@ -1481,111 +1504,197 @@ __device__ double logprod_d_serial(const double* a, int64_t n, int64_t sep) {
 //   inferalpha, one alpha: ln prod Q over all N*K (1 output)
 //   diffalpha:             ln prod Q[., k] (K outputs)
 //   location prior+admix:  ln prod Q[i in s, k] (S*K outputs)
-// Reference streams use the serial exponent-split product (a zero resets its
-// running mantissa, as in the reference); counter streams a parallel sum.
-constexpr int LPQ_BLOCKS = 64;
+// Reference streams: the serial exponent-split product (a zero resets its
+// running mantissa, as in the reference), one thread per sequence; counter
+// streams form plain sums in k_update_alpha_ctr.
 __global__ void k_logprod_q(const DevChain* chains, const int4* map = nullptr) {
     const VBlock vb = vblock(map);
     const DevChain& c = chains[vb.z];
     if (map && run_over(c)) return;
     const DevData& D = c.D;
     const int K = c.K, m = c.ctl->m;
-    __shared__ double sh[32];
     int nseq, mode;
     if (c.locpriori && c.admix) { nseq = D.S * K; mode = 2; }
     else if (c.inferalpha && (c.admix || m < c.nadmburnin)) { nseq = c.diffalpha ? K : 1; mode = c.diffalpha; }
     else return;
-    if (c.rng == 0) {
-        // reference streams: the serial exponent-split product, one thread per sequence
-        for (int s = vb.x * blockDim.x + threadIdx.x; s < nseq; s += vb.gx * blockDim.x) {
-            const float* base; int64_t n, sep;
-            if (mode == 2) { int sp = s / K, k = s % K; base = c.Q + (int64_t)D.pop_ind0[sp] * K + k; n = D.pop_nind[sp]; sep = K; }
-            else if (mode == 1) { base = c.Q + s; n = D.N; sep = K; }
-            else { base = c.Q; n = (int64_t)D.N * K; sep = 1; }
-            c.red[s] = logprod_f_serial(base, n, sep);
-        }
-        return;
+    for (int s = vb.x * blockDim.x + threadIdx.x; s < nseq; s += vb.gx * blockDim.x) {
+        const float* base; int64_t n, sep;
+        if (mode == 2) { int sp = s / K, k = s % K; base = c.Q + (int64_t)D.pop_ind0[sp] * K + k; n = D.pop_nind[sp]; sep = K; }
+        else if (mode == 1) { base = c.Q + s; n = D.N; sep = K; }
+        else { base = c.Q; n = (int64_t)D.N * K; sep = 1; }
+        c.red[s] = logprod_f_serial(base, n, sep);
     }
-    if (mode == 2 && D.popcontig) {
-        // counter streams, one sequence per (location, cluster) over the
-        // location's consecutive rows: one block per location, one block sum
-        // per cluster (deterministic)
-        for (int sp = vb.x; sp < D.S; sp += vb.gx) {
-            const int64_t r0 = D.pop_ind0[sp], n = D.pop_nind[sp];
-            for (int k = 0; k < K; ++k) {
-                double v = 0;
-                for (int64_t rr = threadIdx.x; rr < n; rr += blockDim.x) {
-                    const float q = c.Q[(r0 + rr) * K + k];
-                    v += q > 0.f ? (double)logf(q) : -709.0895657128241;
-                }
-                v = block_sum(v, sh);
-                if (threadIdx.x == 0) c.red[sp * K + k] = v;
-            }
-        }
-        return;
-    }
-    // counter streams: sum of ln Q per sequence, per-block partials reduced by
-    // the last block in a fixed order
-    double* part = c.red + (D.S * K + K + 1);   // [LPQ_BLOCKS][nseq]
-    const int64_t NK = (int64_t)D.N * K;
-    for (int s = 0; s < nseq; ++s) {
-        double v = 0;
-        const int64_t per = (NK + vb.gx - 1) / vb.gx;
-        const int64_t j0 = vb.x * per, j1 = min(NK, j0 + per);
-        for (int64_t j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
-            const int i = (int)(j / K), k = (int)(j % K);
-            const int sq = mode == 2 ? D.popid[i] * K + k : mode == 1 ? k : 0;
-            if (sq != s) continue;
-            const float q = c.Q[j];
-            v += q > 0.f ? (double)logf(q) : -709.0895657128241;
-        }
-        v = block_sum(v, sh);
-        if (threadIdx.x == 0) part[vb.x * nseq + s] = v;
-    }
-    if (!last_block_done(c.ctl, vb.gx)) return;
-    for (int s = threadIdx.x; s < nseq; s += blockDim.x) {
-        double t = 0;
-        for (int b2 = 0; b2 < (int)vb.gx; ++b2) t += part[b2 * nseq + s];
-        c.red[s] = t;
-    }
-    if (threadIdx.x == 0) c.ctl->done = 0;
 }
 
-// UpdateAlpha (src/structure.cpp:1499-1594), reference stream
-// RNG(seed + m, SALT_UPDATEALPHA), on one thread
-// counter streams, location prior with admixture. The K global steps are
-// independent of one another (each moves Alpha[k] against AlphaLocal[., k]):
-// one thread per cluster, each on its own Philox stream. A location's K
-// local steps share its SumAlpha and stay in order on one thread, but every
-// term that does not involve SumAlpha (the proposal on its own Philox
-// stream, ln(am/ao), lgamma(am), lgamma(ao), the ln Q sum) is formed first by
-// one thread per (location, cluster); the ordered pass then adds the two
-// SumAlpha lgamma terms and decides. Needs blockDim.x >= K.
-__device__ void update_alpha_locprior_ctr(const DevChain& c, int m) {
+// UpdateAlpha (src/structure.cpp:1499-1594) with counter streams in one launch:
+// the blocks form the sums of ln Q, and the last one to finish takes the step.
+// What is left is a chain of FP64 lgammas and logarithms on one block, so the
+// ones that do not wait for a decision are formed side by side and the
+// decisions, sums and random numbers are those of the serial step:
+//   one alpha    the four lgammas on four lanes;
+//   diffalpha    a cluster's proposal depends on the decisions before it only
+//                through the count of uniforms they took from the stream
+//                (at most one each), so the log ratio of every (cluster,
+//                count) is formed at once and a serial pass picks;
+//   location prior with admixture
+//                the global steps' lgammas and the logarithms of every local
+//                alpha side by side, every SumAlpha-free term of the local
+//                steps side by side, then the ordered SumAlpha chain of each
+//                location with one lgamma a step (the other one is the
+//                previous step's).
+// With a launch of its own for the sums, one alpha took 11 + 20 us (N = 300,
+// K = 4), the location prior 13 + 105 us (20 locations, K = 8); now 25 and 65.
+constexpr int LPQ_BLOCKS = 64, UA_LPQ_T = 256;
+__device__ __forceinline__ double ln_q(float q) { return q > 0.f ? (double)logf(q) : -709.0895657128241; }
+// out[k] = sum of ln of column k of the n rows at q: a thread keeps to one
+// column, the threads of a column are added in order
+__device__ void column_ln_sums(const float* q, int64_t n, int K, double* sh, double* out) {
+    const int t = threadIdx.x, T = UA_LPQ_T / K * K;
+    double v = 0;
+    if (t < T)
+        for (int64_t j = t; j < n * K; j += T) v += ln_q(q[j]);
+    sh[t] = v;
+    __syncthreads();
+    if (t < K) {
+        double s = 0;
+        for (int u = t; u < T; u += K) s += sh[u];
+        out[t] = s;
+    }
+    __syncthreads();
+}
+__device__ void alpha_step_one(const DevChain& c, int m) {
+    const int K = c.K, N = c.D.N, lane = threadIdx.x;
+    if (lane >= 32) return;
+    Rng64 rng;
+    rng.init(c.seed + (uint64_t)m, VP_SALT_UPDATEALPHA);
+    const double am = rng.normal(c.Alpha[0], c.stdalpha);
+    if (am <= 0 || (am >= c.maxalpha && c.uniformalpha)) return;
+    const double ao = c.Alpha[0], d = am - ao;
+    double dlnL = c.uniformalpha ? 0 : ((c.alphapriora - 1) * ref_mylog(am / ao) + (ao - am) / c.alphapriorb);
+    const double lg = lgamma((lane & 1 ? ao : am) * (lane & 2 ? 1.0 : (double)K));
+    const double gkm = __shfl_sync(0xffffffffu, lg, 0), gko = __shfl_sync(0xffffffffu, lg, 1);
+    const double gm = __shfl_sync(0xffffffffu, lg, 2), go = __shfl_sync(0xffffffffu, lg, 3);
+    dlnL += d * c.red[0] + (gkm - gko - K * gm + K * go) * N;
+    __syncwarp();
+    if (dlnL >= VP_NZERO || rng.uniform() < exp(dlnL))
+        for (int k = lane; k < K; k += 32) c.Alpha[k] = am;
+}
+// the serial diffalpha step, one thread
+__device__ void alpha_step_diff_serial(const DevChain& c, Rng64& rng) {
+    const int K = c.K, N = c.D.N;
+    double sumalpha = 0;
+    for (int k = 0; k < K; ++k) sumalpha += c.Alpha[k];
+    for (int k = 0; k < K; ++k) {
+        double am = rng.normal(c.Alpha[k], c.stdalpha);
+        if (am <= 0 || (am >= c.maxalpha && c.uniformalpha)) continue;
+        double ao = c.Alpha[k], d = am - ao;
+        double dlnL = c.uniformalpha ? 0 : ((c.alphapriora - 1) * ref_mylog(am / ao) + (ao - am) / c.alphapriorb);
+        dlnL += (am - ao) * c.red[k] + (lgamma(sumalpha + d) - lgamma(sumalpha) - lgamma(am) + lgamma(ao)) * N;
+        if (dlnL >= VP_NZERO || rng.uniform() < exp(dlnL)) c.Alpha[k] = am;
+    }
+}
+constexpr int DIFF_MAXK = 32;    // clusters whose (cluster, count) table fits; above, the serial step
+__device__ void alpha_step_diff(const DevChain& c, int m) {
+    __shared__ uint64_t raw[3 * DIFF_MAXK + 4];
+    __shared__ double s_am[DIFF_MAXK * (DIFF_MAXK + 1) / 2], s_e[DIFF_MAXK * (DIFF_MAXK + 1) / 2], s_lg[DIFF_MAXK + 1];
+    __shared__ int odd_case;
+    const int K = c.K, N = c.D.N, t = threadIdx.x;
+    Rng64 rng;
+    rng.init(c.seed + (uint64_t)m, VP_SALT_UPDATEALPHA);
+    if (K > DIFF_MAXK) {
+        if (t == 0) alpha_step_diff_serial(c, rng);
+        return;
+    }
+    // the stream's raw draws: two for every pair of proposals, at most one
+    // uniform a cluster
+    const int nraw = 2 * ((K + 1) / 2) + K;
+    if (t == 0) {
+        Rng64 r = rng;
+        for (int j = 0; j < nraw; ++j) raw[j] = r.next();
+        odd_case = 0;
+    }
+    double sumalpha = 0;
+    for (int k = 0; k < K; ++k) sumalpha += c.Alpha[k];
+    if (t <= K) s_lg[t] = lgamma(t < K ? c.Alpha[t] : sumalpha);
+    __syncthreads();
+    auto unit = [](uint64_t u) { return __longlong_as_double((long long)(0x3FF0000000000000ull | (u & 0x000FFFFFFFFFFFFFull))) - 1.0; };
+    // entry (k, j): the proposal of cluster k when j uniforms were taken before
+    // its pair (clusters 2q, 2q + 1) was drawn; e = exp of the log ratio, 2 if
+    // accepted without a uniform, -1 if out of bounds
+    for (int e = t; e < K * (K + 1) / 2; e += UA_LPQ_T) {
+        int k = 0;
+        while ((k + 1) * (k + 2) / 2 <= e) ++k;
+        const int j = e - k * (k + 1) / 2, q = k >> 1;
+        const double v1 = unit(raw[2 * q + j]), v2 = unit(raw[2 * q + j + 1]);
+        const double sq = -2.0 * log(v1);
+        const double U1 = sq > 0 ? sqrt(sq) : (sq > -VP_MIN_FREQ ? 0.0 : __longlong_as_double(0x7ff8000000000000ll));
+        const double U2 = 2.0 * 3.14159265358979323846264338328 * v2;
+        // a first normal whose low word marks "no second value kept"
+        if ((uint32_t)__double_as_longlong(U1) == 0xFFFFFFFFu) odd_case = 1;
+        const double ao = c.Alpha[k];
+        const double am = (k & 1 ? U1 * ref_sin(U2) : U1 * ref_cos(U2)) * c.stdalpha + ao;
+        double r = -1;
+        if (!(am <= 0 || (am >= c.maxalpha && c.uniformalpha))) {
+            const double d = am - ao;
+            double dlnL = c.uniformalpha ? 0 : ((c.alphapriora - 1) * ref_mylog(am / ao) + (ao - am) / c.alphapriorb);
+            dlnL += (am - ao) * c.red[k] + (lgamma(sumalpha + d) - s_lg[K] - lgamma(am) + s_lg[k]) * N;
+            r = dlnL >= VP_NZERO ? 2 : exp(dlnL);
+        }
+        s_am[e] = am;
+        s_e[e] = r;
+    }
+    __syncthreads();
+    if (t) return;
+    if (odd_case) {
+        alpha_step_diff_serial(c, rng);
+        return;
+    }
+    int j = 0, jp = 0;
+    for (int k = 0; k < K; ++k) {
+        if (!(k & 1)) jp = j;
+        const int e = k * (k + 1) / 2 + jp;
+        const double r = s_e[e];
+        if (r == -1) continue;
+        if (r == 2 || unit(raw[2 * (k / 2 + 1) + j++]) < r) c.Alpha[k] = s_am[e];
+    }
+}
+__device__ void alpha_step_locprior(const DevChain& c, int m) {
     const DevData& D = c.D;
     const int K = c.K, S = D.S;
     const double r = c.ctl->r;
-    const int t = threadIdx.x;
+    const int t = threadIdx.x, T = blockDim.x;
+    __shared__ double g_am[64], g_u[64], g_lg[128];
+    // proposals and the SumAlpha-free part of each local log ratio, [S][K] x
+    // (proposal, partial ratio, uniform), in the region of c.red past the sums
+    double* pre = c.red + ((int64_t)S * K + K + 1);
+    for (int j = t; j < S * K; j += T) pre[3 * (int64_t)j] = ref_mylog(c.AlphaLocal[j]);
+    if (t < K) {
+        Philox ph;
+        ph.init(c.seed, ST_ALPHA | ((uint32_t)m << 4), 0xFFFFFFFFu, 2u + (uint32_t)t);
+        g_am[t] = c.Alpha[t] + c.stdalpha * ph.normald();
+        g_u[t] = ph.uniformd();
+    }
+    __syncthreads();
+    if (t < 2 * K) {
+        const int k = t >> 1;
+        const double am = g_am[k];
+        g_lg[t] = am > 0 && am < c.maxalpha ? lgamma(r * (t & 1 ? am : c.Alpha[k])) : 0;
+    }
+    __syncthreads();
     if (t < K) {
         const int k = t;
-        Philox ph;
-        ph.init(c.seed, ST_ALPHA | ((uint32_t)m << 4), 0xFFFFFFFFu, 2u + (uint32_t)k);
-        const double a0 = c.Alpha[k], am = a0 + c.stdalpha * ph.normald();
+        const double a0 = c.Alpha[k], am = g_am[k];
         if (am > 0 && am < c.maxalpha) {
             const double d = am - a0;
-            double dlnL = S * (d * r * ref_mylog(r) + lgamma(r * a0) - lgamma(r * am));
+            double dlnL = S * (d * r * ref_mylog(r) + g_lg[2 * k] - g_lg[2 * k + 1]);
             double lp = 0;   // ln of the product over locations of AlphaLocal[., k]
-            for (int sl = 0; sl < S; ++sl) lp += ref_mylog(c.AlphaLocal[sl * K + k]);
+            for (int sl = 0; sl < S; ++sl) lp += pre[3 * ((int64_t)sl * K + k)];
             dlnL += r * d * lp;
-            if (dlnL >= VP_NZERO || ph.uniformd() < exp(dlnL)) c.Alpha[k] = am;
+            if (dlnL >= VP_NZERO || g_u[k] < exp(dlnL)) c.Alpha[k] = am;
         }
     }
     __syncthreads();
-    // proposals and the SumAlpha-free part of each local log ratio, [S][K] x
-    // (proposal, partial ratio, uniform), in the region of c.red that holds
-    // k_logprod_q's block partials (reduced before this kernel runs)
-    double* pre = c.red + ((int64_t)S * K + K + 1);
-    for (int j = t; j < S * K; j += blockDim.x) {
+    for (int j = t; j < S * K; j += T) {
         const int s = j / K, k = j % K;
         Philox ph;
         ph.init(c.seed, ST_ALPHA | ((uint32_t)m << 4), (uint32_t)s, 2u + (uint32_t)k);
@@ -1602,38 +1711,92 @@ __device__ void update_alpha_locprior_ctr(const DevChain& c, int m) {
         pre[3 * (int64_t)j + 2] = u;
     }
     __syncthreads();
-    for (int s = t; s < S; s += blockDim.x) {
+    for (int s = t; s < S; s += T) {
+        double sum = c.SumAlpha[s];
         if (m % 10 == 0) {
-            double tt = 0;
-            for (int k = 0; k < K; ++k) tt += c.AlphaLocal[s * K + k];
-            c.SumAlpha[s] = tt;
+            sum = 0;
+            for (int k = 0; k < K; ++k) sum += c.AlphaLocal[s * K + k];
         }
         const int snind = D.pop_nind[s];
+        double lgs = lgamma(sum);
         for (int k = 0; k < K; ++k) {
             const int64_t j = (int64_t)s * K + k;
             const double ao = c.AlphaLocal[j], am = pre[3 * j];
             if (am > 0 && am < c.maxalpha) {
-                const double d = am - ao;
-                const double dlnL = pre[3 * j + 1] + snind * (lgamma(c.SumAlpha[s] + d) - lgamma(c.SumAlpha[s]));
+                const double d = am - ao, lgn = lgamma(sum + d);
+                const double dlnL = pre[3 * j + 1] + snind * (lgn - lgs);
                 if (dlnL >= VP_NZERO || pre[3 * j + 2] < exp(dlnL)) {
                     c.AlphaLocal[j] = am;
-                    c.SumAlpha[s] += d;
+                    sum += d;
+                    lgs = lgn;
                 }
             }
         }
+        c.SumAlpha[s] = sum;
     }
 }
+__global__ void __launch_bounds__(UA_LPQ_T) k_update_alpha_ctr(const DevChain* chains, const int4* map = nullptr) {
+    const VBlock vb = vblock(map);
+    const DevChain& c = chains[vb.z];
+    if (map && run_over(c)) return;
+    const DevData& D = c.D;
+    const int K = c.K, m = c.ctl->m, t = threadIdx.x;
+    __shared__ double sh[UA_LPQ_T];
+    __shared__ double col[64];
+    const bool loc = c.locpriori && c.admix;
+    if (!loc && !(c.inferalpha && (c.admix || m < c.nadmburnin))) return;
+    if (loc && D.popcontig) {
+        // a location's rows are consecutive: one block per location
+        for (int sp = vb.x; sp < D.S; sp += vb.gx)
+            column_ln_sums(c.Q + (int64_t)D.pop_ind0[sp] * K, D.pop_nind[sp], K, sh, c.red + sp * K);
+        if (!last_block_done(c.ctl, vb.gx)) return;
+    } else {
+        // per-block partials of a range of rows, added by the last block in order
+        const int nseq = loc ? D.S * K : c.diffalpha ? K : 1;
+        double* part = c.red + (D.S * K + K + 1);   // [LPQ_BLOCKS][nseq]
+        const int64_t per = (D.N + vb.gx - 1) / vb.gx;
+        const int64_t r0 = min((int64_t)D.N, vb.x * per), n = min((int64_t)D.N - r0, per);
+        if (loc) {
+            for (int s = 0; s < nseq; ++s) {
+                double v = 0;
+                for (int64_t j = t; j < n * K; j += UA_LPQ_T) {
+                    const int64_t i = r0 + j / K;
+                    if (D.popid[i] * K + (int)(j % K) == s) v += ln_q(c.Q[i * K + j % K]);
+                }
+                v = block_sum(v, sh);
+                if (t == 0) part[vb.x * nseq + s] = v;
+            }
+        } else {
+            column_ln_sums(c.Q + r0 * K, n, K, sh, col);
+            if (c.diffalpha) {
+                if (t < K) part[vb.x * nseq + t] = col[t];
+            } else if (t == 0) {
+                double v = 0;
+                for (int k = 0; k < K; ++k) v += col[k];
+                part[vb.x] = v;
+            }
+        }
+        if (!last_block_done(c.ctl, vb.gx)) return;
+        for (int s = t; s < nseq; s += UA_LPQ_T) {
+            double v = 0;
+#pragma unroll 8
+            for (int b = 0; b < vb.gx; ++b) v += part[b * nseq + s];
+            c.red[s] = v;
+        }
+    }
+    if (t == 0) c.ctl->done = 0;
+    __syncthreads();
+    if (loc) alpha_step_locprior(c, m);
+    else if (c.diffalpha) alpha_step_diff(c, m);
+    else alpha_step_one(c, m);
+}
 
+// UpdateAlpha, reference stream RNG(seed + m, SALT_UPDATEALPHA), on one thread
 __global__ void k_update_alpha(const DevChain* chains, const int4* map = nullptr) {
     const VBlock vb = vblock(map);
     const DevChain& c = chains[vb.z];
     if (map && run_over(c)) return;
-    if (vb.x) return;
-    if (c.rng != 0 && c.locpriori && c.admix) {
-        update_alpha_locprior_ctr(c, c.ctl->m);
-        return;
-    }
-    if (threadIdx.x) return;
+    if (vb.x || threadIdx.x) return;
     const DevData& D = c.D;
     const int K = c.K, m = c.ctl->m, S = D.S, N = D.N;
     Rng64 rng; rng.init(c.seed + (uint64_t)m, VP_SALT_UPDATEALPHA);
@@ -1675,16 +1838,7 @@ __global__ void k_update_alpha(const DevChain* chains, const int4* map = nullptr
     if (!c.inferalpha) return;
     if (!c.admix && m >= c.nadmburnin) return;
     if (c.diffalpha) {
-        double sumalpha = 0;
-        for (int k = 0; k < K; ++k) sumalpha += c.Alpha[k];
-        for (int k = 0; k < K; ++k) {
-            double am = rng.normal(c.Alpha[k], c.stdalpha);
-            if (am <= 0 || (am >= c.maxalpha && c.uniformalpha)) continue;
-            double ao = c.Alpha[k], d = am - ao;
-            double dlnL = c.uniformalpha ? 0 : ((c.alphapriora - 1) * ref_mylog(am / ao) + (ao - am) / c.alphapriorb);
-            dlnL += (am - ao) * c.red[k] + (lgamma(sumalpha + d) - lgamma(sumalpha) - lgamma(am) + lgamma(ao)) * N;
-            if (dlnL >= VP_NZERO || rng.uniform() < exp(dlnL)) c.Alpha[k] = am;
-        }
+        alpha_step_diff_serial(c, rng);
     } else {
         double am = rng.normal(c.Alpha[0], c.stdalpha);
         if (am <= 0 || (am >= c.maxalpha && c.uniformalpha)) return;
@@ -1696,70 +1850,161 @@ __global__ void k_update_alpha(const DevChain* chains, const int4* map = nullptr
     }
 }
 
-// UpdateLocPriori (src/structure.cpp:1168-1255), one thread
-__global__ void k_update_locpriori(const DevChain* chains, const int4* map = nullptr) {
+// UpdateLocPriori (src/structure.cpp:1168-1255), one block, both random-number
+// families (one xorshift stream a sweep). Thread 0 draws and decides in the
+// reference's order; everything that does not wait for a decision (lgammas,
+// the products over locations, logarithms) is formed side by side and added in
+// that order, so the values are the serial ones. A location's step draws three
+// numbers and takes a fourth, a uniform, only when its log ratio is negative,
+// so where its draws start depends on the decisions before it through a count
+// alone: for LP_G locations at a time every (location, count) is evaluated at
+// once and thread 0 picks. Bound by the FP64 chains' latency; on one thread it
+// took 174-206 us (no admixture, 20 locations, K = 6) and 77 us (admixture, 20
+// locations, K = 8), now 53 and 29.
+constexpr int LP_T = 128, LP_G = 15;
+static_assert(LP_G * (LP_G + 1) / 2 <= LP_T, "an entry a thread");
+__global__ void __launch_bounds__(LP_T) k_update_locpriori(const DevChain* chains, const int4* map = nullptr) {
     const VBlock vb = vblock(map);
     const DevChain& c = chains[vb.z];
     if (map && run_over(c)) return;
-    if (threadIdx.x || vb.x || !c.locpriori) return;
+    if (vb.x || !c.locpriori) return;
     const DevData& D = c.D;
-    const int K = c.K, S = D.S, m = c.ctl->m;
-    Rng64 rng; rng.init(c.seed + (uint64_t)m, VP_SALT_UPDATELOC);
-    double r = c.ctl->r, epsr = c.epsr;
+    const int K = c.K, S = D.S, m = c.ctl->m, t = threadIdx.x;
+    __shared__ double g0[64], g1[64], lp[64], sa[64], s_rm, s_r, s_u[4], s_dl;
+    __shared__ uint64_t raw[4 * LP_G];
+    __shared__ uint8_t res[LP_T];
+    __shared__ int s_i, s_j;
+    Rng64 rng;
+    const double epsr = c.epsr;
+    if (t == 0) {
+        rng.init(c.seed + (uint64_t)m, VP_SALT_UPDATELOC);
+        s_r = c.ctl->r;
+        s_rm = rng.uniform(s_r - epsr, s_r + epsr);
+    }
+    __syncthreads();
+    double r = s_r;
+    const double rm = s_rm;
+    const bool in = rm > 0 && rm < c.maxr;
     if (c.admix) {
-        double rm = rng.uniform(r - epsr, r + epsr);
-        if (rm > 0 && rm < c.maxr) {
-            double dlnL = 0, d = rm - r, dt1 = rm * ref_mylog(rm) - r * ref_mylog(r);
-            for (int k = 0; k < K; ++k) {
-                dlnL += S * (c.Alpha[k] * dt1 - lgamma(rm * c.Alpha[k]) + lgamma(r * c.Alpha[k]));
-                double sa = 0;
-                for (int s = 0; s < S; ++s) sa += c.AlphaLocal[s * K + k];
-                dlnL += c.Alpha[k] * d * logprod_d_serial(c.AlphaLocal + k, S, K) - sa * d;
+        if (!in) return;
+        for (int j = t; j < 3 * K; j += LP_T) {
+            const int k = j % K, what = j / K;
+            if (what == 0) g1[k] = lgamma(rm * c.Alpha[k]);
+            else if (what == 1) g0[k] = lgamma(r * c.Alpha[k]);
+            else {
+                double v = 0;
+                for (int s = 0; s < S; ++s) v += c.AlphaLocal[s * K + k];
+                sa[k] = v;
+                lp[k] = logprod_d_serial(c.AlphaLocal + k, S, K);
             }
-            if (dlnL >= VP_NZERO || rng.uniform() < exp(dlnL)) c.ctl->r = rm;
         }
+        __syncthreads();
+        if (t) return;
+        double dlnL = 0, d = rm - r, dt1 = rm * ref_mylog(rm) - r * ref_mylog(r);
+        for (int k = 0; k < K; ++k) {
+            dlnL += S * (c.Alpha[k] * dt1 - g1[k] + g0[k]);
+            dlnL += c.Alpha[k] * d * lp[k] - sa[k] * d;
+        }
+        if (dlnL >= VP_NZERO || rng.uniform() < exp(dlnL)) c.ctl->r = rm;
         return;
     }
-    double rm = rng.uniform(r - epsr, r + epsr);
-    if (rm > 0 && rm < c.maxr) {
-        double dlnL = lgamma(rm) - lgamma(r);
-        for (int k = 0; k < K; ++k) dlnL += lgamma(r * c.Eta[k]) - lgamma(rm * c.Eta[k]);
-        dlnL *= S;
-        for (int k = 0; k < K; ++k) dlnL += (rm - r) * c.Eta[k] * logprod_d_serial(c.Gamma + k, S, K);
-        if (dlnL >= VP_NZERO || rng.uniform() < exp(dlnL)) c.ctl->r = rm;
+    for (int j = t; j < 3 * K + 2; j += LP_T) {
+        const int k = j % K, what = j / K;
+        if (j >= 3 * K) s_u[j - 3 * K] = in ? lgamma(j == 3 * K ? rm : r) : 0;
+        else if (what == 0) g0[k] = in ? lgamma(r * c.Eta[k]) : 0;
+        else if (what == 1) g1[k] = in ? lgamma(rm * c.Eta[k]) : 0;
+        else lp[k] = logprod_d_serial(c.Gamma + k, S, K);
     }
-    r = c.ctl->r;
+    __syncthreads();
+    if (t == 0) {
+        if (in) {
+            double dlnL = s_u[0] - s_u[1];
+            for (int k = 0; k < K; ++k) dlnL += g0[k] - g1[k];
+            dlnL *= S;
+            for (int k = 0; k < K; ++k) dlnL += (rm - r) * c.Eta[k] * lp[k];
+            if (dlnL >= VP_NZERO || rng.uniform() < exp(dlnL)) c.ctl->r = rm;
+        }
+        s_r = c.ctl->r;
+        if (K >= 2) {
+            s_i = (int)rng.nextn(K);
+            s_j = (int)rng.next_avoid(K, s_i);
+            s_dl = rng.uniform(0, c.epseta);
+        }
+    }
+    __syncthreads();
+    r = s_r;
     if (K >= 2) {
-        int i1 = (int)rng.nextn(K), j1 = (int)rng.next_avoid(K, i1);
-        double delta = rng.uniform(0, c.epseta);
-        double e1 = c.Eta[i1] + delta, e2 = c.Eta[j1] - delta;
-        if (e1 < 1 && e2 > 0) {
-            double dlnL = S * (lgamma(r * c.Eta[i1]) + lgamma(r * c.Eta[j1]) - lgamma(r * e1) - lgamma(r * e2));
-            dlnL += r * delta * (logprod_d_serial(c.Gamma + i1, S, K) - logprod_d_serial(c.Gamma + j1, S, K));
+        const int i1 = s_i, j1 = s_j;
+        const double delta = s_dl, e1 = c.Eta[i1] + delta, e2 = c.Eta[j1] - delta;
+        const bool ok = e1 < 1 && e2 > 0;
+        if (ok && t < 4) s_u[t] = lgamma(r * (t == 0 ? c.Eta[i1] : t == 1 ? c.Eta[j1] : t == 2 ? e1 : e2));
+        __syncthreads();
+        if (ok && t == 0) {
+            double dlnL = S * (s_u[0] + s_u[1] - s_u[2] - s_u[3]);
+            dlnL += r * delta * (lp[i1] - lp[j1]);
             if (dlnL >= VP_NZERO || rng.uniform() < exp(dlnL)) { c.Eta[i1] += delta; c.Eta[j1] -= delta; }
         }
-        for (int s = 0; s < S; ++s) {
-            int a = (int)rng.nextn(K), b = (int)rng.next_avoid(K, a);
-            double dl = rng.uniform(0, c.epsgamma);
-            double* G = c.Gamma + s * K;
-            if (G[a] + dl < 1 && G[b] - dl > 0) {
-                double dlnL = (r * c.Eta[a] - 1.0 + c.Di[s * K + a]) * ref_mylog(1 + dl / G[a]) +
-                              (r * c.Eta[b] - 1.0 + c.Di[s * K + b]) * ref_mylog(1 - dl / G[b]);
-                if (dlnL >= VP_NZERO || rng.uniform() < exp(dlnL)) { G[a] += dl; G[b] -= dl; }
+        for (int b = 0; b < S; b += LP_G) {
+            const int n = min(LP_G, S - b);
+            if (t == 0) {
+                Rng64 peek = rng;
+                for (int j = 0; j < 4 * n; ++j) raw[j] = peek.next();
             }
+            __syncthreads();
+            // entry (u, j): location b + u when j uniforms were taken since b
+            auto draw = [&](int u, int j, int& a, int& a2) {
+                const uint64_t* w = raw + 3 * u + j;
+                a = (int)(w[0] % (uint64_t)K);
+                a2 = (int)(w[1] % (uint64_t)(K - 1));
+                if (a2 >= a) a2++;
+                return (__longlong_as_double((long long)(0x3FF0000000000000ull | (w[2] & 0x000FFFFFFFFFFFFFull))) - 1.0) * c.epsgamma;
+            };
+            if (t < n * (n + 1) / 2) {
+                int u = 0;
+                while ((u + 1) * (u + 2) / 2 <= t) ++u;
+                const int j = t - u * (u + 1) / 2, s = b + u;
+                int a, a2;
+                const double dl = draw(u, j, a, a2);
+                const double* G = c.Gamma + s * K;
+                int v = 0;      // bit 0: accepted, bit 1: a uniform taken
+                if (G[a] + dl < 1 && G[a2] - dl > 0) {
+                    const double dlnL = (r * c.Eta[a] - 1.0 + c.Di[s * K + a]) * ref_mylog(1 + dl / G[a]) +
+                                        (r * c.Eta[a2] - 1.0 + c.Di[s * K + a2]) * ref_mylog(1 - dl / G[a2]);
+                    if (dlnL >= VP_NZERO) v = 1;
+                    else {
+                        const double un = __longlong_as_double((long long)(0x3FF0000000000000ull | (raw[3 * u + j + 3] & 0x000FFFFFFFFFFFFFull))) - 1.0;
+                        v = 2 | (un < exp(dlnL));
+                    }
+                }
+                res[t] = (uint8_t)v;
+            }
+            __syncthreads();
+            if (t == 0) {
+                int j = 0;
+                for (int u = 0; u < n; ++u) {
+                    const int v = res[u * (u + 1) / 2 + j];
+                    if (v & 1) {
+                        int a, a2;
+                        const double dl = draw(u, j, a, a2);
+                        double* G = c.Gamma + (b + u) * K;
+                        G[a] += dl;
+                        G[a2] -= dl;
+                    }
+                    j += v >> 1;
+                }
+                for (int q = 0; q < 3 * n + j; ++q) rng.next();
+            }
+            __syncthreads();
         }
     }
     if (m % 10 == 0) {
-        // Unify (src/math2.cpp:2268-2285)
-        double s = 0;
-        for (int k = 0; k < K; ++k) s += c.Eta[k];
-        double inv = 1.0 / (s + K * VP_MIN_FREQ);
-        for (int k = 0; k < K; ++k) c.Eta[k] = (c.Eta[k] + VP_MIN_FREQ) * inv;
-        for (int sp = 0; sp < S; ++sp) {
-            double* G = c.Gamma + sp * K;
-            double t = 0;
-            for (int k = 0; k < K; ++k) t += G[k];
-            double iv = 1.0 / (t + K * VP_MIN_FREQ);
+        // Unify (src/math2.cpp:2268-2285): a row a thread, then Eta
+        __syncthreads();
+        for (int sp = t; sp <= S; sp += LP_T) {
+            double* G = sp < S ? c.Gamma + sp * K : c.Eta;
+            double v = 0;
+            for (int k = 0; k < K; ++k) v += G[k];
+            const double iv = 1.0 / (v + K * VP_MIN_FREQ);
             for (int k = 0; k < K; ++k) G[k] = (G[k] + VP_MIN_FREQ) * iv;
         }
     }

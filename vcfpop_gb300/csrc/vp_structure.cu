@@ -534,7 +534,7 @@ int launch_step(vp_chain* c, int step, int force) {
             return VP_OK;
         }
         case VP_STEP_LOCPRIORI:
-            if (P.locpriori) SL(c, k_update_locpriori, (1, 1, 1), (32), 0, 0);
+            if (P.locpriori) SL(c, k_update_locpriori, (1, 1, 1), (LP_T), 0, 0);
             return VP_OK;
         case VP_STEP_UPDATEZ:
             if (!P.admix)
@@ -547,8 +547,14 @@ int launch_step(vp_chain* c, int step, int force) {
             return VP_OK;
         case VP_STEP_ALPHA:
             if ((P.inferalpha && (P.admix || c->h.nadmburnin > 0)) || (P.locpriori && P.admix)) {
-                SL(c, k_logprod_q, (ref ? std::max(1, (x->S * K + 255) / 256) : LPQ_BLOCKS, 1, 1), (256), 0, 0);
-                SL(c, k_update_alpha, (1, 1, 1), (128), 0, 0);
+                if (ref) {
+                    SL(c, k_logprod_q, (std::max(1, (x->S * K + 255) / 256), 1, 1), (256), 0, 0);
+                    SL(c, k_update_alpha, (1, 1, 1), (32), 0, 0);
+                } else {
+                    // a block per location, or about 1,024 values a block
+                    const int64_t want = P.locpriori && P.admix && x->D.popcontig ? x->S : cdiv((int64_t)x->N * K, 1024);
+                    SL(c, k_update_alpha_ctr, ((unsigned)std::min<int64_t>(LPQ_BLOCKS, want), 1, 1), (UA_LPQ_T), 0, 0);
+                }
             }
             return VP_OK;
         case VP_STEP_UPDATEA:
