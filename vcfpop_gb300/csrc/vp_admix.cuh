@@ -5,29 +5,9 @@
 
 namespace vp {
 
-// ---------------------------------------------------------------------------
-// Genotypes by slice: word [s][i] holds individual i's 2-bit codes at the
-// PZ_LC loci of slice s (locus 16 s + j at bits 2j, 2j + 1; 3 past the last
-// locus and past the last individual), so that a lane that walks the loci of
-// one individual reads 16 calls with one coalesced load. Built once per
-// context, for chains that draw labels per copy.
-constexpr int PZ_LC = 16;
-static_assert(PZ_LC == ZA_LC, "the Philox streams are per slice of ZA_LC loci");
-__global__ void __launch_bounds__(256) k_build_slices(const DevData D, uint32_t* gt, int Npad) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= Npad) return;
-    const int w = i >> 4, sh = (i & 15) * 2;
-    for (int64_t s = blockIdx.y; s * PZ_LC < D.L; s += gridDim.y) {
-        uint32_t v = 0;
-#pragma unroll
-        for (int j = 0; j < PZ_LC; ++j) {
-            const int64_t l = s * PZ_LC + j;
-            const uint32_t c = l < D.L && i < D.N ? (__ldg(D.g2 + l * D.Nw + w) >> sh) & 3u : 3u;
-            v |= c << (2 * j);
-        }
-        gt[s * Npad + i] = v;
-    }
-}
+// loci of a slice: the Philox streams of the label draws are per slice
+constexpr int PZ_LC = ZA_LC;
+static_assert(PZ_LC == 16, "a slice's codes of one individual fill a word");
 
 // two FP32 values in one 64-bit register pair, and the packed operations on
 // them (each half rounds as the scalar instruction does)
@@ -71,14 +51,20 @@ struct BitTranspose {
         r2 = lane & 2 ? 30 : 2;
         r1 = lane & 1 ? 31 : 1;
     }
-    __device__ __forceinline__ uint32_t operator()(uint32_t x) const {
+    // the outer four steps: a 16 x 16 transpose of two-bit elements in the
+    // even lanes and one in the odd lanes (element p of lane 2 n + w becomes
+    // element n of lane 2 p + w)
+    __device__ __forceinline__ uint32_t codes(uint32_t x) const {
         x = __byte_perm(x, __shfl_xor_sync(0xffffffffu, x, 16), s16);
         x = __byte_perm(x, __shfl_xor_sync(0xffffffffu, x, 8), s8);
         uint32_t y = __shfl_xor_sync(0xffffffffu, x, 4);
         x = (x & k4) | (__funnelshift_l(y, y, r4) & ~k4);
         y = __shfl_xor_sync(0xffffffffu, x, 2);
-        x = (x & k2) | (__funnelshift_l(y, y, r2) & ~k2);
-        y = __shfl_xor_sync(0xffffffffu, x, 1);
+        return (x & k2) | (__funnelshift_l(y, y, r2) & ~k2);
+    }
+    __device__ __forceinline__ uint32_t operator()(uint32_t x) const {
+        x = codes(x);
+        const uint32_t y = __shfl_xor_sync(0xffffffffu, x, 1);
         return (x & k1) | (__funnelshift_l(y, y, r1) & ~k1);
     }
 };
@@ -91,6 +77,15 @@ __device__ __forceinline__ uint32_t label_mask(const uint32_t* p, int k) {
     if (KM > 4) m &= k & 4 ? p[2] : ~p[2];
     if (KM > 8) m &= k & 8 ? p[3] : ~p[3];
     return m;
+}
+
+// lane's word of slice s for the warp's 32 individuals from ib: locus lane / 2,
+// the first genotype word in even lanes, the second in odd ones (missing codes
+// past the last locus and word)
+__device__ __forceinline__ uint32_t slice_word(const DevData& D, int s, int ib, int lane) {
+    const int64_t l = (int64_t)s * PZ_LC + (lane >> 1);
+    const int w = (ib >> 4) + (lane & 1);
+    return l < D.L && w < D.Nw ? __ldg(D.g2 + l * D.Nw + w) : 0xFFFFFFFFu;
 }
 
 // 16-byte chunks (two clusters' frequency pairs) of a table row, an odd count:
@@ -114,6 +109,9 @@ __host__ __device__ constexpr int pz_chunks() { return ((KM + 1) / 2) | 1; }
 //    the first copy's allele, of the second's) of every cluster, so that one
 //    16-byte load brings two clusters of both copies and packed FP32
 //    instructions serve both copies at once;
+//  - a warp reads the slice's 32 genotype words (16 loci x 32 individuals),
+//    one a lane, and transposes them in registers, so that each lane holds
+//    its individual's 16 codes in one word;
 //  - labels go four bits each into a word (eight copies), the words become
 //    bit planes of a slice's 32 copies, and a lane's copies per cluster are
 //    one population count a cluster and slice;
@@ -135,13 +133,18 @@ __host__ __device__ constexpr int pz_chunks() { return ((KM + 1) / 2) | 1; }
 // memory instead of added up gave 1.7%, 2 or 4 CTAs per SM instead of 3 lost 1%.
 constexpr int PZ_MAXK = 16;
 constexpr int PZ_MAXT = 256;
-template <int KM, bool EXACT>
-__global__ void __launch_bounds__(PZ_MAXT, KM <= 6 ? 3 : 2) k_z_admix_pk(const DevChain* chains, int force,
+// INIT: the initial labels (InitAdmix, as k_init_admix_ctr: a Philox stream a
+// call, draws modulo K) with the same counting, for the padded cluster count
+// only. N = 2,000 x L = 50,000, K = 5 801 -> 311 us, N = 4,999 x L =
+// 40,009, K = 11 1,676 -> 631 us against k_init_admix_ctr, which adds every copy
+// to shared histograms.
+template <int KM, bool EXACT, bool INIT = false>
+__global__ void __launch_bounds__(PZ_MAXT, KM <= 6 || INIT ? 3 : 2) k_z_admix_pk(const DevChain* chains, int force,
                                                                         const int4* map = nullptr) {
     constexpr int CH = pz_chunks<KM>();
     constexpr int NPL = KM <= 2 ? 1 : KM <= 4 ? 2 : KM <= 8 ? 3 : 4;      // bit planes of a label
     constexpr int NF = (PZ_LC * KM + 127) / 128;                          // staged frequencies a thread (128 threads or more)
-    __shared__ __align__(16) float2 sF[2][PZ_LC][4][CH * 2];
+    __shared__ __align__(16) float2 sF[INIT ? 1 : 2][INIT ? 1 : PZ_LC][4][CH * 2];
     __shared__ uint32_t hs[2][KM][PZ_LC];
     __shared__ double sh[32];
     const VBlock vb = vblock(map);
@@ -149,7 +152,7 @@ __global__ void __launch_bounds__(PZ_MAXT, KM <= 6 ? 3 : 2) k_z_admix_pk(const D
     if (map && run_over(c)) return;
     const DevData& D = c.D;
     const int K = EXACT ? KM : c.K, m = c.ctl->m;
-    if (!force && binaryq_at(c, m)) return;
+    if (!INIT && !force && binaryq_at(c, m)) return;
     const int lane = threadIdx.x & 31, T = blockDim.x;
     const int ib = vb.x * T + (threadIdx.x & ~31);
     const int i = ib + (lane >> 1) + 16 * (lane & 1);
@@ -157,12 +160,11 @@ __global__ void __launch_bounds__(PZ_MAXT, KM <= 6 ? 3 : 2) k_z_admix_pk(const D
     const uint32_t lives = __ballot_sync(0xffffffffu, live);
     const int nsl = (int)((D.L + PZ_LC - 1) / PZ_LC);
     const int s0 = vb.y * c.pz_slices, s1 = min(nsl, s0 + c.pz_slices);
-    const int Npad = (D.N + 31) & ~31;
     f2x q[KM];
     int32_t mi[KM];
 #pragma unroll
     for (int k = 0; k < KM; ++k) {
-        const float v = (live && (EXACT || k < K)) ? c.Q[(int64_t)i * K + k] : 0.f;
+        const float v = (!INIT && live && (EXACT || k < K)) ? c.Q[(int64_t)i * K + k] : 0.f;
         q[k] = f2_pack(v, v);
         mi[k] = 0;
     }
@@ -172,7 +174,7 @@ __global__ void __launch_bounds__(PZ_MAXT, KM <= 6 ? 3 : 2) k_z_admix_pk(const D
     const int slot = 7 - (lane >> 2), pl = 4 * (3 - (lane & 3)) + (slot >> 1);
     const bool second = slot & 1;
     const BitTranspose tr(lane);
-    const bool rec = force || record_at(c, m);
+    const bool rec = !INIT && (force || record_at(c, m));
     float ls = 0.f, lc = 0.f;                       // Kahan sum of ln(sum_k q_k p)
     const float minf = (float)VP_MIN_FREQ;
     const f2x kmin = f2_pack((float)(VP_MIN_FREQ * K), (float)(VP_MIN_FREQ * K));
@@ -202,29 +204,25 @@ __global__ void __launch_bounds__(PZ_MAXT, KM <= 6 ? 3 : 2) k_z_admix_pk(const D
         }
     };
     if (s0 >= s1) return;
-    for (int j = threadIdx.x; j < 2 * PZ_LC * CH * 2; j += T)
-        sF[j / (PZ_LC * CH * 2)][j / (CH * 2) % PZ_LC][3][j % (CH * 2)] = make_float2(0.f, 0.f);
+    if constexpr (!INIT)
+        for (int j = threadIdx.x; j < 2 * PZ_LC * CH * 2; j += T)
+            sF[j / (PZ_LC * CH * 2)][j / (CH * 2) % PZ_LC][3][j % (CH * 2)] = make_float2(0.f, 0.f);
     for (int j = threadIdx.x; j < 2 * KM * PZ_LC; j += T) (&hs[0][0][0])[j] = 0;
-    load_f(s0);
-    store_f(0);
-    uint32_t gn = ib < Npad ? __ldg(D.gt + (int64_t)s0 * Npad + i) : 0xFFFFFFFFu;
+    if constexpr (!INIT) {
+        load_f(s0);
+        store_f(0);
+    }
+    const uint32_t modm = INIT ? (uint32_t)min(0x100000000ull / (uint32_t)K, 0xFFFFFFFFull) : 0;
+    uint32_t wn = slice_word(D, s0, ib, lane);
     __syncthreads();
     int buf = 0;
     for (int s = s0; s < s1; ++s, buf ^= 1) {
-        uint32_t gw = gn;
-        // this lane's locus for the counts: its two genotype words
-        uint32_t w0 = 0xFFFFFFFFu, w1 = 0xFFFFFFFFu;
-        {
-            const int64_t l = (int64_t)s * PZ_LC + pl;
-            const int w = ib >> 4;
-            if (l < D.L) {
-                if (w < D.Nw) w0 = __ldg(D.g2 + l * D.Nw + w);
-                if (w + 1 < D.Nw) w1 = __ldg(D.g2 + l * D.Nw + w + 1);
-            }
-        }
+        const uint32_t w = wn;
+        uint32_t gw = tr.codes(w);
+        if (!live) gw = 0xFFFFFFFFu;
         if (s + 1 < s1) {
-            if (ib < Npad) gn = __ldg(D.gt + (int64_t)(s + 1) * Npad + i);
-            load_f(s + 1);
+            wn = slice_word(D, s + 1, ib, lane);
+            if constexpr (!INIT) load_f(s + 1);
         }
         uint32_t P[NPL];
 #pragma unroll
@@ -232,6 +230,17 @@ __global__ void __launch_bounds__(PZ_MAXT, KM <= 6 ? 3 : 2) k_z_admix_pk(const D
 #pragma unroll 1
         for (int g = 0; g < 4; ++g) {
             uint32_t Z = 0;
+            if constexpr (INIT) {
+#pragma unroll
+                for (int v = 0; v < 4; ++v) {
+                    const uint4 rb = Philox::round10(make_uint4(ST_INITADM, (uint32_t)(s * PZ_LC + 4 * g + v), (uint32_t)i, 0), key);
+                    // x mod K: the quotient from 2^32 / K rounded down is at most one short
+                    uint32_t za = rb.x - __umulhi(rb.x, modm) * K, zb = rb.y - __umulhi(rb.y, modm) * K;
+                    za = min(za, za - K);
+                    zb = min(zb, zb - K);
+                    Z = (((Z << 4) | za) << 4) | zb;
+                }
+            } else {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const uint4 rb = Philox::round10(make_uint4(ca, (uint32_t)s, (uint32_t)i, (uint32_t)(2 * g + h)), key);
@@ -275,10 +284,13 @@ __global__ void __launch_bounds__(PZ_MAXT, KM <= 6 ? 3 : 2) k_z_admix_pk(const D
                     }
                 }
             }
+            }
 #pragma unroll
             for (int b = 0; b < NPL; ++b) P[b] = (P[b] << 1) | ((Z >> b) & 0x11111111u);
         }
-        // the genotype words' planes, bit n = lane n's individual
+        // this lane's locus for the counts: its two genotype words' planes, bit
+        // n = lane n's individual
+        const uint32_t w0 = __shfl_sync(0xffffffffu, w, 2 * pl), w1 = __shfl_sync(0xffffffffu, w, 2 * pl + 1);
         const uint32_t LO = (w0 & 0x55555555u) | ((w1 << 1) & 0xAAAAAAAAu);
         const uint32_t HI = ((w0 >> 1) & 0x55555555u) | (w1 & 0xAAAAAAAAu);
         const uint32_t MS = (LO & HI) | ~lives;
@@ -297,7 +309,8 @@ __global__ void __launch_bounds__(PZ_MAXT, KM <= 6 ? 3 : 2) k_z_admix_pk(const D
             const uint32_t n = (uint32_t)__popc(mk & A0) | ((uint32_t)__popc(mk & A1) << 16);
             atomicAdd(&hs[buf][k][pl], n);
         }
-        if (s + 1 < s1) store_f(buf ^ 1);
+        if constexpr (!INIT)
+            if (s + 1 < s1) store_f(buf ^ 1);
         __syncthreads();
         unsigned long long* N2 = reinterpret_cast<unsigned long long*>(c.Ni);
         for (int j = threadIdx.x; j < PZ_LC * K; j += T) {
@@ -313,12 +326,14 @@ __global__ void __launch_bounds__(PZ_MAXT, KM <= 6 ? 3 : 2) k_z_admix_pk(const D
 #pragma unroll
         for (int k = 0; k < KM; ++k)
             if ((EXACT || k < K) && mi[k]) atomicAdd(&c.Mi[(int64_t)i * K + k], mi[k]);
-    const double t = block_sum((double)ls - (double)lc, sh);
-    if (threadIdx.x == 0) c.lnlp[vb.y * vb.gx + vb.x] = t;
+    if constexpr (!INIT) {
+        const double t = block_sum((double)ls - (double)lc, sh);
+        if (threadIdx.x == 0) c.lnlp[vb.y * vb.gx + vb.x] = t;
+    }
 }
 
-// The Metropolis log ratios (UpdateQMetro, src/structure.cpp:1006-1086) on the
-// sliced 2-bit genotypes: per individual the sum over its copies of
+// The Metropolis log ratios (UpdateQMetro, src/structure.cpp:1006-1086) on 2-bit
+// genotypes: per individual the sum over its copies of
 // ln(sum_k q'_k p / sum_k q_k p), one partial per locus range (grid.y) in
 // metrop. The staged table and packed FP32 operations of k_z_admix_pk give the
 // four weighted sums of a call. Their logarithms are not taken one by one: the
@@ -331,7 +346,7 @@ __global__ void __launch_bounds__(PZ_MAXT, KM <= 6 ? 3 : 2) k_z_admix_pk(const D
 // Issue-bound: N = 2,000 x L = 50,000, K = 5 593 -> 149 us a launch, N = 4,999 x
 // L = 40,009, K = 11 1,586 -> 535 us (against k_metro_ratio on the same calls).
 template <int KM, bool EXACT>
-__global__ void __launch_bounds__(PZ_MAXT, 2) k_metro_pk(const DevChain* chains, int force, const int4* map = nullptr) {
+__global__ void __launch_bounds__(PZ_MAXT, KM <= 11 ? 3 : 2) k_metro_pk(const DevChain* chains, int force, const int4* map = nullptr) {
     constexpr int CH = pz_chunks<KM>();
     constexpr int NF = (PZ_LC * KM + 127) / 128;
     __shared__ __align__(16) float2 sF[2][PZ_LC][4][CH * 2];
@@ -341,9 +356,10 @@ __global__ void __launch_bounds__(PZ_MAXT, 2) k_metro_pk(const DevChain* chains,
     const DevData& D = c.D;
     const int K = EXACT ? KM : c.K, m = c.ctl->m;
     if (!force && !metro_turn(c, m)) return;
-    const int T = blockDim.x, i = vb.x * T + threadIdx.x;
+    const int T = blockDim.x, lane = threadIdx.x & 31, ib = vb.x * T + (threadIdx.x & ~31);
+    const int i = ib + (lane >> 1) + 16 * (lane & 1);
     const bool live = i < D.N;
-    const int Npad = (D.N + 31) & ~31;
+    const BitTranspose tr(lane);
     const int nsl = (int)((D.L + PZ_LC - 1) / PZ_LC);
     const int s0 = vb.y * c.pz_slices, s1 = min(nsl, s0 + c.pz_slices);
     if (s0 >= s1) return;
@@ -379,13 +395,13 @@ __global__ void __launch_bounds__(PZ_MAXT, 2) k_metro_pk(const DevChain* chains,
         return (int)(b >> 23) - 127;
     };
     stage(s0, 0);
-    uint32_t gn = i < Npad ? __ldg(D.gt + (int64_t)s0 * Npad + i) : 0xFFFFFFFFu;
+    uint32_t wn = slice_word(D, s0, ib, lane);
     __syncthreads();
     int buf = 0;
     for (int s = s0; s < s1; ++s, buf ^= 1) {
-        uint32_t gw = gn;
+        uint32_t gw = tr.codes(wn);
         if (s + 1 < s1) {
-            if (i < Npad) gn = __ldg(D.gt + (int64_t)(s + 1) * Npad + i);
+            wn = slice_word(D, s + 1, ib, lane);
             stage(s + 1, buf ^ 1);
         }
 #pragma unroll 4

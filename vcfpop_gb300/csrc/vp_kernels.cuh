@@ -19,7 +19,6 @@ struct DevData {
     int32_t popcontig;    // every population's individuals are consecutive
     int64_t L, KT, coprime;
     const uint32_t* g2;   // [L][Nw]
-    const uint32_t* gt;   // the same calls by slice of 16 loci and individual (k_build_slices), or null
     const uint8_t* gb;    // [L][N][vmax]
     const int32_t* k;
     const int64_t* off;
@@ -234,7 +233,7 @@ __global__ void k_init_admix_ref(const DevChain* chains) {
 // two global atomics per copy, left most of the chip idle: N = 2,000 x
 // L = 50,000, K = 5 took 4.10 ms, N = 1,500 x L = 8,000 of mixed ploidy, K = 8
 // 5.93 ms; now 0.80 and
-// 0.24 ms.
+// 0.24 ms (up to 16 clusters of 2-bit data: k_z_admix_pk, 0.31 ms).
 constexpr int IA_LC = 16, IA_T = 256;
 __global__ void __launch_bounds__(IA_T) k_init_admix_ctr(const DevChain* chains, int lc) {
     extern __shared__ int32_t ia_sm[];

@@ -370,7 +370,7 @@ size_t init_smem(const vp_chain* c) { return (size_t)c->P.K * (IA_LC * c->ctx->m
 #define VP_ZADM_EXACT(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12)
 #define VP_ZADM_PADDED(X) X(16) X(32) X(64)
 
-// chains whose per-copy draws run on the sliced 2-bit genotypes (k_z_admix_pk)
+// chains whose per-copy draws run on the 2-bit genotypes, copies in pairs (k_z_admix_pk)
 bool pz_form(bool packed2, const vp_params& P) {
     return packed2 && P.rng == VP_RNG_COUNTER && P.K <= PZ_MAXK;
 }
@@ -846,29 +846,6 @@ int chain_plan(const vp_ctx* x, const vp_params* P, vp_chain* c, size_t* bytes) 
 }
 }  // namespace
 
-// chains that draw a label per allele copy: admixture, or its burn-in
-static bool per_copy(const DevChain& h) { return h.admix || h.nadmburnin > 0; }
-static size_t slices_bytes(const vp_ctx* x) {
-    return (size_t)cdiv(x->L, PZ_LC) * ((x->N + 31) & ~31) * sizeof(uint32_t);
-}
-// the context's genotypes by slice, built on the first chain that needs them
-static int ensure_slices(vp_ctx* x) {
-    if (x->D.gt) return VP_OK;
-    void* p = nullptr;
-    const cudaError_t e = dev_alloc(&p, slices_bytes(x), x->device, x->stream);
-    if (e != cudaSuccess) {
-        vp_set_error("device allocation of %zu bytes for the sliced genotypes failed: %s", slices_bytes(x), cudaGetErrorString(e));
-        return VP_E_MEM;
-    }
-    x->allocs.push_back(p);
-    const int Npad = (x->N + 31) & ~31;
-    k_build_slices<<<dim3(cdiv(Npad, 256), (unsigned)std::min<int64_t>(cdiv(x->L, PZ_LC), 32768), 1), 256, 0, x->stream>>>(
-        x->D, (uint32_t*)p, Npad);
-    if (int rc = check_launch(x, "k_build_slices")) return rc;
-    x->D.gt = (const uint32_t*)p;
-    return VP_OK;
-}
-
 int64_t vp_request_bytes(const vp_dataset* ds, const vp_params* P, int nsm) {
     vp_ctx g;
     g.N = ds->N; g.S = ds->S; g.L = ds->L; g.KT = ds->KT; g.maxK = ds->maxK; g.maxploidy = ds->maxploidy;
@@ -882,7 +859,6 @@ int64_t vp_request_bytes(const vp_dataset* ds, const vp_params* P, int nsm) {
     data += r(ds->k.size() * 4) + r(ds->off.size() * 8) + r(ds->vt.size() * 8) + r(ds->popid.size() * 4) +
             r(ds->pop_ind0.size() * 4) + r(ds->pop_nind.size() * 4) + r(ds->totfreq.size() * 4) +
             r(ds->nhaplo.size() * 4) + (ds->perm.empty() ? 0 : r(ds->perm.size() * 4));
-    if (per_copy(c.h) && pz_form(ds->packed2, *P)) data += r(slices_bytes(&g));
     return data + (int64_t)chain;
 }
 
@@ -898,10 +874,6 @@ extern "C" int vp_chain_create(vp_ctx* x, const vp_params* P, vp_chain** out) {
     const int K = P->K, N = x->N;
     const int64_t L = x->L;
     DevChain& h = c->h;
-    if (per_copy(h) && pz_form(x->packed2, *P)) {
-        if ((prc = ensure_slices(x))) { delete c; return prc; }
-        h.D.gt = x->D.gt;
-    }
     cudaError_t e = dev_alloc(&c->mem, bytes, x->device, x->stream);
     if (e != cudaSuccess) {
         vp_set_error("device allocation of %zu bytes for chain state failed: %s", bytes, cudaGetErrorString(e));
@@ -938,6 +910,10 @@ extern "C" int vp_chain_create(vp_ctx* x, const vp_params* P, vp_chain** out) {
             if (P->rng == VP_RNG_REFERENCE) {
                 k_init_admix_ref<<<cdiv(L, 128), 128, 0, s>>>(c->d);
                 if ((rc = check_launch(x, "k_init_admix_ref"))) break;
+            } else if (pz_form(x->packed2, *P)) {
+                const int T = pz_threads(N);
+                k_z_admix_pk<PZ_MAXK, false, true><<<dim3(cdiv(N, T), cdiv(cdiv(L, PZ_LC), h.pz_slices), 1), T, 0, s>>>(c->d, 1);
+                if ((rc = check_launch(x, "k_z_admix_pk<init>"))) break;
             } else {
                 // about 16 CTAs' worth of locus ranges per SM
                 const int64_t nx = cdiv(N, IA_T), ny = std::max<int64_t>(1, (int64_t)x->nsm * 16 / nx);
