@@ -168,7 +168,11 @@ extern "C" int vp_dataset_prepare(const vp_input* in, vp_dataset** out) {
         }
     const int vmax = p2 ? 2 : in->vmax;
     auto* d = new vp_dataset();
-    d->N = N; d->S = in->n_pop; d->vmax = vmax; d->Nw = Nw; d->packed2 = p2;
+    d->N = N; d->S = in->n_pop; d->vmax = vmax; d->packed2 = p2;
+    // rows of whole 16-byte pieces (asynchronous copies and wide loads of them
+    // need that alignment), the words past the input's filled with missing codes
+    const int pitch = (Nw + 3) & ~3;
+    d->Nw = pitch;
 
     // 1. per input locus: pass flag (polymorphic in the loader's genotype
     //    table) and genotype-id width, from the table facts when given
@@ -214,13 +218,15 @@ extern "C" int vp_dataset_prepare(const vp_input* in, vp_dataset** out) {
     // 3. genotypes in sorted order, typed copies per individual
     d->vt.assign(N, 0);
     if (p2) {
-        d->g2.resize((size_t)L * Nw);
+        d->g2.resize((size_t)L * pitch);
         parallel_for(L, [&](int64_t l) {
-            memcpy(&d->g2[(size_t)l * Nw], in->packed2 + (size_t)d->order[l] * Nw, Nw * sizeof(uint32_t));
+            uint32_t* row = &d->g2[(size_t)l * pitch];
+            memcpy(row, in->packed2 + (size_t)d->order[l] * Nw, Nw * sizeof(uint32_t));
+            for (int w = Nw; w < pitch; ++w) row[w] = 0xFFFFFFFFu;
         });
         std::vector<int64_t> typed(N, 0);
         for (int64_t l = 0; l < L; ++l) {
-            const uint32_t* row = &d->g2[(size_t)l * Nw];
+            const uint32_t* row = &d->g2[(size_t)l * pitch];
             for (int i = 0; i < N; ++i) typed[i] += code_at(row, i) != 3;
         }
         for (int i = 0; i < N; ++i) d->vt[i] = 2 * typed[i];

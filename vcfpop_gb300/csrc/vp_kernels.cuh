@@ -13,6 +13,7 @@ constexpr int KG = 16;          // clusters per thread in the likelihood kernels
 constexpr int LL_BLOCK = 128;   // threads per CTA of the likelihood stream's FMA form
 constexpr int LT_BLOCK = 256;   // threads (= individuals) per CTA of its table form
 constexpr int SUB = 32;         // loci per FP32 sub-sum before folding into FP64
+constexpr double LL_UNIT = 1.0 / 16777216.0;   // the tensor-core likelihood's unit, 2^-24
 
 struct DevData {
     int32_t N, S, vmax, maxploidy, maxK, Nw, packed2;
@@ -36,12 +37,16 @@ struct Ctl {
     double r;
     double lnl;           // likelihood of the last sampled labels (no-admixture form)
     double fprop;         // UpdateF's proposal for the next cluster
+    int32_t err;          // a tensor-core kernel's wait ran out (0: none)
 };
 
 struct DevChain {
     DevData D;
     int32_t K, admix, locpriori, fmodel, nburnin, nreps, nthinning, nadmburnin, writelnl;
     int32_t metrofreq, inferalpha, diffalpha, uniformalpha, fsame, difflambda, rlen, rng, nchunk, lchunk;
+    // tensor-core likelihood (k_loglik_tc): rows of its digit table ltd (0: not
+    // used), stages per locus chunk, chunks
+    int32_t llnb, tcper, tcchunk;
     int32_t pz_slices, nmetro, nlnlp, kp, nsampblk, zadm_lc;
     int32_t ntrace;       // capacity of lnlTrace in records
     double lambda, alpha, stdalpha, maxalpha, alphapriora, alphapriorb, maxr, epsr, epseta, epsgamma;
@@ -49,6 +54,7 @@ struct DevChain {
     uint64_t seed;
     Ctl* ctl;
     float *Freq, *FreqM, *FreqA, *Q, *Qprop, *Di, *lt, *fbuf;
+    char* ltd;
     uint16_t* Z;
     int32_t *Mi, *Ni;
     int64_t* MiSum;
@@ -289,6 +295,42 @@ __device__ __forceinline__ float prior_of(const DevChain& c, int k, int64_t j) {
     if (!c.fmodel) return (float)c.Lambda[k];
     return c.FreqA[j] * (float)c.f[c.fsame ? 0 : k];
 }
+// a logarithm's seven base-32 digits in units of 2^-24 (k_loglik_tc): whole
+// numbers of at most 16 in magnitude, every step exact but the last rounding
+__device__ __forceinline__ void ln_digits(float w, float* d) {
+    float r = w * 16777216.f;
+#pragma unroll
+    for (int j = 6; j >= 0; --j) {
+        const float u = (float)(1u << (5 * j));
+        d[j] = rintf(r * (1.f / u));
+        r = __fmaf_rn(-d[j], u, r);
+    }
+}
+// two whole numbers of at most 16 as e4m3 bytes (the second in the low byte)
+__device__ __forceinline__ uint32_t e4m3x2(float hi, float lo) {
+    uint16_t r;
+    asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+// the digit table is the shared-memory image of k_loglik_tc's B stages: per 32
+// loci llnb rows (row 7 k + digit) of 64 bytes, 32 a half of the loci in the
+// builders' order (call j: byte 4 (2 (j / 8) + (j & 1)) + (j / 2 & 3) for allele
+// 1 and 16 on for allele 0), the 16-byte chunks of row r exchanged by r / 2 mod
+// 4 (the 64-byte swizzle)
+__device__ __forceinline__ void write_digits(const DevChain& c, int k, int64_t l, const float* p) {
+    float d0[7], d1[7];
+    ln_digits(ln_freq(p[0]), d0);
+    ln_digits(ln_freq(p[1]), d1);
+    char* t = c.ltd + (l >> 5) * (c.llnb * 64);
+    const int j = (int)(l & 15), h = (int)(l >> 4) & 1, in = 4 * (2 * (j >> 3) + (j & 1)) + ((j >> 1) & 3);
+#pragma unroll
+    for (int d = 0; d < 7; ++d) {
+        const int row = 7 * k + d, sw = (row >> 1) & 3;
+        const uint32_t v = e4m3x2(d1[d], d0[d]);
+        t[row * 64 + ((2 * h ^ sw) << 4) + in] = (char)(v >> 8);
+        t[row * 64 + (((2 * h + 1) ^ sw) << 4) + in] = (char)v;
+    }
+}
 __device__ __forceinline__ void write_lt(const DevChain& c, int k, int64_t l, const float* p, int k2) {
     const DevData& D = c.D;
     if (D.packed2) {
@@ -303,6 +345,12 @@ __device__ __forceinline__ void write_lt(const DevChain& c, int k, int64_t l, co
     }
 }
 
+// The likelihood of sweep m runs on the tensor cores where the chain has that
+// form, but on sweeps that Record reads: their lnP(D) keeps the FP32 stream, so
+// that what a run reports does not change with the form (the two differ by a
+// few 1e-9, the FP32 stream's own rounding); label draws do not tell.
+__device__ __forceinline__ bool ll_tc_at(const DevChain& c, int m) { return c.llnb && binaryq_at(c, m) && !record_at(c, m); }
+
 // rebuild the lookup table from Freq (after a host-side state import)
 __global__ void k_refresh_lt(const DevChain* chains) {
     const DevChain& c = chains[blockIdx.z];
@@ -311,7 +359,9 @@ __global__ void k_refresh_lt(const DevChain* chains) {
     if (kl >= (int64_t)c.K * D.L) return;
     int k = (int)(kl / D.L);
     int64_t l = kl % D.L;
-    write_lt(c, k, l, c.Freq + k * D.KT + D.off[l], D.k[l]);
+    const float* p = c.Freq + k * D.KT + D.off[l];
+    write_lt(c, k, l, p, D.k[l]);
+    if (c.llnb) write_digits(c, k, l, p);
 }
 
 // reference streams: 128 block streams RNG(seed + m*128 + b, SALT_UPDATEP),
@@ -376,7 +426,8 @@ __global__ void k_update_p_ctr(const DevChain* chains, const int4* map = nullptr
         for (int a = 0; a < k2; ++a) p[a] *= inv;
     }
     for (int a = 0; a < k2; ++a) c.Freq[j + a] = p[a];
-    write_lt(c, k, l, p, k2);
+    if (ll_tc_at(c, m)) write_digits(c, k, l, p);
+    else write_lt(c, k, l, p, k2);
 }
 
 // ---------------------------------------------------------------------------
@@ -447,7 +498,7 @@ __global__ void __launch_bounds__(LT_BLOCK, 3) k_loglik(const DevChain* chains, 
     const int kg0 = (vb.z % kgroups) * KC;
     const DevData& D = c.D;
     const int K = c.K;
-    if (!force && !binaryq_at(c, c.ctl->m)) return;
+    if (!force && (!binaryq_at(c, c.ctl->m) || ll_tc_at(c, c.ctl->m))) return;
     const int i0 = vb.x * LT_BLOCK;
     const int i = i0 + threadIdx.x;
     const int64_t l0 = (int64_t)vb.y * c.lchunk;
@@ -585,7 +636,7 @@ __global__ void __launch_bounds__(LL_BLOCK) k_loglik_fma(const DevChain* chains,
     const int kg0 = (vb.z % kgroups) * KC;
     const DevData& D = c.D;
     const int K = c.K;
-    if (!force && !binaryq_at(c, c.ctl->m)) return;
+    if (!force && (!binaryq_at(c, c.ctl->m) || ll_tc_at(c, c.ctl->m))) return;
     const int64_t l0 = (int64_t)vb.y * c.lchunk;
     const int64_t l1 = min(D.L, l0 + c.lchunk);
     if (l0 >= D.L) return;
@@ -759,13 +810,25 @@ __device__ double sample_warp(const DevChain& c, int i, int m, int lane) {
     // unrolled so that the loads are in flight together.
     const int lg = K <= 1 ? 0 : 32 - __clz(K - 1), step = lg < 5 ? 32 >> lg : 1;
     const int kk = lg < 5 ? lane & ((1 << lg) - 1) : lane;
+    const int ch0 = lg < 5 ? lane >> lg : 0;
+    if (ll_tc_at(c, m)) {
+        // the tensor-core form's partials: whole numbers of 2^-24
+        long long a = 0;
+        const long long* P = reinterpret_cast<const long long*>(c.LLp);
 #pragma unroll 8
-    for (int ch = lg < 5 ? lane >> lg : 0; ch < c.nchunk; ch += step) {
-        const double* p = c.LLp + ((int64_t)ch * N + i) * K;
-        if (kk < K) v0 += p[kk];
-        if (h1) v1 += p[k1];
+        for (int ch = ch0; ch < c.tcchunk; ch += step)
+            if (kk < K) a += P[((int64_t)ch * N + i) * K + kk];
+        for (int o = 1 << lg; o < 32; o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        v0 = (double)a * LL_UNIT;
+    } else {
+#pragma unroll 8
+        for (int ch = ch0; ch < c.nchunk; ch += step) {
+            const double* p = c.LLp + ((int64_t)ch * N + i) * K;
+            if (kk < K) v0 += p[kk];
+            if (h1) v1 += p[k1];
+        }
+        for (int o = 1 << lg; o < 32; o <<= 1) v0 += __shfl_xor_sync(0xffffffffu, v0, o);
     }
-    for (int o = 1 << lg; o < 32; o <<= 1) v0 += __shfl_xor_sync(0xffffffffu, v0, o);
     double* LL = c.LL + (int64_t)i * K;
     float* Q = c.Q + (int64_t)i * K;
     int32_t* Mi = c.Mi + (int64_t)i * K;

@@ -11,6 +11,7 @@
 #include "vp_kernels.cuh"
 #include "vp_admix.cuh"
 #include "vp_tc.cuh"
+#include "vp_plain_tc.cuh"
 
 using namespace vp;
 
@@ -143,6 +144,12 @@ struct TcBatch {
     int nsgrp = 0, sgrp_rows = 0;
 };
 
+#ifndef LL_TC_MINN
+#define LL_TC_MINN 512
+#define LL_TC_MINL 4096
+#define CT_TC_MINN 512
+#define CT_TC_MINL 8192
+#endif
 namespace {
 void free_batch(vp_ctx* x);
 int run_tc(vp_ctx* x, vp_chain** cs, int n, int nsweeps);
@@ -332,10 +339,40 @@ int64_t ll_chunks(bool fma, int kc, int kgroups, int32_t N, int64_t L, int nsm) 
     return nch;
 }
 
+// chains whose likelihood runs on the tensor cores (k_loglik_tc)
+bool ll_tc_form(const vp_ctx* x, const vp_params& P) {
+    return x->packed2 && !P.admix && P.rng == VP_RNG_COUNTER && P.K <= ptc::LL_TCK && P.nthinning > 1 && x->N >= LL_TC_MINN &&
+           x->L >= LL_TC_MINL;
+}
+// its locus chunks, in stages of 32 loci: whole waves of its CTAs (two per SM
+// up to 16 clusters), as few as keep a chunk's sums exact, at least four stages
+void ll_tc_chunks(DevChain& h, int32_t N, int64_t L, int nsm) {
+    const int64_t nst = cdiv(L, ptc::LL_LOCI), nbi = cdiv(N, ptc::LL_M), slots = (int64_t)nsm * (h.llnb <= 80 ? 2 : 1);
+    int64_t nch = 1;
+    for (int64_t w = 1;; ++w) {
+        nch = std::max<int64_t>(1, slots * w / nbi);
+        if (cdiv(nst, nch) <= ptc::LL_MAXST) break;
+    }
+    nch = std::min(nch, std::max<int64_t>(1, nst / 4));
+    const int64_t per = std::min<int64_t>(cdiv(nst, nch), ptc::LL_MAXST);
+    h.tcper = (int32_t)per;
+    h.tcchunk = (int32_t)cdiv(nst, per);
+}
+
 int launch_loglik(vp_chain* c, int force) {
     vp_ctx* x = c->ctx;
     prof_mark(x, true);
     struct End { vp_ctx* x; ~End() { prof_mark(x, false); } } end_{x};
+    if (c->h.llnb && !force) {
+        const dim3 g(cdiv(x->N, ptc::LL_M), c->h.tcchunk, 1);
+        switch (c->h.llnb) {
+            case 32: SL(c, ptc::k_loglik_tc<32>, (g), (ptc::LL_THREADS), 0, 0); break;
+            case 48: SL(c, ptc::k_loglik_tc<48>, (g), (ptc::LL_THREADS), 0, 0); break;
+            case 80: SL(c, ptc::k_loglik_tc<80>, (g), (ptc::LL_THREADS), 0, 0); break;
+            case 112: SL(c, ptc::k_loglik_tc<112>, (g), (ptc::LL_THREADS), 0, 0); break;
+            default: SL(c, ptc::k_loglik_tc<224>, (g), (ptc::LL_THREADS), 0, 0); break;
+        }
+    }
     if (c->ll_fma) {
         const dim3 g(cdiv(x->N, lf_individuals(c->kc)), c->h.nchunk, c->kgroups);
         switch (c->kc) {
@@ -471,12 +508,23 @@ void set_smem_limits(int device) {
 #undef VP_MP
 }
 
+// counts on the tensor cores (k_count_tc)
+bool count_tc_form(const vp_ctx* x, int K) {
+    return x->packed2 && K <= 32 && x->N >= CT_TC_MINN && x->L >= CT_TC_MINL;
+}
+
 // the no-admixture counts: from bit planes on 2-bit packed data with at
 // least 32 words per locus (N >= 512) when the masks of a cluster group fit in
 // shared memory, else the per-individual pass
 int launch_count(vp_chain* c, int force) {
     vp_ctx* x = c->ctx;
     const int K = c->P.K;
+    if (count_tc_form(x, K)) {
+        const dim3 g(cdiv(x->L, ptc::CT_M), 1, 1);
+        if (ptc::ct_rows(K) == 16) SL(c, ptc::k_count_tc<16>, (g), (ptc::CT_THREADS), 0, 1, force);
+        else SL(c, ptc::k_count_tc<32>, (g), (ptc::CT_THREADS), 0, 1, force);
+        return VP_OK;
+    }
     if (x->packed2) {
         const int kc = K <= 4 ? 4 : K <= 8 ? 8 : 16;
         const int kgroups = (K + kc - 1) / kc;
@@ -511,6 +559,8 @@ int launch_step(vp_chain* c, int step, int force) {
             else SL(c, k_update_p_ctr, (cdiv((int64_t)K * x->L, 256), 1, 1), (256), 0, 0);
             return VP_OK;
         case VP_STEP_LOGLIK: {
+            // the FP32 stream, whose table UpdateP leaves alone on tensor-core sweeps
+            if (c->h.llnb) LAUNCH(x, k_refresh_lt, (cdiv((int64_t)K * x->L, 256), 256, 0, x->stream), (c->d));
             int rc = launch_loglik(c, 1);
             if (rc) return rc;
             SL(c, k_sample_noadmix, (c->h.nsampblk, 1, 1), (SAMPLE_BLOCK), 0, 1, 1);
@@ -607,9 +657,22 @@ int ensure_counts(vp_chain* c) {
     return rc;
 }
 
-__global__ void k_set_plain(DevChain* dst, float* lt, double* LLp) {
+__global__ void k_set_plain(DevChain* dst, float* lt, char* ltd, double* LLp) {
     dst->lt = lt;
+    dst->ltd = ltd;
     dst->LLp = LLp;
+}
+
+// bytes of a chain's likelihood table (the per-genotype table of 2-bit data,
+// else ln p), of the tensor-core form's digit table and of the chunk partials
+static size_t lt_bytes_of(const vp_chain* c, const vp_ctx* x) {
+    return ((x->packed2 ? (size_t)x->L * 4 * c->h.kp : (size_t)c->P.K * x->KT) * 4 + 255) & ~(size_t)255;
+}
+static size_t ltd_bytes_of(const vp_chain* c, const vp_ctx* x) {
+    return c->h.llnb ? (size_t)cdiv(x->L, ptc::LL_LOCI) * c->h.llnb * 64 : 0;
+}
+static int64_t llp_count(const vp_chain* c, const vp_ctx* x) {
+    return (int64_t)std::max(c->h.nchunk, c->h.tcchunk) * x->N * c->P.K;
 }
 
 // the plain form's scratch of a chain made for a tensor-core batch, carved on
@@ -619,9 +682,8 @@ int ensure_plain(vp_chain* c) {
     if (!c->plain_lazy || c->plain_mem) return VP_OK;
     vp_ctx* x = c->ctx;
     DevChain& h = c->h;
-    const int64_t ltn = x->packed2 ? x->L * 4 * h.kp : (int64_t)c->P.K * x->KT;
-    const size_t lt_bytes = ((size_t)ltn * 4 + 255) & ~(size_t)255;
-    const size_t bytes = lt_bytes + (size_t)h.nchunk * x->N * c->P.K * 8;
+    const size_t lt_bytes = lt_bytes_of(c, x), ltd_bytes = (ltd_bytes_of(c, x) + 255) & ~(size_t)255;
+    const size_t bytes = lt_bytes + ltd_bytes + (size_t)llp_count(c, x) * 8;
     cudaError_t e = dev_alloc(&c->plain_mem, bytes, x->device, x->stream);
     if (e != cudaSuccess) {
         c->plain_mem = nullptr;
@@ -630,8 +692,9 @@ int ensure_plain(vp_chain* c) {
     }
     CK(cudaMemsetAsync(c->plain_mem, 0, bytes, x->stream));
     h.lt = (float*)c->plain_mem;
-    h.LLp = (double*)((char*)c->plain_mem + lt_bytes);
-    LAUNCH(x, k_set_plain, (1, 1, 0, x->stream), (c->d, h.lt, h.LLp));
+    h.ltd = (char*)c->plain_mem + lt_bytes;
+    h.LLp = (double*)((char*)c->plain_mem + lt_bytes + ltd_bytes);
+    LAUNCH(x, k_set_plain, (1, 1, 0, x->stream), (c->d, h.lt, h.ltd, h.LLp));
     LAUNCH(x, k_refresh_lt, (cdiv((int64_t)c->P.K * x->L, 256), 256, 0, x->stream), (c->d));
     return VP_OK;
 }
@@ -729,15 +792,14 @@ void chain_layout(Carve& cv, vp_chain* c, const vp_ctx* x) {
     DevChain& h = c->h;
     const vp_params* P = &c->P;
     const int K = P->K, N = x->N, S = x->S;
-    const int64_t L = x->L, KT = x->KT;
+    const int64_t KT = x->KT;
     const int64_t ntrace = h.ntrace;
-    const int64_t ltn = x->packed2 ? L * 4 * h.kp : (int64_t)K * KT;
     h.ctl = cv.take<Ctl>(1);
     h.rstate = cv.take<Rng64>(1);
     h.Freq = cv.take<float>(K * KT);
     h.FreqM = cv.take<float>(K * KT);
     h.FreqA = cv.take<float>(P->fmodel ? KT : 1);
-    h.lt = c->plain_lazy ? nullptr : cv.take<float>(ltn);
+    h.lt = c->plain_lazy ? nullptr : cv.take<float>((int64_t)(lt_bytes_of(c, x) / 4));
     h.Q = cv.take<float>((int64_t)N * K);
     h.Qprop = cv.take<float>((int64_t)N * K);
     h.Di = cv.take<float>((int64_t)S * K);
@@ -746,7 +808,8 @@ void chain_layout(Carve& cv, vp_chain* c, const vp_ctx* x) {
     h.Mi = cv.take<int32_t>((int64_t)N * K);
     h.Ni = cv.take<int32_t>(K * KT);
     h.MiSum = cv.take<int64_t>((int64_t)N * K);
-    h.LLp = c->plain_lazy ? nullptr : cv.take<double>((int64_t)h.nchunk * N * K);
+    h.ltd = c->plain_lazy ? nullptr : cv.take<char>((int64_t)ltd_bytes_of(c, x));
+    h.LLp = c->plain_lazy ? nullptr : cv.take<double>(llp_count(c, x));
     h.LL = cv.take<double>((int64_t)N * K);
     h.metro = cv.take<double>(N);
     // Metropolis partials: one per locus range of the per-copy kernels
@@ -805,6 +868,8 @@ int chain_plan(const vp_ctx* x, const vp_params* P, vp_chain* c, size_t* bytes) 
         h.lchunk = (int32_t)((L + nch - 1) / nch);
         h.nchunk = (int32_t)((L + h.lchunk - 1) / h.lchunk);
     }
+    h.llnb = ll_tc_form(x, *P) ? ptc::ll_rows(K) : 0;
+    if (h.llnb) ll_tc_chunks(h, N, L, x->nsm);
     h.kp = (K + 3) & ~3;
     h.nsampblk = (int32_t)cdiv(N, SAMPLE_BLOCK / 32);   // counter-stream sampling: a warp per individual
     {
@@ -1143,6 +1208,7 @@ extern "C" int vp_chain_sizes(vp_chain* c, vp_result* r) {
     CK(cudaStreamSynchronize(c->ctx->stream));
     Ctl ctl;
     CK(cudaMemcpy(&ctl, c->h.ctl, sizeof ctl, cudaMemcpyDeviceToHost));
+    if (ctl.err) { vp_set_error("a tensor-core kernel of this chain timed out (code %d): its results are void", ctl.err); return VP_E_CUDA; }
     r->nr = ctl.nr; r->nlnl = ctl.nlnl;
     return VP_OK;
 }
@@ -1259,8 +1325,9 @@ extern "C" int vp_chain_set(vp_chain* c, int32_t field, const void* host, size_t
         }
     }
     CK(cudaMemcpy(p, host, n, cudaMemcpyHostToDevice));
-    if (field == VP_F_FREQ && c->h.lt) {
-        // keep the likelihood lookup table in step with the frequencies
+    if ((field == VP_F_FREQ || (field == VP_F_M && c->h.llnb)) && c->h.lt) {
+        // keep the likelihood tables in step with the frequencies, and both of
+        // them filled whichever the new sweep index reads
         vp_ctx* x = c->ctx;
         k_refresh_lt<<<cdiv((int64_t)c->P.K * x->L, 256), 256, 0, x->stream>>>(c->d);
         rc = check_launch(x, "k_refresh_lt");
