@@ -54,7 +54,7 @@ struct DevChain {
     uint64_t seed;
     Ctl* ctl;
     float *Freq, *FreqM, *FreqA, *Q, *Qprop, *Di, *lt, *fbuf;
-    char* ltd;
+    char *ltd, *oh;       // digit table (k_loglik_tc), one-hot image of the labels (k_count_tc)
     uint16_t* Z;
     int32_t *Mi, *Ni;
     int64_t* MiSum;
@@ -452,6 +452,10 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool ok) 
 __device__ __forceinline__ void cp_async4(void* dst, const void* src, bool ok) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(src), "r"(ok ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async8(void* dst, const void* src, bool ok) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(ok ? 8 : 0) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>

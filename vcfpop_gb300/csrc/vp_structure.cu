@@ -144,12 +144,6 @@ struct TcBatch {
     int nsgrp = 0, sgrp_rows = 0;
 };
 
-#ifndef LL_TC_MINN
-#define LL_TC_MINN 512
-#define LL_TC_MINL 4096
-#define CT_TC_MINN 512
-#define CT_TC_MINL 8192
-#endif
 namespace {
 void free_batch(vp_ctx* x);
 int run_tc(vp_ctx* x, vp_chain** cs, int n, int nsweeps);
@@ -339,10 +333,16 @@ int64_t ll_chunks(bool fma, int kc, int kgroups, int32_t N, int64_t L, int nsm) 
     return nch;
 }
 
-// chains whose likelihood runs on the tensor cores (k_loglik_tc)
+// Chains whose likelihood runs on the tensor cores (k_loglik_tc) on sweeps that
+// Record does not read. A sweep's time with it against the FP32 stream, us: N =
+// 64, L = 1,000 31 / 41 (K = 6), 33 / 35 (K = 10); N = 512, L = 8,000 62 / 72,
+// 92 / 111; N = 3,000, L = 20,000 139 / 207 (K = 12), 258 / 445 (K = 32). Up to
+// four clusters, where the FP32 kernel is one wave of short chunks, it loses 2
+// us at small sizes (K = 3: N = 512, L = 2,000 39 / 37) and gains from about
+// 2^22 calls on (512 x 8,000 51 / 53, 2,048 x 30,000 74 / 98).
 bool ll_tc_form(const vp_ctx* x, const vp_params& P) {
-    return x->packed2 && !P.admix && P.rng == VP_RNG_COUNTER && P.K <= ptc::LL_TCK && P.nthinning > 1 && x->N >= LL_TC_MINN &&
-           x->L >= LL_TC_MINL;
+    return x->packed2 && !P.admix && P.rng == VP_RNG_COUNTER && P.K <= ptc::LL_TCK && P.nthinning > 1 &&
+           x->L >= 4 * ptc::LL_LOCI && (P.K > 4 || (int64_t)x->N * x->L >= 1 << 22);
 }
 // its locus chunks, in stages of 32 loci: whole waves of its CTAs (two per SM
 // up to 16 clusters), as few as keep a chunk's sums exact, at least four stages
@@ -508,9 +508,17 @@ void set_smem_limits(int device) {
 #undef VP_MP
 }
 
-// counts on the tensor cores (k_count_tc)
+// Counts on the tensor cores (k_onehot, k_count_tc). A sweep's time with them
+// against the kernels below, us at K = 3, 6, 10, 16: N = 64, L = 30,000 62 / 69,
+// 115 / 128, 140 / 161, 160 / 195; N = 256, L = 2,000 34 / 29, 47 / 45, 43 / 41,
+// 47 / 45; N = 512, L = 1,000 33 / 37, 45 / 51, 41 / 47, 43 / 51; N = 2,048, L =
+// 1,000 (eight CTAs) 40 / 36, 53 / 51, 47 / 49, 51 / 53, L = 8,000 58 / 64,
+// 75 / 84, 94 / 129, 117 / 160; K = 20, 32 at 3,000 x 20,000 294 / 401, 303 / 445.
+// So by calls, but for 512 to 1,024 individuals, where the bit-plane kernel's
+// fixed cost already applies and a CTA's walk over them is short.
 bool count_tc_form(const vp_ctx* x, int K) {
-    return x->packed2 && K <= 32 && x->N >= CT_TC_MINN && x->L >= CT_TC_MINL;
+    const int64_t calls = (int64_t)x->N * x->L;
+    return x->packed2 && K <= 32 && (x->N < 512 ? calls >= 1 << 21 : x->N <= 1024 || calls >= 1 << 22);
 }
 
 // the no-admixture counts: from bit planes on 2-bit packed data with at
@@ -520,6 +528,7 @@ int launch_count(vp_chain* c, int force) {
     vp_ctx* x = c->ctx;
     const int K = c->P.K;
     if (count_tc_form(x, K)) {
+        SL(c, ptc::k_onehot, (cdiv(x->N, ptc::CT_IND), 1, 1), (ptc::CT_IND), 0, 1, force);
         const dim3 g(cdiv(x->L, ptc::CT_M), 1, 1);
         if (ptc::ct_rows(K) == 16) SL(c, ptc::k_count_tc<16>, (g), (ptc::CT_THREADS), 0, 1, force);
         else SL(c, ptc::k_count_tc<32>, (g), (ptc::CT_THREADS), 0, 1, force);
@@ -810,6 +819,7 @@ void chain_layout(Carve& cv, vp_chain* c, const vp_ctx* x) {
     h.MiSum = cv.take<int64_t>((int64_t)N * K);
     h.ltd = c->plain_lazy ? nullptr : cv.take<char>((int64_t)ltd_bytes_of(c, x));
     h.LLp = c->plain_lazy ? nullptr : cv.take<double>(llp_count(c, x));
+    h.oh = cv.take<char>(count_tc_form(x, K) && !P->admix ? (int64_t)cdiv(N, ptc::CT_IND) * ptc::ct_rows(K) * (128 + 4) : 0);
     h.LL = cv.take<double>((int64_t)N * K);
     h.metro = cv.take<double>(N);
     // Metropolis partials: one per locus range of the per-copy kernels
