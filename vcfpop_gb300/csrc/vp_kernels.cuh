@@ -33,7 +33,10 @@ struct DevData {
 };
 
 struct Ctl {
-    int32_t m, nr, nlnl, done;     // done: blocks finished, for last-block reductions
+    int32_t m, nr, nlnl;
+    // blocks finished, for last-block reductions: of the kernels in line, and of
+    // the two steps that run beside them (launch_sweep)
+    int32_t done, done_alpha, done_f;
     double r;
     double lnl;           // likelihood of the last sampled labels (no-admixture form)
     double fprop;         // UpdateF's proposal for the next cluster
@@ -159,7 +162,7 @@ __global__ void k_init_state(const DevChain* chains) {
     if (c.locpriori)
         for (int64_t s = tid; s < D.S; s += nt) c.SumAlpha[s] = 0;
     for (int64_t j = tid; j < c.rlen; j += nt) c.rout[j] = 0;
-    if (tid == 0) { c.ctl->m = 0; c.ctl->nr = 0; c.ctl->nlnl = 0; c.ctl->done = 0; c.ctl->r = 1; c.ctl->lnl = 0; }
+    if (tid == 0) { c.ctl->m = 0; c.ctl->nr = 0; c.ctl->nlnl = 0; c.ctl->done = c.ctl->done_alpha = c.ctl->done_f = 0; c.ctl->r = 1; c.ctl->lnl = 0; }
 }
 
 // InitAdmix, single-label form (no admixture, no admixture burn-in):
@@ -760,11 +763,11 @@ __device__ __forceinline__ int polylog(double* ll, int K, double u01, bool ref, 
 // counter streams use one thread per individual, and the last block to finish
 // reduces the per-block likelihoods in a fixed order and rebuilds Di.
 constexpr int SAMPLE_BLOCK = 256;
-__device__ __forceinline__ bool last_block_done(Ctl* ctl, int nblocks) {
+__device__ __forceinline__ bool last_block_done(int32_t* done, int nblocks) {
     __shared__ int is_last;
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) is_last = atomicAdd(&ctl->done, 1) == nblocks - 1;
+    if (threadIdx.x == 0) is_last = atomicAdd(done, 1) == nblocks - 1;
     __syncthreads();
     if (is_last) __threadfence();
     return is_last;
@@ -914,7 +917,7 @@ __global__ void __launch_bounds__(SAMPLE_BLOCK) k_sample_noadmix(const DevChain*
         if (i < N) lnl = sample_warp(c, i, m, lane);
         double t = block_sum(lane == 0 ? lnl : 0.0, sh);
         if (threadIdx.x == 0) c.lnlp[vb.x] = t;
-        if (!last_block_done(c.ctl, vb.gx)) return;
+        if (!last_block_done(&c.ctl->done, vb.gx)) return;
         const double tot = block_sum_partials(c.lnlp, vb.gx, sh);
         if (threadIdx.x == 0) {
             c.ctl->lnl = tot;
@@ -1815,7 +1818,7 @@ __global__ void __launch_bounds__(UA_LPQ_T) k_update_alpha_ctr(const DevChain* c
         // a location's rows are consecutive: one block per location
         for (int sp = vb.x; sp < D.S; sp += vb.gx)
             column_ln_sums(c.Q + (int64_t)D.pop_ind0[sp] * K, D.pop_nind[sp], K, sh, c.red + sp * K);
-        if (!last_block_done(c.ctl, vb.gx)) return;
+        if (!last_block_done(&c.ctl->done_alpha, vb.gx)) return;
     } else {
         // per-block partials of a range of rows, added by the last block in order
         const int nseq = loc ? D.S * K : c.diffalpha ? K : 1;
@@ -1842,7 +1845,7 @@ __global__ void __launch_bounds__(UA_LPQ_T) k_update_alpha_ctr(const DevChain* c
                 part[vb.x] = v;
             }
         }
-        if (!last_block_done(c.ctl, vb.gx)) return;
+        if (!last_block_done(&c.ctl->done_alpha, vb.gx)) return;
         for (int s = t; s < nseq; s += UA_LPQ_T) {
             double v = 0;
 #pragma unroll 8
@@ -1850,7 +1853,7 @@ __global__ void __launch_bounds__(UA_LPQ_T) k_update_alpha_ctr(const DevChain* c
             c.red[s] = v;
         }
     }
-    if (t == 0) c.ctl->done = 0;
+    if (t == 0) c.ctl->done_alpha = 0;
     __syncthreads();
     if (loc) alpha_step_locprior(c, m);
     else if (c.diffalpha) alpha_step_diff(c, m);
@@ -2298,10 +2301,10 @@ __global__ void __launch_bounds__(UF_T) k_update_f(const DevChain* chains, int k
     }
     part = block_sum(part, sh);
     if (threadIdx.x == 0) c.fpart[vb.x] = part;
-    if (!last_block_done(c.ctl, vb.gx)) return;
+    if (!last_block_done(&c.ctl->done_f, vb.gx)) return;
     const double tot = block_sum_partials(c.fpart, vb.gx, sh);
     if (threadIdx.x) return;
-    c.ctl->done = 0;
+    c.ctl->done_f = 0;
     if (k) rng = *c.rstate;
     if (go) {
         const double Fo = c.F[k];
@@ -2424,7 +2427,7 @@ __global__ void k_record_sweep(const DevChain* chains, double* exact, const int4
             for (int64_t j = tid; j < (int64_t)c.K * D.KT; j += nt) c.FreqM[j] += c.Freq[j];
         }
     }
-    if (!last_block_done(c.ctl, vb.gx)) return;
+    if (!last_block_done(&c.ctl->done, vb.gx)) return;
     if (rec && exact) {
         const double t = block_sum_partials(exact + (int64_t)vb.z * vb.gx, vb.gx, sh);
         if (threadIdx.x == 0) c.ctl->lnl = t;

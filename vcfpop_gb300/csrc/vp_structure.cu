@@ -72,6 +72,8 @@ struct vp_ctx {
     // UpdateP blocks on an SM beside a contraction CTA (0, the default: one
     // pass; vp_tc_pipeline)
     int tc_pipeline = 0;
+    // where sweep launches go while a captured sweep is on a branch (null: stream)
+    cudaStream_t branch = nullptr;
     // branch streams and events of a captured sweep's fork and join
     std::vector<cudaStream_t> fork;
     std::vector<cudaEvent_t> fork_ev;
@@ -195,7 +197,7 @@ int sweep_launch(vp_chain* c, const void* fn, const char* name, dim3 g, dim3 b, 
     if (nint >= 1) args[k++] = (void*)&i0;
     if (nint >= 2) args[k++] = (void*)&i1;
     args[k++] = (void*)&map;
-    cudaLaunchKernel(fn, g, b, args, sm, x->stream);
+    cudaLaunchKernel(fn, g, b, args, sm, x->branch ? x->branch : x->stream);
     return check_launch(x, name);
 }
 #define SL(c, fn, g, b, sm, ...)                                                                   \
@@ -640,17 +642,94 @@ int launch_step(vp_chain* c, int step, int force) {
     return VP_E_ARG;
 }
 
+// branch streams and events of a context's captured sweeps, at its stream's priority
+int fork_resources(vp_ctx* x, int nstreams, int nevents) {
+    int priority = 0;
+    cudaStreamGetPriority(x->stream, &priority);
+    while ((int)x->fork.size() < nstreams) {
+        cudaStream_t f;
+        CK(cudaStreamCreateWithPriority(&f, cudaStreamNonBlocking, priority));
+        x->fork.push_back(f);
+    }
+    while ((int)x->fork_ev.size() < nevents) {
+        cudaEvent_t e;
+        CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        x->fork_ev.push_back(e);
+    }
+    return VP_OK;
+}
+
+// the launches made while it lives go to a branch that starts after what is
+// queued on the context's stream; join() makes the stream wait for it
+struct Branch {
+    vp_ctx* x;
+    int i;
+    bool on = false;
+    int open(vp_ctx* ctx, int idx) {
+        x = ctx;
+        i = idx;
+        CK(cudaEventRecord(x->fork_ev[2 * i], x->stream));
+        CK(cudaStreamWaitEvent(x->fork[i], x->fork_ev[2 * i], 0));
+        x->branch = x->fork[i];
+        on = true;
+        return VP_OK;
+    }
+    int close() {
+        x->branch = nullptr;
+        CK(cudaEventRecord(x->fork_ev[2 * i + 1], x->fork[i]));
+        return VP_OK;
+    }
+    int join() {
+        if (on) CK(cudaStreamWaitEvent(x->stream, x->fork_ev[2 * i + 1], 0));
+        return VP_OK;
+    }
+};
+
+// One sweep. Two groups of steps do not touch what the steps in line do until
+// Record: the F model's (UpdateA and UpdateF read the frequencies that UpdateP
+// drew), and the location prior's and alpha's (they read Q, the label draws of
+// UpdateQ and one another). Their FP64 chains keep few warps busy for tens of
+// us, so a captured sweep runs them as branches beside the label draws and the
+// counts (a cohort's merged launches stay in line). A run in line
+// and with branches: N = 300 x L = 3,000, K = 4, 120 sweeps 6.6 / 5.3 ms; the F
+// model at N = 600 x L = 6,000, 12 sweeps 2.65 / 2.07; the location prior, 21
+// sweeps, at N = 1,500 polyploids 9.9 / 8.3, without admixture at N = 3,001 3.4 / 3.0.
 int launch_sweep(vp_chain* c) {
-    static const int seq[] = {VP_STEP_UPDATEP, VP_STEP_UPDATEQ, VP_STEP_LOCPRIORI, VP_STEP_UPDATEZ, VP_STEP_ALPHA,
-                              VP_STEP_UPDATEA, VP_STEP_UPDATEF};
-    for (int st : seq) {
-        int rc = launch_step(c, st, 0);
+    vp_ctx* x = c->ctx;
+    const vp_params& P = c->P;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool side = !x->rec && P.rng == VP_RNG_COUNTER && cudaStreamIsCapturing(x->stream, &cap) == cudaSuccess &&
+                      cap == cudaStreamCaptureStatusActive;
+    const bool alpha = P.locpriori || (P.inferalpha && (P.admix || c->h.nadmburnin > 0));
+    Branch bf{}, ba{};
+    struct Reset { vp_ctx* x; ~Reset() { x->branch = nullptr; } } reset_{x};
+    auto steps = [&](std::initializer_list<int> seq) {
+        for (int st : seq)
+            if (int rc = launch_step(c, st, 0)) return rc;
+        return (int)VP_OK;
+    };
+    if (int rc = steps({VP_STEP_UPDATEP})) return rc;
+    if (side && P.fmodel) {
+        int rc = bf.open(x, 0);
+        if (!rc) rc = steps({VP_STEP_UPDATEA, VP_STEP_UPDATEF});
+        if (!rc) rc = bf.close();
         if (rc) return rc;
     }
+    if (int rc = steps({VP_STEP_UPDATEQ})) return rc;
+    if (side && alpha) {
+        int rc = ba.open(x, 1);
+        if (!rc) rc = steps({VP_STEP_LOCPRIORI, VP_STEP_ALPHA});
+        if (!rc) rc = ba.close();
+        if (!rc) rc = steps({VP_STEP_UPDATEZ});
+        if (rc) return rc;
+    } else if (int rc = steps({VP_STEP_LOCPRIORI, VP_STEP_UPDATEZ, VP_STEP_ALPHA})) return rc;
+    if (!bf.on)
+        if (int rc = steps({VP_STEP_UPDATEA, VP_STEP_UPDATEF})) return rc;
+    if (int rc = bf.join()) return rc;
+    if (int rc = ba.join()) return rc;
     // Record and m += 1 as one launch; at most 128 blocks: the element-wise
     // part only runs on recorded sweeps, and every block takes part in the
     // last-block count
-    vp_ctx* x = c->ctx;
     SL(c, k_record_sweep, (std::min<unsigned>(128, cdiv((int64_t)c->P.K * x->KT, 256)), 1, 1), (256), 0, -1);
     return VP_OK;
 }
@@ -1039,6 +1118,7 @@ static int capture_sweep(vp_chain** cs, int n, cudaGraphExec_t* exec, int* nodes
     cudaGraph_t g;
     x->prof_next = 0;
     x->prof_used = 0;
+    if (int rc0 = fork_resources(x, 2, 4)) return rc0;
     CK(cudaStreamBeginCapture(x->stream, cudaStreamCaptureModeThreadLocal));
     int64_t before = x->launches;
     int rc = VP_OK;
@@ -2096,19 +2176,6 @@ unsigned updatep_blocks(const vp_ctx* x, int64_t nloci, int R) {
 }
 
 // branch streams and events for a sweep's fork and join
-int fork_resources(vp_ctx* x, int nstreams, int nevents) {
-    while ((int)x->fork.size() < nstreams) {
-        cudaStream_t f;
-        CK(cudaStreamCreateWithFlags(&f, cudaStreamNonBlocking));
-        x->fork.push_back(f);
-    }
-    while ((int)x->fork_ev.size() < nevents) {
-        cudaEvent_t e;
-        CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        x->fork_ev.push_back(e);
-    }
-    return VP_OK;
-}
 
 // dynamic shared memory of an UpdateP block that lets at most `share` of
 // them sit on an SM beside one CTA of the likelihood contraction (the
