@@ -1151,58 +1151,34 @@ __device__ __forceinline__ void dirichlet_ctr(Philox& p, float* q, const double*
     for (int k = 0; k < K; ++k) q[k] *= inv;
 }
 
-// UpdateQAdmix (src/structure.cpp:984-1004): Q_i ~ Dirichlet(alpha + Mi_i),
-// used by the admixture model and the no-admixture burn-in
+// UpdateQAdmix (src/structure.cpp:984-1004): Q_i ~ Dirichlet(alpha + Mi_i), used
+// by the admixture model and the no-admixture burn-in; on a Metropolis sweep
+// instead the proposals of UpdateQMetro (1006-1086), Q'_i ~ Dirichlet(alpha)
 __global__ void k_update_q_admix(const DevChain* chains, int force, const int4* map = nullptr) {
     const VBlock vb = vblock(map);
     const DevChain& c = chains[vb.z];
     if (map && run_over(c)) return;
     const DevData& D = c.D;
     const int K = c.K, m = c.ctl->m;
-    if (!force) {
-        if (c.admix && metro_turn(c, m)) return;
-        if (!c.admix && m >= c.nadmburnin) return;
-    }
+    const bool prop = !force && metro_turn(c, m);
+    if (!force && !c.admix && m >= c.nadmburnin) return;
+    float* Q = prop ? c.Qprop : c.Q;
     if (c.rng == 0) {
         if (vb.x || threadIdx.x) return;
         Rng64 r; r.init(c.seed + (uint64_t)m, VP_SALT_UPDATEQ);
         for (int i = 0; i < D.N; ++i)
             if (D.vt[i])
-                dirichlet_ref(r, c.Q + (int64_t)i * K, c.locpriori ? c.AlphaLocal + D.popid[i] * K : c.Alpha,
-                              c.Mi + (int64_t)i * K, K);
+                dirichlet_ref(r, Q + (int64_t)i * K, c.locpriori ? c.AlphaLocal + D.popid[i] * K : c.Alpha,
+                              prop ? nullptr : c.Mi + (int64_t)i * K, K);
+        if (prop) *c.rstate = r;  // the acceptance draws continue this stream
         return;
     }
     for (int i = vb.x * blockDim.x + threadIdx.x; i < D.N; i += vb.gx * blockDim.x) {
         if (!D.vt[i]) continue;
-        Philox p; p.init(c.seed, ST_Q | ((uint32_t)m << 4), (uint32_t)i, 1);
-        dirichlet_ctr(p, c.Q + (int64_t)i * K, c.locpriori ? c.AlphaLocal + D.popid[i] * K : c.Alpha,
-                      c.Mi + (int64_t)i * K, K);
-    }
-}
-
-// UpdateQMetro (src/structure.cpp:1006-1086): proposals Q'_i ~ Dirichlet(alpha)
-__global__ void k_metro_propose(const DevChain* chains, int force, const int4* map = nullptr) {
-    const VBlock vb = vblock(map);
-    const DevChain& c = chains[vb.z];
-    if (map && run_over(c)) return;
-    const DevData& D = c.D;
-    const int K = c.K, m = c.ctl->m;
-    if (!force && !metro_turn(c, m)) return;
-    if (c.rng == 0) {
-        if (vb.x || threadIdx.x) return;
-        Rng64 r; r.init(c.seed + (uint64_t)m, VP_SALT_UPDATEQ);
-        for (int i = 0; i < D.N; ++i)
-            if (D.vt[i])
-                dirichlet_ref(r, c.Qprop + (int64_t)i * K, c.locpriori ? c.AlphaLocal + D.popid[i] * K : c.Alpha,
-                              nullptr, K);
-        *c.rstate = r;  // the acceptance draws continue this stream
-        return;
-    }
-    for (int i = vb.x * blockDim.x + threadIdx.x; i < D.N; i += vb.gx * blockDim.x) {
-        if (!D.vt[i]) continue;
-        Philox p; p.init(c.seed, ST_METRO_P | ((uint32_t)m << 4), (uint32_t)i, 0);
-        dirichlet_ctr(p, c.Qprop + (int64_t)i * K, c.locpriori ? c.AlphaLocal + D.popid[i] * K : c.Alpha,
-                      nullptr, K);
+        Philox p;
+        p.init(c.seed, (prop ? ST_METRO_P : ST_Q) | ((uint32_t)m << 4), (uint32_t)i, prop ? 0u : 1u);
+        dirichlet_ctr(p, Q + (int64_t)i * K, c.locpriori ? c.AlphaLocal + D.popid[i] * K : c.Alpha,
+                      prop ? nullptr : c.Mi + (int64_t)i * K, K);
     }
 }
 
@@ -1218,15 +1194,33 @@ __global__ void k_metro_propose(const DevChain* chains, int force, const int4* m
 template <int KM, bool EXACT>
 __global__ void __launch_bounds__(256) k_metro_ratio(const DevChain* chains, int force, const int4* map = nullptr);
 
-// Acceptance of the proposals. Counter streams: a CTA takes MA_I individuals,
-// one per lane, and its warps share the locus ranges' partials (coalesced over
-// the individuals; one thread an individual walked all of them: N = 2,000,
-// K = 5 164 -> 20 us), added per warp, then over the warps in order.
-constexpr int MA_I = 32, MA_T = 256;
-__global__ void __launch_bounds__(MA_T) k_metro_accept(const DevChain* chains, int force, const int4* map = nullptr) {
+// Zero Mi and Ni ahead of the per-copy label draws
+__device__ __forceinline__ void zero_counts(const DevChain& c, const VBlock& vb) {
+    int64_t tid = vb.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)vb.gx * blockDim.x;
+    for (int64_t j = tid; j < (int64_t)c.D.N * c.K; j += nt) c.Mi[j] = 0;
+    for (int64_t j = tid; j < (int64_t)c.K * c.D.KT; j += nt) c.Ni[j] = 0;
+    for (int64_t j = tid; j < c.nlnlp; j += nt) c.lnlp[j] = 0;
+}
+__global__ void k_zero_counts(const DevChain* chains, int force, const int4* map = nullptr) {
     const VBlock vb = vblock(map);
     const DevChain& c = chains[vb.z];
     if (map && run_over(c)) return;
+    if (!force && binaryq_at(c, c.ctl->m)) return;
+    zero_counts(c, vb);
+}
+
+// Acceptance of the proposals. Counter streams: a CTA takes MA_I individuals,
+// one per lane, and its warps share the locus ranges' partials (coalesced over
+// the individuals; one thread an individual walked all of them: N = 2,000,
+// K = 5 164 -> 20 us), added per warp, then over the warps in order. In a sweep
+// the same launch zeroes the counts ahead of the label draws (zero): on nine
+// sweeps of ten it would have nothing else to do.
+constexpr int MA_I = 32, MA_T = 256;
+__global__ void __launch_bounds__(MA_T) k_metro_accept(const DevChain* chains, int force, int zero, const int4* map = nullptr) {
+    const VBlock vb = vblock(map);
+    const DevChain& c = chains[vb.z];
+    if (map && run_over(c)) return;
+    if (zero) zero_counts(c, vb);
     const DevData& D = c.D;
     const int K = c.K, m = c.ctl->m, nm = c.nmetro;
     if (!force && !metro_turn(c, m)) return;
@@ -1264,18 +1258,6 @@ __global__ void __launch_bounds__(MA_T) k_metro_accept(const DevChain* chains, i
     }
     if (acc)
         for (int k = 0; k < K; ++k) c.Q[(int64_t)i * K + k] = c.Qprop[(int64_t)i * K + k];
-}
-
-// Zero Mi and Ni ahead of the per-copy label draws
-__global__ void k_zero_counts(const DevChain* chains, int force, const int4* map = nullptr) {
-    const VBlock vb = vblock(map);
-    const DevChain& c = chains[vb.z];
-    if (map && run_over(c)) return;
-    if (!force && binaryq_at(c, c.ctl->m)) return;
-    int64_t tid = vb.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)vb.gx * blockDim.x;
-    for (int64_t j = tid; j < (int64_t)c.D.N * c.K; j += nt) c.Mi[j] = 0;
-    for (int64_t j = tid; j < (int64_t)c.K * c.D.KT; j += nt) c.Ni[j] = 0;
-    for (int64_t j = tid; j < c.nlnlp; j += nt) c.lnlp[j] = 0;
 }
 
 // Poly over float weights (src/statistics.cpp:357-385) with the reference's

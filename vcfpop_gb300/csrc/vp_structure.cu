@@ -559,7 +559,13 @@ unsigned f_blocks(const vp_ctx* x, const vp_params& P) {
     return (unsigned)std::min<int64_t>(cdiv((P.fsame ? P.K : 1) * x->KT, UF_T), (int64_t)x->nsm * 8);
 }
 
-int launch_step(vp_chain* c, int step, int force) {
+unsigned zero_blocks(const vp_chain* c) { return std::min<unsigned>(1024, cdiv((int64_t)c->P.K * c->ctx->KT, 256)); }
+// in a sweep (not a single step) the Metropolis acceptance also zeroes the counts
+bool accept_zeroes(const vp_chain* c, bool sweep) {
+    return sweep && c->P.admix && c->P.metrofreq > 0 && c->P.rng == VP_RNG_COUNTER;
+}
+
+int launch_step(vp_chain* c, int step, int force, bool sweep = false) {
     vp_ctx* x = c->ctx;
     const vp_params& P = c->P;
     const int K = P.K;
@@ -587,9 +593,10 @@ int launch_step(vp_chain* c, int step, int force) {
             } else {
                 SL(c, k_update_q_admix, (ref ? 1 : gi, 1, 1), (ref ? 32 : 256), 0, 1, 0);
                 if (P.metrofreq > 0) {
-                    SL(c, k_metro_propose, (ref ? 1 : gi, 1, 1), (ref ? 32 : 256), 0, 1, 0);
                     if (int rc = launch_metro_ratio(c, 0)) return rc;
-                    SL(c, k_metro_accept, (ref ? 1 : cdiv(x->N, MA_I), 1, 1), (ref ? 32 : MA_T), 0, 1, 0);
+                    const bool zero = accept_zeroes(c, sweep);
+                    const unsigned ga = std::max<unsigned>(cdiv(x->N, MA_I), zero ? zero_blocks(c) : 0);
+                    SL(c, k_metro_accept, (ref ? 1 : ga, 1, 1), (ref ? 32 : MA_T), 0, 2, 0, (int)zero);
                 }
             }
             return VP_OK;
@@ -601,7 +608,7 @@ int launch_step(vp_chain* c, int step, int force) {
             if (!P.admix)
                 if (int rc = launch_count(c, 0)) return rc;
             if (P.admix || c->h.nadmburnin > 0) {
-                SL(c, k_zero_counts, (std::min<unsigned>(1024, cdiv((int64_t)K * x->KT, 256)), 1, 1), (256), 0, 1, 0);
+                if (!accept_zeroes(c, sweep)) SL(c, k_zero_counts, (zero_blocks(c), 1, 1), (256), 0, 1, 0);
                 if (ref) SL(c, k_update_z_admix_ref, (cdiv(x->L, 128), 1, 1), (128), 0, 1, 0);
                 else if (int rc = launch_zadm_ctr(c, 0)) return rc;
             }
@@ -705,7 +712,7 @@ int launch_sweep(vp_chain* c) {
     struct Reset { vp_ctx* x; ~Reset() { x->branch = nullptr; } } reset_{x};
     auto steps = [&](std::initializer_list<int> seq) {
         for (int st : seq)
-            if (int rc = launch_step(c, st, 0)) return rc;
+            if (int rc = launch_step(c, st, 0, true)) return rc;
         return (int)VP_OK;
     };
     if (int rc = steps({VP_STEP_UPDATEP})) return rc;
