@@ -1582,7 +1582,7 @@ __global__ void k_logprod_q(const DevChain* chains, const int4* map = nullptr) {
 // What is left is a chain of FP64 lgammas and logarithms on one block, so the
 // ones that do not wait for a decision are formed side by side and the
 // decisions, sums and random numbers are those of the serial step:
-//   one alpha    the four lgammas on four lanes;
+//   one alpha    the proposal and its four lgammas on the last warp, beside the sums;
 //   diffalpha    a cluster's proposal depends on the decisions before it only
 //                through the count of uniforms they took from the stream
 //                (at most one each), so the log ratio of every (cluster,
@@ -1594,13 +1594,14 @@ __global__ void k_logprod_q(const DevChain* chains, const int4* map = nullptr) {
 //                location with one lgamma a step (the other one is the
 //                previous step's).
 // With a launch of its own for the sums, one alpha took 11 + 20 us (N = 300,
-// K = 4), the location prior 13 + 105 us (20 locations, K = 8); now 25 and 65.
+// K = 4), the location prior 13 + 105 us (20 locations, K = 8); now 21 and 65.
 constexpr int LPQ_BLOCKS = 64, UA_LPQ_T = 256;
 __device__ __forceinline__ double ln_q(float q) { return q > 0.f ? (double)logf(q) : -709.0895657128241; }
 // out[k] = sum of ln of column k of the n rows at q: a thread keeps to one
 // column, the threads of a column are added in order
 __device__ void column_ln_sums(const float* q, int64_t n, int K, double* sh, double* out) {
-    const int t = threadIdx.x, T = UA_LPQ_T / K * K;
+    // (the last warp may be busy: it takes no column)
+    const int t = threadIdx.x, T = (UA_LPQ_T - 32) / K * K;
     double v = 0;
     if (t < T)
         for (int64_t j = t; j < n * K; j += T) v += ln_q(q[j]);
@@ -1613,22 +1614,37 @@ __device__ void column_ln_sums(const float* q, int64_t n, int K, double* sh, dou
     }
     __syncthreads();
 }
-__device__ void alpha_step_one(const DevChain& c, int m) {
-    const int K = c.K, N = c.D.N, lane = threadIdx.x;
-    if (lane >= 32) return;
+// one alpha: the proposal and its lgammas need no sums, so the last warp of
+// every block forms them while the others add (the block that finishes last
+// has them ready); the rest of the step is then an exponential
+struct AlphaOne {
+    double am, g[4];     // proposal; lgamma of K am, K ao, am, ao
+    Rng64 rng;
+};
+__device__ __forceinline__ bool alpha_one_in(const DevChain& c, double am) {
+    return !(am <= 0 || (am >= c.maxalpha && c.uniformalpha));
+}
+__device__ void alpha_one_prepare(const DevChain& c, int m, AlphaOne& a) {
+    const int K = c.K, lane = threadIdx.x & 31;
     Rng64 rng;
     rng.init(c.seed + (uint64_t)m, VP_SALT_UPDATEALPHA);
-    const double am = rng.normal(c.Alpha[0], c.stdalpha);
-    if (am <= 0 || (am >= c.maxalpha && c.uniformalpha)) return;
-    const double ao = c.Alpha[0], d = am - ao;
+    const double am = rng.normal(c.Alpha[0], c.stdalpha), ao = c.Alpha[0];
+    if (alpha_one_in(c, am) && lane < 4) a.g[lane] = lgamma((lane & 1 ? ao : am) * (lane & 2 ? 1.0 : (double)K));
+    if (lane == 0) {
+        a.am = am;
+        a.rng = rng;
+    }
+}
+__device__ void alpha_step_one(const DevChain& c, AlphaOne& a) {
+    const int K = c.K, N = c.D.N;
+    if (threadIdx.x >= 32 || !alpha_one_in(c, a.am)) return;
+    Rng64 rng = a.rng;
+    const double am = a.am, ao = c.Alpha[0], d = am - ao;
     double dlnL = c.uniformalpha ? 0 : ((c.alphapriora - 1) * ref_mylog(am / ao) + (ao - am) / c.alphapriorb);
-    const double lg = lgamma((lane & 1 ? ao : am) * (lane & 2 ? 1.0 : (double)K));
-    const double gkm = __shfl_sync(0xffffffffu, lg, 0), gko = __shfl_sync(0xffffffffu, lg, 1);
-    const double gm = __shfl_sync(0xffffffffu, lg, 2), go = __shfl_sync(0xffffffffu, lg, 3);
-    dlnL += d * c.red[0] + (gkm - gko - K * gm + K * go) * N;
+    dlnL += d * c.red[0] + (a.g[0] - a.g[1] - K * a.g[2] + K * a.g[3]) * N;
     __syncwarp();
     if (dlnL >= VP_NZERO || rng.uniform() < exp(dlnL))
-        for (int k = lane; k < K; k += 32) c.Alpha[k] = am;
+        for (int k = threadIdx.x; k < K; k += 32) c.Alpha[k] = am;
 }
 // the serial diffalpha step, one thread
 __device__ void alpha_step_diff_serial(const DevChain& c, Rng64& rng) {
@@ -1794,8 +1810,10 @@ __global__ void __launch_bounds__(UA_LPQ_T) k_update_alpha_ctr(const DevChain* c
     const int K = c.K, m = c.ctl->m, t = threadIdx.x;
     __shared__ double sh[UA_LPQ_T];
     __shared__ double col[64];
+    __shared__ AlphaOne one;
     const bool loc = c.locpriori && c.admix;
     if (!loc && !(c.inferalpha && (c.admix || m < c.nadmburnin))) return;
+    if (!loc && !c.diffalpha && t >= UA_LPQ_T - 32) alpha_one_prepare(c, m, one);
     if (loc && D.popcontig) {
         // a location's rows are consecutive: one block per location
         for (int sp = vb.x; sp < D.S; sp += vb.gx)
@@ -1839,7 +1857,7 @@ __global__ void __launch_bounds__(UA_LPQ_T) k_update_alpha_ctr(const DevChain* c
     __syncthreads();
     if (loc) alpha_step_locprior(c, m);
     else if (c.diffalpha) alpha_step_diff(c, m);
-    else alpha_step_one(c, m);
+    else alpha_step_one(c, one);
 }
 
 // UpdateAlpha, reference stream RNG(seed + m, SALT_UPDATEALPHA), on one thread
@@ -2244,13 +2262,10 @@ __global__ void __launch_bounds__(UA_T) k_update_a(const DevChain* chains, const
 // The stream is one xorshift sequence per sweep, whose state waits in rstate
 // between launches. Bound by the latency of the FP64 chains (two lgammas and a
 // logarithm an allele, then the decision's on one thread); one block for all of
-// it took 2,000 us at KT = 12,000, K = 4, now 12-32 us a launch (two lanes an
-// allele, an lgamma each: 12-31).
-constexpr int UF_T = 128;
-__device__ __forceinline__ void f_propose(const DevChain& c, Rng64& rng, int k) {
-    c.ctl->fprop = rng.normal(c.F[k], c.stdf);
-    *c.rstate = rng;
-}
+// it took 2,000 us at KT = 12,000, K = 4, a launch per cluster with the decision's
+// terms after the sum 12 (out of bounds) to 32 us, beside it 11 to 26.
+constexpr int UF_T = 160;      // four warps for the alleles, one for the decision's terms
+constexpr int UF_A = UF_T - 32;
 __global__ void __launch_bounds__(UF_T) k_update_f(const DevChain* chains, int k, const int4* map = nullptr) {
     const VBlock vb = vblock(map);
     const DevChain& c = chains[vb.z];
@@ -2259,26 +2274,45 @@ __global__ void __launch_bounds__(UF_T) k_update_f(const DevChain* chains, int k
     const DevData& D = c.D;
     const int K = c.K, m = c.ctl->m;
     __shared__ double sh[32];
-    __shared__ double s_Fm;
+    __shared__ double s_Fm, s_lg[2], s_log, s_next[2], s_u;
+    __shared__ Rng64 s_rng[2];
     Rng64 rng;
     if (threadIdx.x == 0) {
         if (k == 0) {   // every block draws the first proposal for itself
             rng.init(c.seed + (uint64_t)m, VP_SALT_UPDATEF);
             s_Fm = rng.normal(c.F[0], c.stdf);
         } else {
+            rng = *c.rstate;
             s_Fm = c.ctl->fprop;
         }
+        s_rng[0] = rng;
     }
     __syncthreads();
     const double Fm = s_Fm, fm = (1 - Fm) / Fm, fo = c.f[k];
     const bool go = !(Fm < 0 || Fm > 1);
     double part = 0;
-    if (go) {
-        const int64_t n = (c.fsame ? K : 1) * D.KT;
-        const float* p = c.Freq + k * D.KT;
-        for (int64_t e = vb.x * (int64_t)UF_T + threadIdx.x; e < n; e += (int64_t)vb.gx * UF_T) {
-            const float pa2 = c.FreqA[e % D.KT];
-            part += pa2 * (fm - fo) * ref_mylog(p[e]) + lgamma(fo * pa2) - lgamma(fm * pa2);
+    if (threadIdx.x < UF_A) {
+        if (go) {
+            const int64_t n = (c.fsame ? K : 1) * D.KT;
+            const float* p = c.Freq + k * D.KT;
+            for (int64_t e = vb.x * (int64_t)UF_A + threadIdx.x; e < n; e += (int64_t)vb.gx * UF_A) {
+                const float pa2 = c.FreqA[e % D.KT];
+                part += pa2 * (fm - fo) * ref_mylog(p[e]) + lgamma(fo * pa2) - lgamma(fm * pa2);
+            }
+        }
+    } else {
+        // what the decision needs beside the sum, a lane each: two lgammas and a
+        // logarithm, and the next cluster's proposal from the stream as it
+        // stands and after the uniform that the decision may take
+        const int j = threadIdx.x - UF_A;
+        if (go && j < 2) s_lg[j] = lgamma(j ? fo : fm);
+        if (go && j == 2) s_log = ref_mylog(Fm / c.F[k]);
+        if (j == 3 || j == 4) {
+            Rng64 r = s_rng[0];
+            if (j == 4) s_u = r.uniform();
+            if (!c.fsame && k + 1 < K) s_next[j - 3] = r.normal(c.F[k + 1], c.stdf);
+            __syncwarp(3u << 3);
+            s_rng[j - 3] = r;
         }
     }
     part = block_sum(part, sh);
@@ -2287,19 +2321,23 @@ __global__ void __launch_bounds__(UF_T) k_update_f(const DevChain* chains, int k
     const double tot = block_sum_partials(c.fpart, vb.gx, sh);
     if (threadIdx.x) return;
     c.ctl->done_f = 0;
-    if (k) rng = *c.rstate;
+    int taken = 0;
     if (go) {
         const double Fo = c.F[k];
         double dlnL = c.pmeanf * (Fo - Fm) / (c.pstdf * c.pstdf) +
-                      (c.pmeanf * c.pmeanf / (c.pstdf * c.pstdf) - 1) * ref_mylog(Fm / Fo) +
-                      (c.fsame ? K : 1) * D.L * (lgamma(fm) - lgamma(fo));
+                      (c.pmeanf * c.pmeanf / (c.pstdf * c.pstdf) - 1) * s_log +
+                      (c.fsame ? K : 1) * D.L * (s_lg[0] - s_lg[1]);
         dlnL += tot;
-        if (dlnL >= VP_NZERO || rng.uniform() < exp(dlnL)) {
-            if (c.fsame) for (int j = 0; j < K; ++j) { c.F[j] = Fm; c.f[j] = fm; }
+        taken = !(dlnL >= VP_NZERO);
+        if (!taken || s_u < exp(dlnL)) {
+            if (c.fsame) for (int i = 0; i < K; ++i) { c.F[i] = Fm; c.f[i] = fm; }
             else { c.F[k] = Fm; c.f[k] = fm; }
         }
     }
-    if (!c.fsame && k + 1 < K) f_propose(c, rng, k + 1);
+    if (!c.fsame && k + 1 < K) {
+        c.ctl->fprop = s_next[taken];
+        *c.rstate = s_rng[taken];
+    }
 }
 
 // Record (src/structure.cpp:1941-2045): likelihood trace, running sums of the

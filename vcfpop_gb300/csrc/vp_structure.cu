@@ -556,7 +556,7 @@ int launch_count(vp_chain* c, int force) {
 
 // blocks of an UpdateF launch: one allele a thread up to 8 blocks per SM
 unsigned f_blocks(const vp_ctx* x, const vp_params& P) {
-    return (unsigned)std::min<int64_t>(cdiv((P.fsame ? P.K : 1) * x->KT, UF_T), (int64_t)x->nsm * 8);
+    return (unsigned)std::min<int64_t>(cdiv((P.fsame ? P.K : 1) * x->KT, UF_A), (int64_t)x->nsm * 8);
 }
 
 unsigned zero_blocks(const vp_chain* c) { return std::min<unsigned>(1024, cdiv((int64_t)c->P.K * c->ctx->KT, 256)); }
