@@ -1,5 +1,6 @@
 // Internal types shared by the host translation units of the library.
 #pragma once
+#include <cuda_runtime.h>
 #include <stdint.h>
 
 #include <atomic>
@@ -54,6 +55,9 @@ int64_t vp_request_bytes(const vp_dataset* ds, const vp_params* P, int nsm);
 // vp_open with the context's stream at a CUDA stream priority (lower numbers
 // run first; 0 is the default)
 int vp_open_ex(const vp_dataset* ds, int device, int priority, vp_ctx** out);
+// device memory from the library's pool, which keeps freed blocks for the next
+// call (freed with cudaFreeAsync; vp_release_memory gives the kept blocks back)
+cudaError_t vp_pool_alloc(void** p, size_t bytes, int device, cudaStream_t s);
 // one more reference to a dataset; vp_dataset_free drops one
 void vp_dataset_retain(const vp_dataset* ds);
 // vp_finish without the final wait

@@ -794,6 +794,8 @@ int ensure_plain(vp_chain* c) {
     return VP_OK;
 }
 
+cudaError_t vp_pool_alloc(void** p, size_t bytes, int device, cudaStream_t s) { return dev_alloc(p, bytes, device, s); }
+
 extern "C" int vp_open(const vp_dataset* ds, int device, vp_ctx** out) { return vp_open_ex(ds, device, 0, out); }
 
 int vp_open_ex(const vp_dataset* ds, int device, int priority, vp_ctx** out) {
