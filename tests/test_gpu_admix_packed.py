@@ -96,3 +96,26 @@ def test_initial_labels(N, L, K, poly):
     assert np.array_equal(c.get("NI").reshape(K, -1), Ni)
     c.close()
     ctx.close()
+
+
+# the byte layout's kernel over its call widths (1 to 16 bytes), ploidies and
+# cluster counts: every copy counted once, in its individual and its allele
+@pytest.mark.parametrize("ploidy,alleles", [((1,), 3), ((2,), 5), ((3, 4), 2), ((2, 4, 6), 8), ((8,), 4), ((2, 10), 6)])
+@pytest.mark.parametrize("K", [1, 5, 13, 17])
+def test_byte_layout_counts(ploidy, alleles, K):
+    rng = np.random.default_rng(K + len(ploidy))
+    N, L = 290, 37
+    pl = np.resize(np.array(ploidy, np.int32), N)
+    d = synth.fmodel(K, N, L, 3, 0.1, 0.1, admix_alpha=0.5, ploidy=pl, n_alleles=rng.integers(2, alleles + 1, L))
+    ds = S.Dataset.from_synth(d, packed=False)
+    ctx = S.Context(ds)
+    c = S.Chain(ctx, S.params(K, 5, admix=1))
+    c.run(3)
+    G, k = d["G"][ds.order()], d["k"][ds.order()]
+    ni = c.get("NI").reshape(K, -1).sum(0)
+    off = np.concatenate([[0], np.cumsum(k)])
+    for l in range(ds.L):
+        assert np.array_equal(ni[off[l]:off[l + 1]], [(G[l] == a).sum() for a in range(k[l])])
+    assert np.array_equal(c.get("MI").reshape(N, K).sum(1), (G >= 0).sum((0, 2)))
+    c.close()
+    ctx.close()

@@ -443,4 +443,159 @@ __global__ void __launch_bounds__(PZ_MAXT, KM <= 11 ? 3 : 2) k_metro_pk(const De
         c.metrop[(int64_t)vb.y * D.N + i] = (double)ex * 0.693147180559945309 + (double)logf(R1 / R0) + (double)single;
 }
 
+// Label draws per copy of the byte layout (any ploidy and allele count), up to
+// 16 clusters, on the same streams and with the same operations a copy as
+// k_update_z_admix_ctr: one lane per individual (in ascending ploidy with mixed
+// ploidy), 256 individuals per CTA. A call is one aligned load; the staged
+// frequencies of an allele are whole 16-byte chunks, an odd count, so that a
+// copy's weights take a quarter of the loads; the label is the number of
+// thresholds that the uniform reaches, its count goes to the lane's own column
+// of a shared array and to the slice's shared histogram. The Philox block is
+// formed when the warp's draw index enters it (mixed ploidy skips some).
+// N = 1,500 x L = 8,000, ploidy 2, 4 and 6, 2-8 alleles, K = 8: 295 -> 254 us.
+// Issue-bound (64% active, about 140 instructions a warp and copy); loading the
+// calls four loci ahead or taking 16 to 64 CTAs per SM made no difference.
+constexpr int ZG_T = 256, ZG_G = 4;
+static_assert(ZA_LC % ZG_G == 0, "whole groups a slice");
+__host__ __device__ constexpr int zg_stride(int km) { return 4 * (((km + 3) / 4) | 1); }   // floats of an allele's row
+template <int KM, bool EXACT, bool WIDE = false>
+__global__ void __launch_bounds__(ZG_T, KM <= 8 ? 3 : 2) k_z_admix_gen(const DevChain* chains, int force, const int4* map = nullptr) {
+    constexpr int FS = zg_stride(KM);
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const VBlock vb = vblock(map);
+    const DevChain& c = chains[vb.z];
+    if (map && run_over(c)) return;
+    const DevData& D = c.D;
+    const int K = EXACT ? KM : c.K, m = c.ctl->m, MK = D.maxK;
+    if (!force && binaryq_at(c, m)) return;
+    __shared__ double sh[32];
+    const int nbins = K * MK, t = threadIdx.x, vmax = D.vmax;
+    float* sF = reinterpret_cast<float*>(smraw);                                 // [ZA_LC][MK][FS]
+    int32_t* hs = reinterpret_cast<int32_t*>(sF + ZA_LC * MK * FS);              // [ZA_LC][K][MK]
+    int32_t* ms = hs + ZA_LC * nbins + t;                                        // [K][ZG_T]
+    const int slot = vb.x * ZG_T + t;
+    const bool live = slot < D.N;
+    const int i = live && D.perm ? D.perm[slot] : slot;
+    float q[KM];
+#pragma unroll
+    for (int k = 0; k < KM; ++k) {
+        q[k] = (live && (EXACT || k < K)) ? c.Q[(int64_t)i * K + k] : 0.f;
+        if (EXACT || k < K) ms[k * ZG_T] = 0;
+    }
+    const int64_t lb0 = (int64_t)vb.y * c.zadm_lc, lb1 = min(D.L, lb0 + c.zadm_lc);
+    float ls = 0.f, lc = 0.f;  // Kahan sum of ln(sum_k q_k p)
+    const bool rec = force || record_at(c, m);
+    const float minf = (float)VP_MIN_FREQ, kmin = (float)(VP_MIN_FREQ * K);
+    const uint2 key = make_uint2((uint32_t)c.seed, (uint32_t)(c.seed >> 32));
+    const uint32_t ca = ST_ZSLICE | ((uint32_t)m << 4);
+    // a call's bytes: copy a in byte a, 0xFF past the last one (WIDE: 16 bytes)
+    const uint8_t* gp = D.gb + (size_t)i * D.vstr;
+    const size_t row = (size_t)D.N * D.vstr;
+    auto call = [&](int64_t l, uint64_t& lo, uint64_t& hi) {
+        lo = hi = ~0ull;
+        if (!live || l >= lb1) return;
+        const uint8_t* g = gp + l * row;
+        if constexpr (WIDE) {
+            const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2*>(g));
+            lo = v.x;
+            hi = v.y;
+        } else if (D.vstr == 8) {
+            lo = __ldg(reinterpret_cast<const unsigned long long*>(g));
+        } else if (D.vstr == 4) {
+            lo = 0xFFFFFFFF00000000ull | __ldg(reinterpret_cast<const uint32_t*>(g));
+        } else if (D.vstr == 2) {
+            lo = 0xFFFFFFFFFFFF0000ull | __ldg(reinterpret_cast<const uint16_t*>(g));
+        } else {
+            lo = 0xFFFFFFFFFFFFFF00ull | __ldg(g);
+        }
+    };
+    // the calls of ZG_G loci are loaded while the ones before are drawn
+    uint64_t nlo[ZG_G], nhi[ZG_G];
+#pragma unroll
+    for (int u = 0; u < ZG_G; ++u) call(lb0 + u, nlo[u], nhi[u]);
+    for (int64_t l0 = lb0; l0 < lb1; l0 += ZA_LC) {
+        const int nl = (int)min((int64_t)ZA_LC, lb1 - l0);
+        __syncthreads();
+        for (int j = t; j < ZA_LC * MK * FS; j += ZG_T) {
+            const int k = j % FS, a = (j / FS) % MK, ll = j / (FS * MK);
+            float v = 0.f;
+            if (ll < nl && k < K && a < D.k[l0 + ll]) v = __ldg(c.Freq + (int64_t)k * D.KT + D.off[l0 + ll] + a);
+            sF[j] = v;
+        }
+        for (int j = t; j < ZA_LC * nbins; j += ZG_T) hs[j] = 0;
+        __syncthreads();
+        int block = -1;
+        uint4 rb = make_uint4(0, 0, 0, 0);
+        for (int lg = 0; lg < nl; lg += ZG_G) {
+          uint64_t clo[ZG_G], chi[ZG_G];
+#pragma unroll
+          for (int u = 0; u < ZG_G; ++u) {
+            clo[u] = nlo[u];
+            chi[u] = nhi[u];
+            call(l0 + lg + ZG_G + u, nlo[u], nhi[u]);
+          }
+#pragma unroll
+          for (int u = 0; u < ZG_G; ++u) {
+            const int ll = lg + u;
+            if (ll >= nl) break;
+            const uint64_t lo = clo[u], hi = chi[u];
+            // allele indices are below 64: a copy past the last has its high bit set
+            const uint64_t e0 = lo & 0x8080808080808080ull, e1 = hi & 0x8080808080808080ull;
+            const int n = min(vmax, e0 ? (__ffsll((long long)e0) - 1) >> 3 : WIDE && e1 ? 8 + ((__ffsll((long long)e1) - 1) >> 3) : WIDE ? 16 : 8);
+            const int nw = (int)__reduce_max_sync(0xffffffffu, (unsigned)n);
+            float lacc = 0.f;
+            for (int a = 0; a < nw; ++a) {
+                const int pos = ll * vmax + a;
+                if ((pos >> 2) != block) {
+                    block = pos >> 2;
+                    rb = Philox::round10(make_uint4(ca, (uint32_t)(l0 / ZA_LC), (uint32_t)i, (uint32_t)block), key);
+                }
+                const uint32_t x = pos & 2 ? (pos & 1 ? rb.w : rb.z) : (pos & 1 ? rb.y : rb.x);
+                if (a < n) {
+                    const int al = (int)((!WIDE || a < 8 ? lo >> (8 * a) : hi >> (8 * (a - 8))) & 63u);
+                    const float4* f = reinterpret_cast<const float4*>(sF + (ll * MK + al) * FS);
+                    float sx = 0.f, pre[KM];
+#pragma unroll
+                    for (int k = 0; k < KM; k += 4) {
+                        const float4 v = f[k >> 2];
+                        sx = __fmaf_rn(q[k], v.x, sx);
+                        pre[k] = sx;
+                        if (k + 1 < KM) { sx = __fmaf_rn(q[k + 1], v.y, sx); pre[k + 1] = sx; }
+                        if (k + 2 < KM) { sx = __fmaf_rn(q[k + 2], v.z, sx); pre[k + 2] = sx; }
+                        if (k + 3 < KM) { sx = __fmaf_rn(q[k + 3], v.w, sx); pre[k + 3] = sx; }
+                    }
+                    if (rec) lacc += logf(sx);
+                    const float tt = Philox::to_uniformf(x) * (sx + kmin);
+                    int z = 0;
+#pragma unroll
+                    for (int k = 0; k < KM - 1; ++k)
+                        if ((EXACT || k < K - 1) && !(tt < __fmaf_rn((float)(k + 1), minf, pre[k]))) ++z;
+                    atomicAdd(&ms[z * ZG_T], 1);
+                    atomicAdd(&hs[ll * nbins + z * MK + al], 1);
+                }
+            }
+            const float y = lacc - lc, sum = ls + y;
+            lc = (sum - ls) - y;
+            ls = sum;
+          }
+        }
+        __syncthreads();
+        for (int j = t; j < nl * nbins; j += ZG_T) {
+            const int v = hs[j];
+            if (!v) continue;
+            const int a = j % MK, k = (j / MK) % K, ll = j / nbins;
+            atomicAdd(&c.Ni[(int64_t)k * D.KT + D.off[l0 + ll] + a], v);
+        }
+    }
+    if (live)
+#pragma unroll
+        for (int k = 0; k < KM; ++k)
+            if (EXACT || k < K) {
+                const int v = ms[k * ZG_T];
+                if (v) atomicAdd(&c.Mi[(int64_t)i * K + k], v);
+            }
+    const double tot = block_sum((double)ls - (double)lc, sh);
+    if (t == 0) c.lnlp[vb.y * vb.gx + vb.x] = tot;
+}
+
 }  // namespace vp

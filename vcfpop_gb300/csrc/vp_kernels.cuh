@@ -16,11 +16,11 @@ constexpr int SUB = 32;         // loci per FP32 sub-sum before folding into FP6
 constexpr double LL_UNIT = 1.0 / 16777216.0;   // the tensor-core likelihood's unit, 2^-24
 
 struct DevData {
-    int32_t N, S, vmax, maxploidy, maxK, Nw, packed2;
+    int32_t N, S, vmax, vstr, maxploidy, maxK, Nw, packed2;
     int32_t popcontig;    // every population's individuals are consecutive
     int64_t L, KT, coprime;
     const uint32_t* g2;   // [L][Nw]
-    const uint8_t* gb;    // [L][N][vmax]
+    const uint8_t* gb;    // [L][N][vstr], vstr a power of two
     const int32_t* k;
     const int64_t* off;
     const int64_t* vt;
@@ -204,7 +204,7 @@ __device__ __forceinline__ void load_copies(const DevData& D, int64_t l, int i, 
         cp.a[1] = code == 0 ? 0 : 1;
         return;
     }
-    const uint8_t* g = D.gb + ((size_t)l * D.N + i) * D.vmax;
+    const uint8_t* g = D.gb + ((size_t)l * D.N + i) * D.vstr;
     int n = 0;
     if (g[0] != 0xFF)
         for (; n < D.vmax && g[n] != 0xFF; ++n) cp.a[n] = g[n];
@@ -1313,19 +1313,14 @@ __global__ void k_update_z_admix_ref(const DevChain* chains, int force, const in
     if (threadIdx.x == 0) c.lnlp[vb.x] = t;
 }
 
-// UpdateZAdmix with counter streams. Warp = 32 individuals (one per lane),
-// CTA = 8 warps = 256 individuals; grid.y splits the loci into ranges that a
-// CTA walks in slices of ZA_LC loci. A lane keeps its individual's Q row and
-// its Mi counts in registers; the slice's frequencies are staged in shared
-// memory. With at most ZA_PACKED = 32 (cluster, allele) bins, one per lane,
-// the per-copy increments of Ni are reduced across the warp before they reach
-// the slice histogram in shared memory: each lane's bin becomes a 1 in one of
-// five 6-bit fields of a word and redux.sync adds the words of the 32 lanes
-// (one reduction per five bins), then lane j adds bin j; with more bins (multi-
-// allelic data) each copy adds to the shared histogram directly (measured
-// faster there than grouping lanes with __match_any_sync). The slice
-// histogram is flushed to Ni with one global atomic per non-zero entry. KM is
-// the cluster count rounded up to a compiled size; EXACT means K == KM.
+// UpdateZAdmix with counter streams, above 16 clusters (up to 16: k_z_admix_pk
+// and k_z_admix_gen). Warp = 32 individuals (one per lane), CTA = 8 warps = 256
+// individuals; grid.y splits the loci into ranges that a CTA walks in slices
+// of ZA_LC loci. A lane keeps its individual's Q row and its Mi counts in
+// registers; the slice's frequencies are staged in shared memory, and each
+// copy adds to the slice's shared histogram, which is flushed to Ni with one
+// global atomic per non-zero entry. KM is the cluster count rounded up to a
+// compiled size.
 // Uniforms: one Philox stream per (individual, slice of ZA_LC loci); every
 // locus takes vmax consecutive draws, used or not, so a block of four serves
 // two diploid loci and a missing call shifts nothing.
@@ -1333,24 +1328,20 @@ __global__ void k_update_z_admix_ref(const DevChain* chains, int force, const in
 // on sweeps that Record reads (thinning points) or when the step is forced.
 constexpr int ZA_WARPS = 8;
 constexpr int ZA_LC = 16;
-constexpr int ZA_PACKED = 32;   // lane j flushes bin j
-static_assert(ZA_PACKED <= 32, "one histogram bin per lane");
-template <int KM, bool EXACT>
+template <int KM>
 __global__ void __launch_bounds__(ZA_WARPS * 32) k_update_z_admix_ctr(const DevChain* chains, int force, const int4* map = nullptr) {
     extern __shared__ unsigned char smraw[];
     const VBlock vb = vblock(map);
     const DevChain& c = chains[vb.z];
     if (map && run_over(c)) return;
     const DevData& D = c.D;
-    const int K = EXACT ? KM : c.K, m = c.ctl->m, MK = D.maxK;
+    const int K = c.K, m = c.ctl->m, MK = D.maxK;
     if (!force && binaryq_at(c, m)) return;
     __shared__ double sh[32];
     const int KPAD = K | 1;                                       // odd stride: no bank conflicts
     const int nbins = K * MK;
-    const bool packed = nbins <= ZA_PACKED;
     float* sF = reinterpret_cast<float*>(smraw);                  // [ZA_LC][MK][KPAD]
     int32_t* hs = reinterpret_cast<int32_t*>(sF + ZA_LC * MK * KPAD);  // [ZA_LC][K][MK]
-    const int lane = threadIdx.x & 31;
     const int slot = vb.x * (ZA_WARPS * 32) + threadIdx.x;
     const bool live = slot < D.N;
     const int i = live && D.perm ? D.perm[slot] : slot;   // ascending ploidy with mixed ploidy
@@ -1359,7 +1350,7 @@ __global__ void __launch_bounds__(ZA_WARPS * 32) k_update_z_admix_ctr(const DevC
     float q[KM];
     int32_t mi[KM];
 #pragma unroll
-    for (int k = 0; k < KM; ++k) { q[k] = (live && (EXACT || k < K)) ? c.Q[(int64_t)i * K + k] : 0.f; mi[k] = 0; }
+    for (int k = 0; k < KM; ++k) { q[k] = (live && k < K) ? c.Q[(int64_t)i * K + k] : 0.f; mi[k] = 0; }
     const int64_t lb0 = (int64_t)vb.y * c.zadm_lc, lb1 = min(D.L, lb0 + c.zadm_lc);
     float ls = 0.f, lc = 0.f;  // Kahan sum of ln(sum_k q_k p)
     const bool rec = force || record_at(c, m);
@@ -1399,7 +1390,7 @@ __global__ void __launch_bounds__(ZA_WARPS * 32) k_update_z_admix_ctr(const DevC
                     float sx = 0.f, pre[KM];
 #pragma unroll
                     for (int k = 0; k < KM; ++k) {
-                        if (EXACT || k < K) sx = __fmaf_rn(q[k], f[k], sx);
+                        if (k < K) sx = __fmaf_rn(q[k], f[k], sx);
                         pre[k] = sx;
                     }
                     if (rec) lacc += logf(sx);
@@ -1411,7 +1402,7 @@ __global__ void __launch_bounds__(ZA_WARPS * 32) k_update_z_admix_ctr(const DevC
                     int k2 = K - 1;
 #pragma unroll
                     for (int k = KM - 1; k >= 0; --k)
-                        if ((EXACT || k < K) && t < __fmaf_rn((float)(k + 1), (float)VP_MIN_FREQ, pre[k])) k2 = k;
+                        if (k < K && t < __fmaf_rn((float)(k + 1), (float)VP_MIN_FREQ, pre[k])) k2 = k;
                     // this slice's label counts, 8 bits per cluster (at most
                     // ZA_LC x 10 copies per slice)
 #pragma unroll
@@ -1419,23 +1410,7 @@ __global__ void __launch_bounds__(ZA_WARPS * 32) k_update_z_admix_ctr(const DevC
                         if (w == (k2 >> 3)) pk[w] += 1ull << (8 * (k2 & 7));
                     key = k2 * MK + al;
                 }
-                if (packed) {
-                    // every lane of the warp takes part (a < vmax is warp-uniform)
-                    uint32_t mine = 0;
-#pragma unroll
-                    for (int w = 0; w < (ZA_PACKED + 4) / 5; ++w) {
-                        if (w * 5 >= nbins) break;
-                        const uint32_t v = (key >= 0 && key / 5 == w) ? 1u << (6 * (key % 5)) : 0u;
-                        const uint32_t sw = __reduce_add_sync(0xffffffffu, v);
-                        if (lane / 5 == w) mine = sw;
-                    }
-                    if (lane < nbins) {
-                        const int cnt = (int)((mine >> (6 * (lane % 5))) & 63u);
-                        if (cnt) atomicAdd(&hl[lane], cnt);
-                    }
-                } else if (act) {
-                    atomicAdd(&hl[key], 1);
-                }
+                if (act) atomicAdd(&hl[key], 1);
             }
             ph.skip(D.vmax - nw);
             float y = lacc - lc, tt = ls + y;
@@ -1455,7 +1430,7 @@ __global__ void __launch_bounds__(ZA_WARPS * 32) k_update_z_admix_ctr(const DevC
     if (live)
 #pragma unroll
         for (int k = 0; k < KM; ++k)
-            if ((EXACT || k < K) && mi[k]) atomicAdd(&c.Mi[(int64_t)i * K + k], mi[k]);
+            if (k < K && mi[k]) atomicAdd(&c.Mi[(int64_t)i * K + k], mi[k]);
     double t = block_sum((double)ls - (double)lc, sh);
     if (threadIdx.x == 0) c.lnlp[vb.y * vb.gx + vb.x] = t;
 }

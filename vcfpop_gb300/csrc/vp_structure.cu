@@ -403,6 +403,10 @@ size_t zadm_smem(const vp_chain* c) {
     const int K = c->P.K, MK = c->ctx->maxK;
     return (size_t)ZA_LC * MK * (K | 1) * 4 + (size_t)ZA_LC * K * MK * 4;
 }
+size_t zgen_smem(const vp_chain* c, int km) {
+    const size_t MK = c->ctx->maxK, K = c->P.K;
+    return ((size_t)ZA_LC * MK * zg_stride(km) + ZA_LC * K * MK + K * ZG_T) * 4;
+}
 size_t init_smem(const vp_chain* c) { return (size_t)c->P.K * (IA_LC * c->ctx->maxK + IA_T) * sizeof(int32_t); }
 // instantiations of the per-copy label kernel: exact cluster counts up to
 // 12, then padded sizes
@@ -431,21 +435,23 @@ int launch_zadm_ctr(vp_chain* c, int force) {
         SL(c, (k_z_admix_pk<PZ_MAXK, false>), (g), (T), 0, 1, force);
         return VP_OK;
     }
-    dim3 g(cdiv(x->N, ZA_WARPS * 32), cdiv(x->L, c->h.zadm_lc), 1);
-    size_t sm = zadm_smem(c);
+    const dim3 g(cdiv(x->N, ZA_WARPS * 32), cdiv(x->L, c->h.zadm_lc), 1);
+    static_assert(ZG_T == ZA_WARPS * 32, "one grid for both");
     prof_mark(x, true);
     struct End { vp_ctx* x; ~End() { prof_mark(x, false); } } end_{x};
     const int K = c->P.K;
+    if (K <= PZ_MAXK && x->D.vstr == 16) {
+        SL(c, (k_z_admix_gen<PZ_MAXK, false, true>), (g), (ZG_T), zgen_smem(c, PZ_MAXK), 1, force);
+        return VP_OK;
+    }
 #define VP_ZE(n) \
-    if (K == n) { SL(c, (k_update_z_admix_ctr<n, true>), (g), (ZA_WARPS * 32), sm, 1, force); return VP_OK; }
-#define VP_ZP(n) \
-    if (K <= n) { SL(c, (k_update_z_admix_ctr<n, false>), (g), (ZA_WARPS * 32), sm, 1, force); return VP_OK; }
+    if (K == n) { SL(c, (k_z_admix_gen<n, true>), (g), (ZG_T), zgen_smem(c, n), 1, force); return VP_OK; }
     VP_ZADM_EXACT(VP_ZE)
-    VP_ZADM_PADDED(VP_ZP)
 #undef VP_ZE
-#undef VP_ZP
-    vp_set_error("K = %d out of range", K);
-    return VP_E_ARG;
+    if (K <= PZ_MAXK) SL(c, (k_z_admix_gen<PZ_MAXK, false>), (g), (ZG_T), zgen_smem(c, PZ_MAXK), 1, force);
+    else if (K <= 32) SL(c, (k_update_z_admix_ctr<32>), (g), (ZA_WARPS * 32), zadm_smem(c), 1, force);
+    else SL(c, (k_update_z_admix_ctr<64>), (g), (ZA_WARPS * 32), zadm_smem(c), 1, force);
+    return VP_OK;
 }
 
 // the Metropolis ratio kernel on the same K instantiations as the label kernel
@@ -496,12 +502,13 @@ void set_smem_limits(int device) {
     cudaFuncSetAttribute(k_count_packed<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     cudaFuncSetAttribute(k_count_packed<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     cudaFuncSetAttribute(k_count_packed<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-#define VP_ZE(n) cudaFuncSetAttribute(k_update_z_admix_ctr<n, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-#define VP_ZP(n) cudaFuncSetAttribute(k_update_z_admix_ctr<n, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+#define VP_ZE(n) cudaFuncSetAttribute(k_z_admix_gen<n, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     VP_ZADM_EXACT(VP_ZE)
-    VP_ZADM_PADDED(VP_ZP)
 #undef VP_ZE
-#undef VP_ZP
+    cudaFuncSetAttribute(k_z_admix_gen<PZ_MAXK, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+    cudaFuncSetAttribute(k_z_admix_gen<PZ_MAXK, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+    cudaFuncSetAttribute(k_update_z_admix_ctr<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+    cudaFuncSetAttribute(k_update_z_admix_ctr<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
 #define VP_ME(n) cudaFuncSetAttribute(k_metro_ratio<n, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
 #define VP_MP(n) cudaFuncSetAttribute(k_metro_ratio<n, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     VP_ZADM_EXACT(VP_ME)
@@ -816,7 +823,7 @@ int vp_open_ex(const vp_dataset* ds, int device, int priority, vp_ctx** out) {
     x->N = ds->N; x->S = ds->S; x->L = ds->L; x->KT = ds->KT; x->maxK = ds->maxK; x->maxploidy = ds->maxploidy;
     x->packed2 = ds->packed2;
     DevData& D = x->D;
-    D.N = ds->N; D.S = ds->S; D.vmax = ds->vmax; D.maxploidy = ds->maxploidy; D.maxK = ds->maxK; D.Nw = ds->Nw;
+    D.N = ds->N; D.S = ds->S; D.vmax = ds->vmax; D.vstr = ds->vstr; D.maxploidy = ds->maxploidy; D.maxK = ds->maxK; D.Nw = ds->Nw;
     D.packed2 = ds->packed2; D.L = ds->L; D.KT = ds->KT; D.coprime = ds->coprime;
     D.popcontig = 1;
     for (int32_t sp = 0; sp < ds->S; ++sp)
