@@ -21,7 +21,8 @@ struct TcOperands {
     int bk8 = 128;            // e4m3 K elements per stage of the count contraction
     int64_t Apad = 0, Npad = 0;
     __nv_bfloat16* C = nullptr;   // [Npad][Apad] bf16 counts: the likelihood contraction's A
-    uint8_t* CT = nullptr;        // [Apad][Npad] e4m3 counts: the count contraction's A
+    uint8_t* CT = nullptr;        // [Apad][Npad] e4m3 counts: the count contraction's A (packed: [Apad / 2][Npad] e5m2)
+    tc::PackedCounts packed;
     float* logpbar = nullptr;
     double* Bc = nullptr;
     int* err = nullptr;
@@ -136,6 +137,7 @@ struct TcBatch {
     uint8_t* OH = nullptr;
     float* LLpart = nullptr;
     int32_t* NiAll = nullptr;
+    int32_t* nk = nullptr;    // [Rpad] cluster sizes (packed counts)
     CUtensorMap mapC1, mapWhi, mapWlo, mapOH;
     cudaGraphExec_t graph = nullptr;
     int graph_nodes = 0;
@@ -1826,7 +1828,11 @@ int tc_operands(vp_ctx* x) {
     const int64_t A = 2 * x->L;
     t.Apad = (A + 63) / 64 * 64;
     t.Npad = (x->N + 127) / 128 * 128;
-    const size_t cbytes = (size_t)t.Npad * t.Apad * 2, ctbytes = ((size_t)t.Npad * t.Apad + 255) / 256 * 256;
+    int32_t least = 2 * x->N;           // typed copies of the locus with most missing calls
+    for (int32_t nh : x->hold->nhaplo) least = std::min(least, nh);
+    t.packed = tc::PackedCounts::of(x->N, x->N - least / 2);
+    const int64_t ctrows = t.packed.shift ? t.Apad / 2 : t.Apad;
+    const size_t cbytes = (size_t)t.Npad * t.Apad * 2, ctbytes = ((size_t)t.Npad * ctrows + 255) / 256 * 256;
     // locus groups of the operand build (BUILD_TILES tiles of 64 loci each)
     const unsigned groups = cdiv(cdiv(x->L, 64), tc::BUILD_TILES);
     const size_t tail = t.Apad * 4 + t.Npad * 8 + 256 + (size_t)groups * t.Npad * 4;
@@ -1851,12 +1857,12 @@ int tc_operands(vp_ctx* x) {
         tc::k_allele_center<<<cdiv(x->L * 32, 256), 256, 0, x->stream>>>(x->D, t.logpbar);
         if ((rc = check_launch(x, "k_allele_center"))) break;
         tc::k_build_counts<<<dim3((unsigned)(t.Npad / 128), groups, 1), 256, 0, x->stream>>>(
-            x->D, t.C, t.CT, t.Apad, t.Npad, t.logpbar, part);
+            x->D, t.C, t.CT, t.Apad, t.Npad, t.logpbar, part, t.packed.shift ? t.packed.miss_byte() : 0u);
         if ((rc = check_launch(x, "k_build_counts"))) break;
         tc::k_center_sum<<<cdiv(x->N, 256), 256, 0, x->stream>>>(x->D, part, (int)groups, t.Npad, t.Bc);
         if ((rc = check_launch(x, "k_center_sum"))) break;
         if ((rc = make_map(&t.mapC, t.C, t.Npad, t.Apad, t.Apad, 128, t.bk))) break;
-        rc = make_map(&t.mapCT, t.CT, t.Apad, t.Npad, t.Npad, 128, t.bk8, 1);
+        rc = make_map(&t.mapCT, t.CT, ctrows, t.Npad, t.Npad, 128, t.bk8, 1);
     } while (0);
     if (rc) {
         // nothing keeps the operands: a later call starts over
@@ -2094,6 +2100,7 @@ int make_batch(vp_ctx* x, vp_chain** cs, int n, const TcChoice* force) {
         b->OH = cv.take<uint8_t>((int64_t)b->Rpad * t.Npad);
         b->LLpart = cv.take<float>((int64_t)b->splits * x->N * b->Rpad);
         b->NiAll = cv.take<int32_t>((int64_t)b->Rpad * x->KT);
+        b->nk = cv.take<int32_t>(b->Rpad);
     };
     lay(probe);
     cudaError_t e = dev_alloc(&b->mem, probe.off, x->device, x->stream);
@@ -2153,6 +2160,7 @@ int make_batch(vp_ctx* x, vp_chain** cs, int n, const TcChoice* force) {
     for (int i = 0; i < n; ++i) pending |= cs[i]->counts_pending;
     if (pending) {
         tc::BatchDev bd = batch_dev(x);
+        CK(cudaMemsetAsync(b->nk, 0, (size_t)b->Rpad * 4, x->stream));
         LAUNCH(x, tc::k_onehot_from_z, (dim3(cdiv(x->N, 256), n, 1), 256, 0, x->stream), (bd));
         if ((rc = launch_counts_gemm(x))) return rc;
         for (int i = 0; i < n; ++i) cs[i]->counts_pending = false;
@@ -2168,6 +2176,8 @@ tc::BatchDev batch_dev(vp_ctx* x) {
     d.Apad = x->tc.Apad; d.Npad = x->tc.Npad; d.Whi = b->Whi; d.Wlo = b->Wlo; d.OH = b->OH;
     d.logpbar = x->tc.logpbar; d.Bc = x->tc.Bc; d.LLpart = b->LLpart;
     d.sgrp = b->sgrp; d.sgrp_ld = b->sgrp_rows | 1;
+    d.one = x->tc.packed.shift ? tc::E5M2_ONE : tc::E4M3_ONE;
+    d.nk = b->nk;
     return d;
 }
 
@@ -2342,10 +2352,12 @@ int launch_counts_gemm(vp_ctx* x, int32_t* out) {
     const TcOperands& t = x->tc;
     {
         tc::GemmArgs g{};
-        g.M = (int)(2 * x->L); g.N = b->Rpad; g.kblocks = (int)(t.Npad / t.bk8); g.kb_per_split = g.kblocks;
+        const bool packed = t.packed.shift != 0;
+        g.M = (int)(packed ? x->L : 2 * x->L); g.N = b->Rpad; g.kblocks = (int)(t.Npad / t.bk8); g.kb_per_split = g.kblocks;
         g.BN = b->BN; g.piece = b->piece; g.nb = 1; g.mt = b->mt2; g.stages = b->cfg.st2; g.bk = t.bk8; g.esz = 1;
-        g.mode = 1; g.out_i = out ? out : b->NiAll; g.ldo = x->KT; g.err = t.err;
-        const unsigned mtiles = cdiv(t.Apad, 128 * b->mt2);
+        g.mode = packed ? 2 : 1; g.e5m2 = packed; g.miss_shift = t.packed.shift; g.nk = b->nk;
+        g.out_i = out ? out : b->NiAll; g.ldo = x->KT; g.err = t.err;
+        const unsigned mtiles = cdiv(packed ? t.Apad / 2 : t.Apad, 128 * b->mt2);
         g.group_major = b->cfg.gm2 && mtiles <= 65535;     // grid.y limit; otherwise row tiles on x
         const dim3 grid = g.group_major ? dim3(b->G, mtiles, 1) : dim3(mtiles, b->G, 1);
         return launch_gemm(x, t.mapCT, b->mapOH, b->mapOH, g, grid);
@@ -2501,6 +2513,7 @@ int tune_batch(vp_ctx* x, int effort, TcChoice* best, vp_tc_config* info) {
     // may come from per-copy draws that the labels do not give back)
     {
         tc::BatchDev bd = batch_dev(x);
+        CK(cudaMemsetAsync(b->nk, 0, (size_t)b->Rpad * 4, x->stream));
         LAUNCH(x, tc::k_onehot_from_z, (dim3(cdiv(x->N, 256), (unsigned)b->chains.size(), 1), 256, 0, x->stream), (bd));
     }
     int32_t* ni_scratch = nullptr;

@@ -40,11 +40,17 @@ struct GemmArgs {
     int stages;
     int bk;                 // K elements per stage (rows of bk * esz bytes: 128 or 64)
     int esz;                // element bytes: 2 bf16 (kind::f16), 1 e4m3 (kind::f8f6f4)
-    int mode;               // 0: FP32 partials D[z][m][n]; 1: int32 transpose Dt[n][m] (no split)
+    int mode;               // 0: FP32 partials D[z][m][n]; 1: int32 transpose Dt[n][m] (no split); 2: packed
+                            //    counts (no split): row m is a locus, its sum copies of allele 1 + missing calls
+                            //    << miss_shift, written as Dt[n][2 m] = 2 (nk[n] - missing) - copies, Dt[n][2 m + 1]
+                            //    = copies
+    int e5m2;               // esz 1: e5m2 operands (else e4m3)
+    int miss_shift;         // mode 2
+    const int32_t* nk;      // mode 2: individuals of each column's cluster
     int group_major;        // 1: blockIdx.x is the column group and blockIdx.y the row tile, so the
                             //    groups that share an A tile run side by side and A streams from DRAM once
     float* out_f;           // mode 0: [splits][M][ldo]
-    int32_t* out_i;         // mode 1: [N][ldo]
+    int32_t* out_i;         // modes 1, 2: [N][ldo]
     int64_t ldo;
     int* err;
     int tx_extra;           // diagnostics only: bytes a stage barrier expects beyond what its copies
@@ -148,7 +154,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     constexpr uint32_t B_BYTES = BNT * ROW;
     constexpr uint32_t STAGE = A_BYTES + B_BYTES * NB;
     constexpr uint32_t NCOLS = MT * BNT <= 32 ? 32 : MT * BNT <= 64 ? 64 : MT * BNT <= 128 ? 128 : MT * BNT <= 256 ? 256 : 512;
-    constexpr uint32_t FMT = ESZ == 2 ? 1u : 0u;   // bf16 / e4m3
+    constexpr uint32_t FMT = ESZ == 2 ? 1u : 0u;   // bf16 / e4m3 (e5m2: 1, at run time)
     constexpr uint32_t IDESC = (1u << 4) | (FMT << 7) | (FMT << 10) | ((uint32_t)(PIECE >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -220,6 +226,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             // added to the address field in 16-byte units (a shared-memory
             // address below 256 KB never carries out of its 14 bits)
             const uint64_t d0 = sw_desc(smem_u32(smem), ROW);
+            const uint32_t idesc = ESZ == 1 && g.e5m2 ? IDESC | (1u << 7) | (1u << 10) : IDESC;
             for (int it = 0; it < nk; ++it) {
                 const int s = it % stages;
                 if (!mbar_wait(&full[s], (it / stages) & 1, lim) || *(volatile int*)abort_flag) {
@@ -241,8 +248,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 #pragma unroll
                             for (int p = 0; p < BNT; p += PIECE) {
                                 const uint64_t bd = ds + (uint64_t)((A_BYTES + b * B_BYTES + p * ROW + kk * 32) >> 4);
-                                if (ESZ == 2) mma_bf16(tmem + (uint32_t)(t * BNT + p), ad, bd, IDESC, (kk | b) ? 1u : acc0);
-                                else mma_e4m3(tmem + (uint32_t)(t * BNT + p), ad, bd, IDESC, (kk | b) ? 1u : acc0);
+                                if (ESZ == 2) mma_bf16(tmem + (uint32_t)(t * BNT + p), ad, bd, idesc, (kk | b) ? 1u : acc0);
+                                else mma_e4m3(tmem + (uint32_t)(t * BNT + p), ad, bd, idesc, (kk | b) ? 1u : acc0);
                             }
                     }
                 mma_commit(&empty[s]);  // frees the stage once these MMAs have read it
@@ -274,6 +281,15 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                         for (int j = 0; j < 16; ++j)
                             if (n0 + c0 + j < g.N) o[j] = v[j];
                     }
+                } else if (g.mode == 2) {
+                    if (row < g.M)
+#pragma unroll
+                        for (int j = 0; j < 16; ++j)
+                            if (n0 + c0 + j < g.N) {
+                                const int x = __float2int_rn(v[j]), a1 = x & ((1 << g.miss_shift) - 1);
+                                reinterpret_cast<int2*>(g.out_i + (int64_t)(n0 + c0 + j) * g.ldo)[row] =
+                                    make_int2(2 * (__ldg(g.nk + n0 + c0 + j) - (x >> g.miss_shift)) - a1, a1);
+                            }
                 } else {
                     if (row < g.M)
 #pragma unroll
@@ -309,7 +325,28 @@ namespace tc {
 // C  [Npad][Apad]: C[i][2l+a]  copies of allele a at locus l in individual i (bf16)
 // CT [Apad][Npad]: the transpose (alleles x individuals) as e4m3 bytes
 // Missing calls and the padding are zero. 0, 1 and 2 are exact in both types.
-constexpr uint8_t E4M3_ONE = 0x38, E4M3_TWO = 0x40;
+constexpr uint8_t E4M3_ONE = 0x38, E5M2_ONE = 0x3C;
+// Packed counts: where the sums allow it (PackedCounts), CT has one row a locus
+// instead of one an allele, [Lpad][Npad] in e5m2: a call's copies of allele 1,
+// or 2^shift for a missing call with 2^shift above every cluster's copies, so
+// that a sum holds both counts and copies of allele 0 follow from the
+// cluster's size. Sums of whole numbers below 2^24 are exact in FP32, so the
+// form needs 2^shift x (most missing calls at a locus) + 2 N below that; it
+// halves the count contraction's rows and operand. N = 10,000 x L = 100,000,
+// 550 cluster rows: a sweep 4.39 -> 4.0 ms; N = 2,003
+// x L = 20,011, 60 rows: 49 -> 30 us the launch.
+struct PackedCounts {
+    int shift = 0;          // 0: not used
+    // individuals and the largest number of missing calls at a locus
+    static PackedCounts of(int64_t n, int64_t most_missing) {
+        PackedCounts p;
+        int s = 1;
+        while ((1ll << s) <= 2 * n) ++s;
+        if (s <= 15 && (most_missing << s) + 2 * n < (1ll << 24)) p.shift = s;    // e5m2 holds 2^15
+        return p;
+    }
+    uint32_t miss_byte() const { return (uint32_t)(shift + 15) << 2; }
+};
 // One CTA = 128 individuals x BUILD_TILES tiles of 64 loci. Per tile the
 // 2-bit codes are decoded into shared memory and written as whole 128-byte
 // lines of both layouts: CT rows (allele 2l+a, 128 individuals as e4m3
@@ -322,7 +359,7 @@ constexpr uint8_t E4M3_ONE = 0x38, E4M3_TWO = 0x40;
 // adds them in FP64 in a fixed order.
 constexpr int BUILD_TILES = 8;
 __global__ void __launch_bounds__(256) k_build_counts(const DevData D, __nv_bfloat16* C, uint8_t* CT, int64_t Apad,
-                                                      int64_t Npad, const float* logpbar, float* part) {
+                                                      int64_t Npad, const float* logpbar, float* part, uint32_t miss) {
     __shared__ __align__(16) uint8_t code[64][128 + 16];   // [locus][individual]; 3 = missing or padding
     const int t = threadIdx.x;
     const int i0 = blockIdx.x * 128;
@@ -368,16 +405,16 @@ __global__ void __launch_bounds__(256) k_build_counts(const DevData D, __nv_bflo
         __syncthreads();
         uint32_t wnext[2] = {0xFFFFFFFFu, 0xFFFFFFFFu};
         if (tile + 1 < BUILD_TILES && 2 * (l0 + 64) < Apad) load_words(l0 + 64, wnext);
-        // CT rows 2l+a: eight 16-byte pieces per row
-        for (int j = t; j < 128 * 8; j += 256) {
-            const int ra = j >> 3, pc = j & 7, ll = ra >> 1, a = ra & 1;
-            const int64_t row = 2 * (l0 + ll) + a;
-            if (row >= Apad) continue;
+        // CT rows 2l+a (packed counts: l): eight 16-byte pieces per row
+        for (int j = t; j < (miss ? 64 : 128) * 8; j += 256) {
+            const int ra = j >> 3, pc = j & 7, ll = miss ? ra : ra >> 1, a = ra & 1;
+            const int64_t row = miss ? l0 + ll : 2 * (l0 + ll) + a;
+            if (row >= (miss ? Apad / 2 : Apad)) continue;
             const uint4 cw = *reinterpret_cast<const uint4*>(&code[ll][pc * 16]);
             const uint32_t in[4] = {cw.x, cw.y, cw.z, cw.w};
             // code c -> e4m3 copies of allele a: byte permutation tables
             // (allele 1: c; allele 0: 2 - c; missing: 0)
-            const uint32_t lut = a ? 0x00403800u : 0x00003840u;
+            const uint32_t lut = miss ? (miss << 24) | 0x00403C00u : a ? 0x00403800u : 0x00003840u;
             uint32_t o[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
@@ -469,7 +506,9 @@ struct BatchDev {
     int R, Rpad, nchains, splits;
     int64_t Apad, Npad;
     __nv_bfloat16 *Whi, *Wlo;
-    uint8_t* OH;              // [Rpad][Npad] one-hot labels, e4m3
+    uint8_t* OH;              // [Rpad][Npad] one-hot labels, e4m3 (packed counts: e5m2)
+    uint8_t one;              // the byte of 1 in OH
+    int32_t* nk;              // [Rpad] individuals of each cluster row
     const float* logpbar;
     const double* Bc;
     const float* LLpart;      // [splits][N][Rpad]
@@ -493,6 +532,7 @@ __global__ void __launch_bounds__(256) k_update_p_tc(BatchDev b, int64_t l0, int
     const int k = b.rowk[r], m = c.ctl->m;
     const uint64_t seed = c.seed;
     const float lam = (float)c.Lambda[k];
+    if (blockIdx.x == 0 && threadIdx.x == 0) b.nk[r] = 0;    // the label draw counts anew
     const int32_t* Ni = c.Ni + (int64_t)k * c.D.KT;
     float* Freq = c.Freq + (int64_t)k * c.D.KT;
     __nv_bfloat162* Whi = reinterpret_cast<__nv_bfloat162*>(b.Whi + (int64_t)r * b.Apad);
@@ -519,13 +559,27 @@ __global__ void __launch_bounds__(256) k_update_p_tc(BatchDev b, int64_t l0, int
 
 // one-hot rows of every chain's current labels (the initial counts of a
 // batch: the count contraction of these rows is the no-admixture UpdateZ)
+// adds the individuals of each cluster among the warp's labels z (-1: none) to nk
+__device__ __forceinline__ void add_sizes(int32_t* nk, int K, int z) {
+    const int lane = threadIdx.x & 31;
+    for (int k0 = 0; k0 < K; k0 += 32) {
+        int mine = 0;
+        for (int k = k0; k < min(K, k0 + 32); ++k) {
+            const int n = __popc(__ballot_sync(0xffffffffu, z == k));
+            if (lane == k - k0) mine = n;
+        }
+        if (mine) atomicAdd(nk + k0 + lane, mine);
+    }
+}
 __global__ void k_onehot_from_z(BatchDev b) {
     const int ci = blockIdx.y;
     const DevChain& c = b.chains[ci];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.D.N) return;
-    const int r0 = b.row0[ci], z = c.Z[i];
-    for (int k = 0; k < c.K; ++k) b.OH[(int64_t)(r0 + k) * b.Npad + i] = k == z ? E4M3_ONE : 0;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, r0 = b.row0[ci];
+    const bool live = i < c.D.N;
+    const int z = live ? (int)c.Z[i] : -1;
+    add_sizes(b.nk + r0, c.K, z);
+    if (!live) return;
+    for (int k = 0; k < c.K; ++k) b.OH[(int64_t)(r0 + k) * b.Npad + i] = k == z ? b.one : 0;
 }
 
 // One (chain, individual). The split-K partials sum (`sums`, the chain's K
@@ -538,7 +592,7 @@ __global__ void k_onehot_from_z(BatchDev b) {
 // registers.
 template <int KM, bool WIDE>
 __device__ __forceinline__ double sample_tc_body(const BatchDev& b, const DevChain& c, int i, int m, int r0,
-                                                 const float* sums) {
+                                                 const float* sums, int* zout) {
     const DevData& D = c.D;
     const int K = c.K;
     constexpr int UNR = WIDE ? 1 : KM;   // the wide copy keeps its loops rolled (arrays in local memory)
@@ -588,14 +642,15 @@ __device__ __forceinline__ double sample_tc_body(const BatchDev& b, const DevCha
         if (k >= K) break;
         c.Q[(int64_t)i * K + k] = k == z ? 1.f : 0.f;
         c.Mi[(int64_t)i * K + k] = k == z ? vt : 0;
-        b.OH[(int64_t)(r0 + k) * b.Npad + i] = k == z ? E4M3_ONE : 0;
+        b.OH[(int64_t)(r0 + k) * b.Npad + i] = k == z ? b.one : 0;
     }
+    *zout = z;
     return lnl;
 }
 
 __device__ __noinline__ double sample_tc_wide(const BatchDev& b, const DevChain& c, int i, int m, int r0,
-                                              const float* sums) {
-    return sample_tc_body<64, true>(b, c, i, m, r0, sums);
+                                              const float* sums, int* zout) {
+    return sample_tc_body<64, true>(b, c, i, m, r0, sums, zout);
 }
 
 // Label draw for every (chain, individual) from the tensor-core likelihoods;
@@ -638,11 +693,13 @@ __global__ void __launch_bounds__(TS_THREADS) k_sample_tc_tiles(BatchDev b) {
         const DevChain& c = b.chains[ci];
         const int r0 = b.row0[ci], m = c.ctl->m;
         double lnl = 0;
+        int z = -1;
         if (lane < ni) {
             const float* sums = rs + lane * ld + (r0 - gr.z);
-            lnl = c.K <= 16 ? sample_tc_body<16, false>(b, c, i0 + lane, m, r0, sums)
-                            : sample_tc_wide(b, c, i0 + lane, m, r0, sums);
+            lnl = c.K <= 16 ? sample_tc_body<16, false>(b, c, i0 + lane, m, r0, sums, &z)
+                            : sample_tc_wide(b, c, i0 + lane, m, r0, sums, &z);
         }
+        add_sizes(b.nk + r0, c.K, z);
         for (int o = 16; o > 0; o >>= 1) lnl += __shfl_xor_sync(0xffffffffu, lnl, o);
         int last = 0;
         if (lane == 0) {
