@@ -231,7 +231,8 @@ int vp_tc_status(vp_ctx* ctx);
  * column groups of one individual tile launch next to each other. The count
  * contraction has `count_stages` and `count_group_major`. Compiled tiles
  * (bk, row_tiles, cols, piece): (64, 2, 192, 192), (64, 2, 144, 144),
- * (64, 1, 288, 144), (32, 2, 192, 192). */
+ * (64, 1, 288, 144), (32, 2, 192, 192). The first runs a batch of few cluster
+ * rows in groups of 128, 96 or 64 instead (the same sums, bit for bit). */
 typedef struct vp_tc_config {
     int32_t bk, row_tiles, cols, piece, stages, splits, group_major;
     int32_t count_stages, count_group_major;

@@ -62,7 +62,7 @@ struct DevChain {
     int32_t *Mi, *Ni;
     int64_t* MiSum;
     double *LLp, *LL, *metro, *metrop, *Alpha, *Lambda, *f, *F, *Eta, *Gamma, *AlphaLocal, *SumAlpha;
-    double *rout, *lnlTrace, *red, *lnlp, *fpart;
+    double *rout, *lnlTrace, *red, *lnlp, *fpart, *ancestry;
     Rng64* rstate;
 };
 
@@ -2437,8 +2437,9 @@ __global__ void k_record_sweep(const DevChain* chains, double* exact, const int4
 }
 
 // Arrange (src/structure.cpp:1860-1869)
-__global__ void k_arrange(const DevChain* chains, double* ancestry) {
+__global__ void k_arrange(const DevChain* chains) {
     const DevChain& c = chains[blockIdx.z];
+    double* ancestry = c.ancestry;
     const DevData& D = c.D;
     const int K = c.K;
     int nr = c.ctl->nr;

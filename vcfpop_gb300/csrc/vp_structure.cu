@@ -132,7 +132,7 @@ struct TcBatch {
     // the count contraction's 128-row A tiles per CTA (compiled in)
     int mt2 = 2;
     TcChoice cfg;
-    int G1 = 0;               // column groups of the likelihood contraction (Rpad / cfg.bn1)
+    int bnc = 192;            // columns per group of the count contraction
     __nv_bfloat16 *Whi = nullptr, *Wlo = nullptr;
     uint8_t* OH = nullptr;
     float* LLpart = nullptr;
@@ -934,7 +934,7 @@ void chain_layout(Carve& cv, vp_chain* c, const vp_ctx* x) {
     h.red = cv.take<double>(((int64_t)S * K + K + 1) * (1 + LPQ_BLOCKS));
     h.lnlp = cv.take<double>(h.nlnlp);
     h.fpart = cv.take<double>(P->fmodel ? f_blocks(x, *P) : 1);
-    c->ancestry = cv.take<double>((int64_t)N * K);
+    h.ancestry = c->ancestry = cv.take<double>((int64_t)N * K);
     c->d = cv.take<DevChain>(1);
 }
 
@@ -1241,10 +1241,25 @@ int vp_finish_issue(vp_chain** cs, int32_t n) {
     int rc = vp_run(cs, n, mx);
     if (rc) return rc;
     vp_ctx* x = cs[0]->ctx;
+    // the chains of the context's batch in one launch (its headers are
+    // consecutive; K = 1..5 x 4 at 20,011 loci: 24 us, 20 launches took 180)
+    if (x->batch && (int)x->batch->chains.size() == n && std::equal(cs, cs + n, x->batch->chains.begin()) &&
+        std::none_of(cs, cs + n, [](const vp_chain* c) { return c->arranged; })) {
+        int kmax = 1;
+        for (int i = 0; i < n; ++i) kmax = std::max(kmax, cs[i]->P.K);
+        const unsigned gx = std::min<unsigned>(256, cdiv((int64_t)kmax * x->KT, 1024));
+        for (int i0 = 0; i0 < n; i0 += 65535) {
+            const unsigned nz = (unsigned)std::min(65535, n - i0);
+            k_arrange<<<dim3(gx, 1, nz), 256, 0, x->stream>>>(x->batch->dchains + i0);
+            if ((rc = check_launch(x, "k_arrange"))) return rc;
+        }
+        for (int i = 0; i < n; ++i) cs[i]->arranged = true;
+        return VP_OK;
+    }
     for (int i = 0; i < n; ++i) {
         vp_chain* c = cs[i];
         if (c->arranged) continue;
-        k_arrange<<<std::min<unsigned>(1024, cdiv((int64_t)c->P.K * x->KT, 256)), 256, 0, x->stream>>>(c->d, c->ancestry);
+        k_arrange<<<std::min<unsigned>(1024, cdiv((int64_t)c->P.K * x->KT, 256)), 256, 0, x->stream>>>(c->d);
         rc = check_launch(x, "k_arrange");
         if (rc) return rc;
         c->arranged = true;
@@ -1389,7 +1404,8 @@ extern "C" int vp_chain_get(vp_chain* c, int32_t field, void* host, size_t bytes
     if (!c || !host) { vp_set_error("null argument"); return VP_E_ARG; }
     cudaSetDevice(c->ctx->device);
     if (int rc0 = ensure_counts(c)) return rc0;
-    CK(cudaStreamSynchronize(c->ctx->stream));
+    // (a single array's copy below is ordered after the stream's work)
+    if (field == VP_F_FF || field == VP_F_LOCP) CK(cudaStreamSynchronize(c->ctx->stream));
     if (field == VP_F_FF) {
         size_t K = c->P.K;
         if (bytes != 2 * K * 8) { vp_set_error("field %d holds %zu bytes", field, 2 * K * 8); return VP_E_ARG; }
@@ -1795,8 +1811,14 @@ int launch_gemm_t(vp_ctx* x, const CUtensorMap& A, const CUtensorMap& B0, const 
 #define VP_GEMM_TILES(X)             \
     X(64, 2, 2, 2, 192, 192)         \
     X(64, 2, 2, 2, 144, 144)         \
+    X(64, 2, 2, 2, 128, 128)         \
+    X(64, 2, 2, 2, 96, 96)           \
+    X(64, 2, 2, 2, 64, 64)           \
     X(64, 2, 2, 1, 192, 192)         \
     X(128, 1, 2, 1, 192, 192)        \
+    X(128, 1, 2, 1, 128, 128)        \
+    X(128, 1, 2, 1, 96, 96)          \
+    X(128, 1, 2, 1, 64, 64)          \
     X(64, 2, 1, 2, 288, 144)         \
     X(64, 2, 1, 1, 256, 256)         \
     X(32, 2, 2, 2, 192, 192)
@@ -1899,6 +1921,33 @@ constexpr int kMaxStages = 6, kMaxSplits = 64;
 // individuals within 48 KB)
 constexpr int kSampleGroupRows = 160;
 
+// The width of the column groups that covers R cluster rows soonest: a K step
+// of 32 bytes costs a 128-row tile max(bn / 2, 32 + bn / 4) cycles, the tensor
+// core's or shared memory's time, whichever is longer (equal at bn = 128).
+int group_width(int R) {
+    int best = 192, cost = INT32_MAX;
+    for (int bn : {192, 128, 96, 64}) {
+        const int c = (int)cdiv(R, bn) * std::max(2 * bn, 128 + bn);
+        if (c < cost && cdiv(R, bn) * bn <= cdiv(R, 192) * 192) { cost = c; best = bn; }
+    }
+    return best;
+}
+
+// Choice c as it is launched: the (64, 2, 192, 192) tile takes the narrower
+// groups where they cover the rows sooner, with up to twice the stages as
+// they fit. The slices stay c's, so every sum is the same bit for bit.
+// N = 2,003, L = 20,011, 60 rows (K = 1..5 x 4): one 64-row group takes 48 us
+// where the 192-row group took 96 (164 MB of counts: 25 us of HBM reads); the
+// count contraction of the same rows, likewise in 64-row groups, 18 for 30.
+TcChoice run_choice(const TcChoice& c, int R) {
+    TcChoice r = c;
+    if (c.bk1 != 64 || c.mt1 != 2 || c.bn1 != 192) return r;
+    r.bn1 = r.piece1 = group_width(R);
+    while (r.bn1 < c.bn1 && r.st1 < std::min(2 * c.st1, kMaxStages) &&
+           tc::gemm_smem_bytes(r.bn1, 2, r.st1 + 1, r.mt1, r.bk1, 2) <= 227 * 1024)
+        ++r.st1;
+    return r;
+}
 
 int64_t gemm1_tiles(const vp_ctx* x, int Rpad, const TcChoice& c) {
     return cdiv(x->tc.Npad, 128 * c.mt1) * (int64_t)(Rpad / c.bn1);
@@ -1991,10 +2040,11 @@ void tune_store(const vp_ctx* x, int R, const TcChoice& c) {
 // the likelihood contraction of the current batch under choice c
 // the likelihood contraction in `splits` split-K slices: all of them, or the
 // `nz` slices from slice z0 on
-int launch_gemm1(vp_ctx* x, const TcChoice& c, const CUtensorMap& A, const CUtensorMap& W0, const CUtensorMap& W1,
+int launch_gemm1(vp_ctx* x, const TcChoice& cfg, const CUtensorMap& A, const CUtensorMap& W0, const CUtensorMap& W1,
                  int splits, float* out, int z0 = 0, int nz = -1) {
     const TcOperands& t = x->tc;
     const TcBatch* b = x->batch;
+    const TcChoice c = run_choice(cfg, b->R);
     tc::GemmArgs g{};
     g.M = x->N; g.N = b->Rpad; g.kblocks = (int)(t.Apad / c.bk1);
     g.kb_per_split = (g.kblocks + splits - 1) / splits;
@@ -2003,7 +2053,7 @@ int launch_gemm1(vp_ctx* x, const TcChoice& c, const CUtensorMap& A, const CUten
     g.out_f = out; g.ldo = b->Rpad; g.err = t.err;
     g.z0 = z0;
     const unsigned nzs = nz < 0 ? (unsigned)splits : (unsigned)nz;
-    const unsigned mtiles = cdiv(t.Npad, 128 * c.mt1), groups = (unsigned)(b->Rpad / c.bn1);
+    const unsigned mtiles = cdiv(t.Npad, 128 * c.mt1), groups = cdiv(b->R, c.bn1);
     return launch_gemm(x, A, W0, W1, g, c.gm1 ? dim3(groups, mtiles, nzs) : dim3(mtiles, groups, nzs));
 }
 
@@ -2063,11 +2113,15 @@ int make_batch(vp_ctx* x, vp_chain** cs, int n, const TcChoice* force) {
     }
     b->R = (int)rowchain.size();
     // chain groups of the label draw: consecutive chains, at most
-    // kSampleGroupRows cluster rows unless one chain has more
+    // kSampleGroupRows cluster rows unless one chain has more, and few enough
+    // that the draw has about four blocks an SM (N = 2,003, 60 rows: 63 blocks
+    // of all chains took 48 us, 756 blocks of 6 rows take 17)
+    const int64_t tiles = cdiv(x->N, tc::TS_TILE);
+    const int grows = (int)std::min<int64_t>(kSampleGroupRows, std::max<int64_t>(1, (int64_t)b->R * tiles / (x->nsm * 4)));
     std::vector<int4> sgrp;
     for (int i = 0; i < n; ++i) {
         const int K = cs[i]->P.K;
-        if (sgrp.empty() || sgrp.back().w + K > kSampleGroupRows) sgrp.push_back(make_int4(i, i, row0[i], 0));
+        if (sgrp.empty() || sgrp.back().w + K > grows) sgrp.push_back(make_int4(i, i, row0[i], 0));
         sgrp.back().y = i + 1;
         sgrp.back().w += K;
     }
@@ -2081,8 +2135,8 @@ int make_batch(vp_ctx* x, vp_chain** cs, int n, const TcChoice* force) {
         if (force) { delete b; return VP_E_ARG; }
         b->cfg = TcChoice{};
     }
-    b->G1 = b->Rpad / b->cfg.bn1;
     b->splits = b->cfg.splits > 0 ? b->cfg.splits : tc_splits(gemm1_tiles(x, b->Rpad, b->cfg), x->nsm);
+    b->bnc = group_width(b->R);
     const int64_t kblocks = t.Apad / b->cfg.bk1;
     b->splits = (int)std::min<int64_t>(b->splits, kblocks);
     b->splits = (int)cdiv(kblocks, cdiv(kblocks, b->splits));   // splits that hold k-blocks
@@ -2145,10 +2199,11 @@ int make_batch(vp_ctx* x, vp_chain** cs, int n, const TcChoice* force) {
     if ((e = cudaGetLastError()) != cudaSuccess) return undo("launch of k_scatter_chains", e);
     for (int i = 0; i < n; ++i)
         if (cs[i]->graph) { cudaGraphExecDestroy(cs[i]->graph); cs[i]->graph = nullptr; }
+    const uint32_t piece = run_choice(b->cfg, b->R).piece1;
     if ((rc = make_map(&b->mapC1, t.C, t.Npad, t.Apad, t.Apad, 128, b->cfg.bk1)) ||
-        (rc = make_map(&b->mapWhi, b->Whi, b->Rpad, t.Apad, t.Apad, b->cfg.piece1, b->cfg.bk1)) ||
-        (rc = make_map(&b->mapWlo, b->Wlo, b->Rpad, t.Apad, t.Apad, b->cfg.piece1, b->cfg.bk1)) ||
-        (rc = make_map(&b->mapOH, b->OH, b->Rpad, t.Npad, t.Npad, b->piece, t.bk8, 1))) {
+        (rc = make_map(&b->mapWhi, b->Whi, b->Rpad, t.Apad, t.Apad, piece, b->cfg.bk1)) ||
+        (rc = make_map(&b->mapWlo, b->Wlo, b->Rpad, t.Apad, t.Apad, piece, b->cfg.bk1)) ||
+        (rc = make_map(&b->mapOH, b->OH, b->Rpad, t.Npad, t.Npad, b->bnc, t.bk8, 1))) {
         x->batch = b;
         free_batch(x);
         return rc;
@@ -2208,7 +2263,7 @@ unsigned updatep_blocks(const vp_ctx* x, int64_t nloci, int R) {
 // contraction's issuing warps then share their schedulers with fewer ALU
 // warps); 0 when the contraction leaves no room to divide
 size_t updatep_share_smem(const vp_ctx* x, int share) {
-    const TcChoice& c = x->batch->cfg;
+    const TcChoice c = run_choice(x->batch->cfg, x->batch->R);
     size_t g = tc::gemm_smem_bytes(c.bn1, 2, c.st1, c.mt1, c.bk1, 2);
     if (c.mt1 * c.bn1 > 256) g = std::max<size_t>(g, 115 * 1024);     // launch_gemm's TMEM rule
     int per_sm = 0, reserved = 0;
@@ -2354,12 +2409,13 @@ int launch_counts_gemm(vp_ctx* x, int32_t* out) {
         tc::GemmArgs g{};
         const bool packed = t.packed.shift != 0;
         g.M = (int)(packed ? x->L : 2 * x->L); g.N = b->Rpad; g.kblocks = (int)(t.Npad / t.bk8); g.kb_per_split = g.kblocks;
-        g.BN = b->BN; g.piece = b->piece; g.nb = 1; g.mt = b->mt2; g.stages = b->cfg.st2; g.bk = t.bk8; g.esz = 1;
+        g.BN = g.piece = b->bnc; g.nb = 1; g.mt = b->mt2; g.stages = b->cfg.st2; g.bk = t.bk8; g.esz = 1;
         g.mode = packed ? 2 : 1; g.e5m2 = packed; g.miss_shift = t.packed.shift; g.nk = b->nk;
         g.out_i = out ? out : b->NiAll; g.ldo = x->KT; g.err = t.err;
         const unsigned mtiles = cdiv(packed ? t.Apad / 2 : t.Apad, 128 * b->mt2);
         g.group_major = b->cfg.gm2 && mtiles <= 65535;     // grid.y limit; otherwise row tiles on x
-        const dim3 grid = g.group_major ? dim3(b->G, mtiles, 1) : dim3(mtiles, b->G, 1);
+        const unsigned groups = cdiv(b->R, b->bnc);
+        const dim3 grid = g.group_major ? dim3(groups, mtiles, 1) : dim3(mtiles, groups, 1);
         return launch_gemm(x, t.mapCT, b->mapOH, b->mapOH, g, grid);
     }
 }
@@ -2493,10 +2549,11 @@ int tune_batch(vp_ctx* x, int effort, TcChoice* best, vp_tc_config* info) {
     int rc = VP_OK;
     for (size_t i = 0; i < c1.size() && !rc; ++i) {
         const TcChoice& c = c1[i];
+        const uint32_t piece = run_choice(c, b->R).piece1;
         CUtensorMap mA, mW0, mW1;
         if ((rc = make_map(&mA, t.C, t.Npad, t.Apad, t.Apad, 128, c.bk1)) ||
-            (rc = make_map(&mW0, b->Whi, b->Rpad, t.Apad, t.Apad, c.piece1, c.bk1)) ||
-            (rc = make_map(&mW1, b->Wlo, b->Rpad, t.Apad, t.Apad, c.piece1, c.bk1)))
+            (rc = make_map(&mW0, b->Whi, b->Rpad, t.Apad, t.Apad, piece, c.bk1)) ||
+            (rc = make_map(&mW1, b->Wlo, b->Rpad, t.Apad, t.Apad, piece, c.bk1)))
             break;
         float ms = 0.f;
         rc = time_candidate(x, [&] { return launch_gemm1(x, c, mA, mW0, mW1, c.splits, (float*)scratch); }, iters, &ms);
