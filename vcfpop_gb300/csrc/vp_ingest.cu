@@ -520,6 +520,7 @@ extern "C" int vp_vcf_pack2_ex(const char* text, size_t bytes, int32_t n_ind, in
             rc = VP_E_CUDA;
         }
         std::vector<int32_t> hb(L);
+        vp_touch_pages(packed, (size_t)L * Nw * 4);     // while the kernels run
         if (!rc && ((e = cudaMemcpyAsync(packed, dp, (size_t)L * Nw * 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
                     (e = cudaMemcpyAsync(hb.data(), flags, (size_t)L * 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
                     (line_start && (e = cudaMemcpyAsync(line_start, ix.starts, (size_t)(L + 1) * 8, cudaMemcpyDeviceToHost,
@@ -595,6 +596,7 @@ extern "C" int vp_vcf_parse_ex(const char* text, size_t bytes, int32_t n_ind, in
             break;
         }
         std::vector<int32_t> hb(L);
+        vp_touch_pages(alleles, gb);                    // while the kernels run
         if ((e = cudaMemcpyAsync(alleles, dG, gb, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
             (e = cudaMemcpyAsync(n_alleles, dnall, (size_t)L * 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
             (e = cudaMemcpyAsync(ploidy, dploidy, (size_t)n_ind * 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||

@@ -58,6 +58,8 @@ int vp_open_ex(const vp_dataset* ds, int device, int priority, vp_ctx** out);
 // device memory from the library's pool, which keeps freed blocks for the next
 // call (freed with cudaFreeAsync; vp_release_memory gives the kept blocks back)
 cudaError_t vp_pool_alloc(void** p, size_t bytes, int device, cudaStream_t s);
+// maps the pages of a caller's buffer before the device writes all of it
+void vp_touch_pages(void* host, size_t bytes);
 // one more reference to a dataset; vp_dataset_free drops one
 void vp_dataset_retain(const vp_dataset* ds);
 // vp_finish without the final wait

@@ -123,11 +123,29 @@ __device__ __forceinline__ double block_sum_partials(const double* p, int n, dou
     return block_sum(v, sh);
 }
 
+// InitAdmix, single-label form (no admixture, no admixture burn-in):
+// Z_i ~ U{0..K-1} from RNG(seed-1, SALT_INITADM), Mi[i, Z_i] = vt_i
+// (src/structure.cpp:564-573); here from the individual's counter
+__device__ __forceinline__ void init_label(const DevChain& c, int i) {
+    Philox p; p.init(c.seed, ST_INITZ, (uint32_t)i, 0);
+    int z = (int)(p.next() % (uint32_t)c.K);
+    c.Z[i] = (uint16_t)z;
+    c.Mi[i * c.K + z] = (int32_t)c.D.vt[i];
+}
+
 // ---------------------------------------------------------------------------
 // initialisation: InitFix (src/structure.cpp:466-553), InitLocPriori (651-675),
 // InitFmodel (677-708)
-__global__ void k_init_state(const DevChain* chains) {
-    const DevChain& c = chains[blockIdx.z];
+// One launch a chain: the header comes with the launch, block 0 writes the
+// device copy that every later kernel reads, and with `zlabels` the threads
+// draw the initial labels of the counter streams too (19 us a chain with three
+// launches, 11 with one: N = 2,003, L = 20,011).
+__global__ void k_init_chain(DevChain* dst, const __grid_constant__ DevChain c, int zlabels) {
+    static_assert(sizeof(DevChain) % 4 == 0 && sizeof(DevChain) <= 4000, "DevChain as a kernel parameter");
+    if (blockIdx.x == 0) {
+        const uint32_t* a = reinterpret_cast<const uint32_t*>(&c);
+        for (int j = threadIdx.x; j < (int)(sizeof(DevChain) / 4); j += blockDim.x) reinterpret_cast<uint32_t*>(dst)[j] = a[j];
+    }
     const DevData& D = c.D;
     const int K = c.K;
     int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
@@ -163,29 +181,20 @@ __global__ void k_init_state(const DevChain* chains) {
         for (int64_t s = tid; s < D.S; s += nt) c.SumAlpha[s] = 0;
     for (int64_t j = tid; j < c.rlen; j += nt) c.rout[j] = 0;
     if (tid == 0) { c.ctl->m = 0; c.ctl->nr = 0; c.ctl->nlnl = 0; c.ctl->done = c.ctl->done_alpha = c.ctl->done_f = 0; c.ctl->r = 1; c.ctl->lnl = 0; }
+    if (zlabels)
+        for (int64_t i = tid; i < D.N; i += nt) init_label(c, (int)i);
 }
 
-// InitAdmix, single-label form (no admixture, no admixture burn-in):
-// Z_i ~ U{0..K-1} from RNG(seed-1, SALT_INITADM), Mi[i, Z_i] = vt_i
-// (src/structure.cpp:564-573)
-__global__ void k_init_z_single(const DevChain* chains) {
+// the single-label form's initial labels from the reference's one stream
+__global__ void k_init_z_ref(const DevChain* chains) {
     const DevChain& c = chains[blockIdx.z];
     const int K = c.K, N = c.D.N;
-    if (c.rng == 0) {
-        if (blockIdx.x || threadIdx.x) return;
-        Rng64 r; r.init(c.seed - 1, VP_SALT_INITADM);
-        for (int i = 0; i < N; ++i) {
-            int z = (int)r.nextn(K);
-            c.Z[i] = (uint16_t)z;
-            c.Mi[i * K + z] = (int32_t)c.D.vt[i];
-        }
-    } else {
-        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-            Philox p; p.init(c.seed, ST_INITZ, (uint32_t)i, 0);
-            int z = (int)(p.next() % (uint32_t)K);
-            c.Z[i] = (uint16_t)z;
-            c.Mi[i * K + z] = (int32_t)c.D.vt[i];
-        }
+    if (blockIdx.x || threadIdx.x) return;
+    Rng64 r; r.init(c.seed - 1, VP_SALT_INITADM);
+    for (int i = 0; i < N; ++i) {
+        int z = (int)r.nextn(K);
+        c.Z[i] = (uint16_t)z;
+        c.Mi[i * K + z] = (int32_t)c.D.vt[i];
     }
 }
 

@@ -1,5 +1,7 @@
 // Host side of the device STRUCTURE sweep: contexts, chain state, the launch
 // sequence of one sweep, CUDA-graph replay, and the C ABI.
+#include <unistd.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -805,6 +807,19 @@ int ensure_plain(vp_chain* c) {
 
 cudaError_t vp_pool_alloc(void** p, size_t bytes, int device, cudaStream_t s) { return dev_alloc(p, bytes, device, s); }
 
+// Where the GPU writes pageable memory through the host's page tables (Grace),
+// its first write to a page the host has not mapped yet is a fault on the GPU:
+// 22 MB in 100 arrays of fresh pages copied in 18 ms, in 6.6 ms with the pages
+// mapped here first (3.4 ms into pages in use). One write per page, of its own
+// byte.
+void vp_touch_pages(void* host, size_t bytes) {
+    static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    volatile char* p = (volatile char*)host;
+    if (!p || bytes < page) return;
+    for (size_t j = 0; j < bytes; j += page) p[j] = p[j];
+    p[bytes - 1] = p[bytes - 1];
+}
+
 extern "C" int vp_open(const vp_dataset* ds, int device, vp_ctx** out) { return vp_open_ex(ds, device, 0, out); }
 
 int vp_open_ex(const vp_dataset* ds, int device, int priority, vp_ctx** out) {
@@ -1065,14 +1080,15 @@ extern "C" int vp_chain_create(vp_ctx* x, const vp_params* P, vp_chain** out) {
             rc = VP_E_CUDA;
             break;
         }
-        k_set_chain<<<1, 128, 0, s>>>(c->d, h);
-        if ((rc = check_launch(x, "k_set_chain"))) break;
-        k_init_state<<<dim3(std::min<unsigned>(1024, cdiv(std::max<int64_t>(L, (int64_t)N * K), 256)), 1, 1), 256, 0, s>>>(c->d);
-        if ((rc = check_launch(x, "k_init_state"))) break;
         const bool singlez = h.nadmburnin == 0 && !P->admix;
+        const int64_t items = std::max<int64_t>(L, (int64_t)N * K);
+        k_init_chain<<<std::min<unsigned>(1024, cdiv(items, 256)), 256, 0, s>>>(c->d, h, singlez && P->rng != VP_RNG_REFERENCE);
+        if ((rc = check_launch(x, "k_init_chain"))) break;
         if (singlez) {
-            k_init_z_single<<<P->rng ? cdiv(N, 256) : 1, P->rng ? 256 : 32, 0, s>>>(c->d);
-            if ((rc = check_launch(x, "k_init_z_single"))) break;
+            if (P->rng == VP_RNG_REFERENCE) {
+                k_init_z_ref<<<1, 32, 0, s>>>(c->d);
+                if ((rc = check_launch(x, "k_init_z_ref"))) break;
+            }
             if (c->plain_lazy) {
                 c->counts_pending = true;
                 break;
@@ -1345,11 +1361,14 @@ extern "C" int vp_chain_result(vp_chain* c, vp_result* out) {
     CK(cudaStreamSynchronize(c->ctx->stream));
     if (out->rout) CK(cudaMemcpy(out->rout, c->h.rout, sz.rlen * sizeof(double), cudaMemcpyDeviceToHost));
     if (out->lnl) CK(cudaMemcpy(out->lnl, c->h.lnlTrace, sz.nlnl * sizeof(double), cudaMemcpyDeviceToHost));
+    vp_touch_pages(out->Q, NK * sizeof(float));
     if (out->Q) CK(cudaMemcpy(out->Q, c->h.Q, NK * sizeof(float), cudaMemcpyDeviceToHost));
     if (out->ancestry) {
         if (!c->arranged) { vp_set_error("ancestry is available after vp_finish"); return VP_E_STATE; }
+        vp_touch_pages(out->ancestry, NK * sizeof(double));
         CK(cudaMemcpy(out->ancestry, c->ancestry, NK * sizeof(double), cudaMemcpyDeviceToHost));
     }
+    vp_touch_pages(out->freqm, sz.K * sz.KT * sizeof(float));
     if (out->freqm) CK(cudaMemcpy(out->freqm, c->h.FreqM, sz.K * sz.KT * sizeof(float), cudaMemcpyDeviceToHost));
     double *ro = out->rout, *ln = out->lnl;
     float *q = out->Q, *fm = out->freqm;
@@ -1418,6 +1437,7 @@ extern "C" int vp_chain_get(vp_chain* c, int32_t field, void* host, size_t bytes
     int rc = field_ptr(c, field, &p, &n);
     if (rc) return rc;
     if (bytes != n) { vp_set_error("field %d holds %zu bytes, not %zu", field, n, bytes); return VP_E_ARG; }
+    vp_touch_pages(host, n);
     CK(cudaMemcpyAsync(host, p, n, cudaMemcpyDeviceToHost, c->ctx->stream));
     CK(cudaStreamSynchronize(c->ctx->stream));
     return VP_OK;
