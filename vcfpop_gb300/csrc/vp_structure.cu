@@ -1,5 +1,6 @@
 // Host side of the device STRUCTURE sweep: contexts, chain state, the launch
 // sequence of one sweep, CUDA-graph replay, and the C ABI.
+#include <sys/mman.h>
 #include <unistd.h>
 
 #include <algorithm>
@@ -807,15 +808,21 @@ int ensure_plain(vp_chain* c) {
 
 cudaError_t vp_pool_alloc(void** p, size_t bytes, int device, cudaStream_t s) { return dev_alloc(p, bytes, device, s); }
 
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
 // Where the GPU writes pageable memory through the host's page tables (Grace),
 // its first write to a page the host has not mapped yet is a fault on the GPU:
-// 22 MB in 100 arrays of fresh pages copied in 18 ms, in 6.6 ms with the pages
-// mapped here first (3.4 ms into pages in use). One write per page, of its own
-// byte.
+// 22 MB in 100 arrays of fresh pages copied in 18 ms, in 4.4 ms with the pages
+// mapped here first (3.5 into pages in use). One call maps them without
+// changing them; where the kernel has no such call (6.6 ms), one write per
+// page, of its own byte.
 void vp_touch_pages(void* host, size_t bytes) {
     static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    if (!host || bytes < page) return;
+    const uintptr_t a = (uintptr_t)host & ~(uintptr_t)(page - 1);
+    if (madvise((void*)a, (uintptr_t)host + bytes - a, MADV_POPULATE_WRITE) == 0) return;
     volatile char* p = (volatile char*)host;
-    if (!p || bytes < page) return;
     for (size_t j = 0; j < bytes; j += page) p[j] = p[j];
     p[bytes - 1] = p[bytes - 1];
 }
