@@ -41,6 +41,7 @@ struct Ctl {
     double lnl;           // likelihood of the last sampled labels (no-admixture form)
     double fprop;         // UpdateF's proposal for the next cluster
     int32_t err;          // a tensor-core kernel's wait ran out (0: none)
+    int32_t drawn;        // the label draw recorded this sweep and advanced m; its counts follow
 };
 
 struct DevChain {
@@ -75,6 +76,8 @@ __device__ __forceinline__ bool metro_turn(const DevChain& c, int m) { return c.
 __device__ __forceinline__ bool record_at(const DevChain& c, int m) {
     return (c.writelnl && m < c.nburnin && m % c.nthinning == 0) || (m >= c.nburnin && (m - c.nburnin) % c.nthinning == 0);
 }
+// the sweeps whose frequencies enter the mean
+__device__ __forceinline__ bool mean_at(const DevChain& c, int m) { return m >= c.nburnin && record_at(c, m); }
 
 // The block a kernel of the sweep works on. A launch of one chain (or of a
 // tensor-core batch) uses the hardware indices. A cohort launch -- one launch
@@ -96,6 +99,9 @@ __device__ __forceinline__ VBlock vblock(const int4* map) {
 // a cohort keeps launching for runs whose sweeps are all done; their blocks
 // return at once
 __device__ __forceinline__ bool run_over(const DevChain& c) { return c.ctl->m >= c.nburnin + c.nreps; }
+// the same for the counts of the drawn labels, which come after the advance of
+// m where the label draw records
+__device__ __forceinline__ bool counts_over(const DevChain& c) { return !c.ctl->drawn && run_over(c); }
 
 // ---------------------------------------------------------------------------
 // block reductions
@@ -376,11 +382,16 @@ __global__ void k_refresh_lt(const DevChain* chains) {
     if (c.llnb) write_digits(c, k, l, p);
 }
 
+// UpdateP. With `mean` (a sweep; a single step leaves that to Record) the new
+// frequencies of a recorded sweep after burn-in are added to FreqM here, where
+// they are in registers: nothing else of the sweep changes them, so Record
+// reads neither array again.
 // reference streams: 128 block streams RNG(seed + m*128 + b, SALT_UPDATEP),
 // each serial over its share of the K*L range
-__global__ void k_update_p_ref(const DevChain* chains, const int4* map = nullptr) {
+__global__ void k_update_p_ref(const DevChain* chains, int mean, const int4* map = nullptr) {
     const VBlock vb = vblock(map);
     const DevChain& c = chains[vb.z];
+    if (vb.x == 0 && threadIdx.x == 0) c.ctl->drawn = 0;
     if (map && run_over(c)) return;
     const DevData& D = c.D;
     const int K = c.K, m = c.ctl->m;
@@ -403,14 +414,17 @@ __global__ void k_update_p_ref(const DevChain* chains, const int4* map = nullptr
         }
         float inv = (float)(1.0 / s);
         for (int a = 0; a < k2; ++a) { p[a] *= inv; c.Freq[j + a] = p[a]; }
+        if (mean && mean_at(c, m))
+            for (int a = 0; a < k2; ++a) c.FreqM[j + a] += p[a];
         write_lt(c, k, l, p, k2);
     }
 }
 
 // counter streams: one thread per (k, l)
-__global__ void k_update_p_ctr(const DevChain* chains, const int4* map = nullptr) {
+__global__ void k_update_p_ctr(const DevChain* chains, int mean, const int4* map = nullptr) {
     const VBlock vb = vblock(map);
     const DevChain& c = chains[vb.z];
+    if (vb.x == 0 && threadIdx.x == 0) c.ctl->drawn = 0;
     if (map && run_over(c)) return;
     const DevData& D = c.D;
     const int K = c.K, m = c.ctl->m;
@@ -438,6 +452,8 @@ __global__ void k_update_p_ctr(const DevChain* chains, const int4* map = nullptr
         for (int a = 0; a < k2; ++a) p[a] *= inv;
     }
     for (int a = 0; a < k2; ++a) c.Freq[j + a] = p[a];
+    if (mean && mean_at(c, m))
+        for (int a = 0; a < k2; ++a) c.FreqM[j + a] += p[a];
     if (ll_tc_at(c, m)) write_digits(c, k, l, p);
     else write_lt(c, k, l, p, k2);
 }
@@ -813,8 +829,9 @@ __device__ void sample_one(const DevChain& c, int i, int m, bool ref, Rng64* r, 
 // cluster whose cumulative weight exceeds the uniform) are warp reductions,
 // a prefix scan and a ballot, the weights exp(LL_k - max) and the search in
 // FP32. The counter-stream draw is not matched to the reference's stream.
-// Returns, in every lane, LL[i, z] of the drawn label.
-__device__ double sample_warp(const DevChain& c, int i, int m, int lane) {
+// Returns, in every lane, LL[i, z] of the drawn label. With `sum` the new Mi
+// is added to MiSum.
+__device__ double sample_warp(const DevChain& c, int i, int m, int lane, bool sum) {
     const DevData& D = c.D;
     const int K = c.K, N = D.N;
     const int k0 = lane, k1 = lane + 32;
@@ -888,11 +905,20 @@ __device__ double sample_warp(const DevChain& c, int i, int m, int lane) {
     else if (b1) z = 32 + __ffs(b1) - 1;
     if (h0) { Q[k0] = k0 == z ? 1.f : 0.f; Mi[k0] = k0 == z ? vt : 0; }
     if (h1) { Q[k1] = k1 == z ? 1.f : 0.f; Mi[k1] = k1 == z ? vt : 0; }
-    if (lane == 0) c.Z[i] = (uint16_t)z;
+    if (lane == 0) {
+        c.Z[i] = (uint16_t)z;
+        if (sum) c.MiSum[(int64_t)i * K + z] += vt;
+    }
     return __shfl_sync(0xffffffffu, z < 32 ? v0 : v1, z & 31);
 }
 
-__global__ void __launch_bounds__(SAMPLE_BLOCK) k_sample_noadmix(const DevChain* chains, int force, const int4* map = nullptr) {
+// With `record` (counter streams, nothing else left to draw in the sweep) it
+// also does Record: MiSum here, the scalars in the last block, which then
+// advances m; the counts that follow do not depend on it. A launch less a sweep:
+// 300 sweeps at N = 200, L = 2,000, K = 3 take 8.7 ms, 9.5 with a launch for Record.
+__device__ void record_scalars(const DevChain& c, int m, double* sh);
+__global__ void __launch_bounds__(SAMPLE_BLOCK) k_sample_noadmix(const DevChain* chains, int force, int record,
+                                                                 const int4* map = nullptr) {
     const VBlock vb = vblock(map);
     const DevChain& c = chains[vb.z];
     if (map && run_over(c)) return;
@@ -923,7 +949,7 @@ __global__ void __launch_bounds__(SAMPLE_BLOCK) k_sample_noadmix(const DevChain*
         const int lane = threadIdx.x & 31;
         const int i = vb.x * (SAMPLE_BLOCK / 32) + (threadIdx.x >> 5);
         double lnl = 0;
-        if (i < N) lnl = sample_warp(c, i, m, lane);
+        if (i < N) lnl = sample_warp(c, i, m, lane, record && record_at(c, m));
         double t = block_sum(lane == 0 ? lnl : 0.0, sh);
         if (threadIdx.x == 0) c.lnlp[vb.x] = t;
         if (!last_block_done(&c.ctl->done, vb.gx)) return;
@@ -931,6 +957,14 @@ __global__ void __launch_bounds__(SAMPLE_BLOCK) k_sample_noadmix(const DevChain*
         if (threadIdx.x == 0) {
             c.ctl->lnl = tot;
             c.ctl->done = 0;
+        }
+        if (record) {
+            record_scalars(c, m, sh);
+            if (threadIdx.x == 0) {
+                c.ctl->m = m + 1;
+                c.ctl->drawn = 1;
+            }
+            return;
         }
     }
     if (c.locpriori) {
@@ -971,7 +1005,7 @@ __global__ void __launch_bounds__(COUNT_WARPS * 32) k_count_noadmix(const DevCha
     extern __shared__ int32_t hist[];
     const VBlock vb = vblock(map);
     const DevChain& c = chains[vb.z];
-    if (map && run_over(c)) return;
+    if (map && counts_over(c)) return;
     const DevData& D = c.D;
     const int K = c.K;
     if (!force && !binaryq_at(c, c.ctl->m)) return;
@@ -1051,7 +1085,7 @@ __global__ void __launch_bounds__(256) k_count_packed(const DevChain* chains, in
     extern __shared__ uint32_t smask[];   // [KC][Np] masks, then [KC] cluster sizes
     const VBlock vb = vblock(map);
     const DevChain& c = chains[vb.z / kgroups];
-    if (map && run_over(c)) return;
+    if (map && counts_over(c)) return;
     const int kg0 = (vb.z % kgroups) * KC;
     const DevData& D = c.D;
     const int K = c.K, Nw = D.Nw, Np = (D.Nw + 1) >> 1;
@@ -2388,8 +2422,8 @@ __global__ void k_advance(const DevChain* chains) {
 }
 
 // Record and the advance of m in one launch (the end of a captured sweep):
-// every block adds its share of MiSum / FreqM; the last block to finish
-// (after all blocks have read m) does the scalar Record and m += 1.
+// every block adds its share of MiSum (FreqM is UpdateP's); the last block to
+// finish (after all blocks have read m) does the scalar Record and m += 1.
 // With `exact` (the chains of a tensor-core batch), a recorded sweep's
 // lnP(D) is formed from the counts: without admixture Record's sum over
 // individuals and allele copies of ln p (src/structure.cpp:1902-1938) equals
@@ -2400,7 +2434,9 @@ __global__ void k_advance(const DevChain* chains) {
 // block order in FP64: within about 1e-7 relative. The batch's per-sweep sum
 // from the likelihood contraction, whose FP32 accumulation over 10^5 and
 // more alleles per split drifts by a few 1e-6 relative, serves the label
-// draws only.
+// draws only. A thread's four loads of each array are in flight together:
+// K = 1..10 x 10 at L = 100,000: 266 us, 500 when it also summed FreqM and
+// loaded one element at a time.
 __global__ void k_record_sweep(const DevChain* chains, double* exact, const int4* map = nullptr) {
     const VBlock vb = vblock(map);
     const DevChain& c = chains[vb.z];
@@ -2412,23 +2448,28 @@ __global__ void k_record_sweep(const DevChain* chains, double* exact, const int4
     if (rec) {
         int64_t tid = vb.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)vb.gx * blockDim.x;
         for (int64_t j = tid; j < (int64_t)D.N * c.K; j += nt) c.MiSum[j] += c.Mi[j];
-        const bool fm = m >= c.nburnin;
         if (exact) {
             float s = 0.f, cmp = 0.f;
-            for (int64_t j = tid; j < (int64_t)c.K * D.KT; j += nt) {
-                const float p = c.Freq[j];
-                if (fm) c.FreqM[j] += p;
-                const int n = c.Ni[j];
-                if (n) {
-                    const float y = (float)n * ln_freq(p) - cmp, t = s + y;
-                    cmp = (t - s) - y;
-                    s = t;
+            const int64_t n = (int64_t)c.K * D.KT;
+            for (int64_t j0 = tid; j0 < n; j0 += 4 * nt) {
+                float p[4];
+                int ni[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int64_t j = j0 + u * nt;
+                    ni[u] = j < n ? c.Ni[j] : 0;
+                    p[u] = j < n ? c.Freq[j] : 1.f;
                 }
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (ni[u]) {
+                        const float y = (float)ni[u] * ln_freq(p[u]) - cmp, t = s + y;
+                        cmp = (t - s) - y;
+                        s = t;
+                    }
             }
             const double bs = block_sum((double)s - (double)cmp, sh);
             if (threadIdx.x == 0) exact[(int64_t)vb.z * vb.gx + vb.x] = bs;
-        } else if (fm) {
-            for (int64_t j = tid; j < (int64_t)c.K * D.KT; j += nt) c.FreqM[j] += c.Freq[j];
         }
     }
     if (!last_block_done(&c.ctl->done, vb.gx)) return;
@@ -2461,9 +2502,11 @@ __global__ void k_arrange(const DevChain* chains) {
     float finv = (float)(1.0 / nr);
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < (int64_t)K * D.KT; j += (int64_t)gridDim.x * blockDim.x)
         c.FreqM[j] *= finv;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        double inv = 1.0 / nr;
-        for (int j = 0; j < c.rlen; ++j) c.rout[j] *= inv;
+    if (blockIdx.x == 0) {
+        const double inv = 1.0 / nr;
+        for (int j = threadIdx.x; j < c.rlen; j += blockDim.x) c.rout[j] *= inv;
+        __syncthreads();
+        if (threadIdx.x) return;
         c.rout[2] = c.rout[1] - c.rout[0] * c.rout[0];
         c.rout[3] = c.rout[0] - c.rout[2] / 2;
     }

@@ -319,7 +319,7 @@ constexpr uint32_t E5_CODE = 0x6C403C00u, E5_ONE = 0x3Cu;
 __global__ void __launch_bounds__(CT_IND) k_onehot(const DevChain* chains, int force, const int4* map = nullptr) {
     const VBlock vb = vblock(map);
     const DevChain& c = chains[vb.z];
-    if (map && run_over(c)) return;
+    if (map && counts_over(c)) return;
     if (!force && !binaryq_at(c, c.ctl->m)) return;
     const int N = c.D.N, NB = ct_rows(c.K), t = threadIdx.x;
     __shared__ uint16_t z[CT_IND];
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(CT_THREADS, NB == 16 ? 2 : 1) k_count_tc(const
     __shared__ int s_abort;
     const VBlock vb = vblock(map);
     const DevChain& c = chains[vb.z];
-    if (map && run_over(c)) return;
+    if (map && counts_over(c)) return;
     if (!force && !binaryq_at(c, c.ctl->m)) return;
     const DevData& D = c.D;
     const int K = c.K;

@@ -577,6 +577,13 @@ bool accept_zeroes(const vp_chain* c, bool sweep) {
     return sweep && c->P.admix && c->P.metrofreq > 0 && c->P.rng == VP_RNG_COUNTER;
 }
 
+// in a sweep whose label draw is the last thing that Record waits for, the
+// draw does Record
+bool draw_records(const vp_chain* c) {
+    const vp_params& P = c->P;
+    return P.rng == VP_RNG_COUNTER && !P.admix && c->h.nadmburnin == 0 && !P.locpriori && !P.fmodel;
+}
+
 int launch_step(vp_chain* c, int step, int force, bool sweep = false) {
     vp_ctx* x = c->ctx;
     const vp_params& P = c->P;
@@ -584,15 +591,15 @@ int launch_step(vp_chain* c, int step, int force, bool sweep = false) {
     const bool ref = P.rng == VP_RNG_REFERENCE;
     switch (step) {
         case VP_STEP_UPDATEP:
-            if (ref) SL(c, k_update_p_ref, (1, 1, 1), (128), 0, 0);
-            else SL(c, k_update_p_ctr, (cdiv((int64_t)K * x->L, 256), 1, 1), (256), 0, 0);
+            if (ref) SL(c, k_update_p_ref, (1, 1, 1), (128), 0, 1, (int)sweep);
+            else SL(c, k_update_p_ctr, (cdiv((int64_t)K * x->L, 256), 1, 1), (256), 0, 1, (int)sweep);
             return VP_OK;
         case VP_STEP_LOGLIK: {
             // the FP32 stream, whose table UpdateP leaves alone on tensor-core sweeps
             if (c->h.llnb) LAUNCH(x, k_refresh_lt, (cdiv((int64_t)K * x->L, 256), 256, 0, x->stream), (c->d));
             int rc = launch_loglik(c, 1);
             if (rc) return rc;
-            SL(c, k_sample_noadmix, (c->h.nsampblk, 1, 1), (SAMPLE_BLOCK), 0, 1, 1);
+            SL(c, k_sample_noadmix, (c->h.nsampblk, 1, 1), (SAMPLE_BLOCK), 0, 2, 1, 0);
             return VP_OK;
         }
         case VP_STEP_UPDATEQ: {
@@ -600,7 +607,8 @@ int launch_step(vp_chain* c, int step, int force, bool sweep = false) {
             if (!P.admix) {
                 int rc = launch_loglik(c, force);
                 if (rc) return rc;
-                SL(c, k_sample_noadmix, (ref ? 1 : c->h.nsampblk, 1, 1), (SAMPLE_BLOCK), 0, 1, 0);
+                SL(c, k_sample_noadmix, (ref ? 1 : c->h.nsampblk, 1, 1), (SAMPLE_BLOCK), 0, 2, 0,
+                   (int)(sweep && draw_records(c)));
                 if (c->h.nadmburnin > 0) SL(c, k_update_q_admix, (ref ? 1 : gi, 1, 1), (ref ? 32 : 256), 0, 1, 0);
             } else {
                 SL(c, k_update_q_admix, (ref ? 1 : gi, 1, 1), (ref ? 32 : 256), 0, 1, 0);
@@ -746,10 +754,11 @@ int launch_sweep(vp_chain* c) {
         if (int rc = steps({VP_STEP_UPDATEA, VP_STEP_UPDATEF})) return rc;
     if (int rc = bf.join()) return rc;
     if (int rc = ba.join()) return rc;
+    if (draw_records(c)) return VP_OK;
     // Record and m += 1 as one launch; at most 128 blocks: the element-wise
     // part only runs on recorded sweeps, and every block takes part in the
     // last-block count
-    SL(c, k_record_sweep, (std::min<unsigned>(128, cdiv((int64_t)c->P.K * x->KT, 256)), 1, 1), (256), 0, -1);
+    SL(c, k_record_sweep, (std::min<unsigned>(128, cdiv((int64_t)c->P.K * x->N, 256)), 1, 1), (256), 0, -1);
     return VP_OK;
 }
 

@@ -540,6 +540,8 @@ __global__ void __launch_bounds__(256) k_update_p_tc(BatchDev b, int64_t l0, int
     const float2* lpb = reinterpret_cast<const float2*>(b.logpbar);
     const int2* Ni2 = reinterpret_cast<const int2*>(Ni);
     float2* F2 = reinterpret_cast<float2*>(Freq);
+    float2* M2 = reinterpret_cast<float2*>(c.FreqM + (int64_t)k * c.D.KT);
+    const bool mean = mean_at(c, m);
     l1 = min(l1, L);
     for (int64_t l = l0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; l < l1; l += (int64_t)gridDim.x * blockDim.x) {
         const int64_t kl = (int64_t)k * L + l;
@@ -549,6 +551,10 @@ __global__ void __launch_bounds__(256) k_update_p_tc(BatchDev b, int64_t l0, int
         float p0, p1;
         ph.dirichlet2(lam + (float)n.x, lam + (float)n.y, p0, p1);
         F2[l] = make_float2(p0, p1);
+        if (mean) {
+            const float2 t = M2[l];
+            M2[l] = make_float2(t.x + p0, t.y + p1);
+        }
         const float2 lb = lpb[l];
         const float w0 = ln_freq_fast(p0) - lb.x, w1 = ln_freq_fast(p1) - lb.y;
         const __nv_bfloat16 h0 = __float2bfloat16(w0), h1 = __float2bfloat16(w1);
