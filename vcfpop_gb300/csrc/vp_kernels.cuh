@@ -112,9 +112,12 @@ __device__ T block_sum(T v, T* sh) {
     __syncthreads();
     if ((threadIdx.x & 31) == 0) sh[w] = v;
     __syncthreads();
+    // the warps' sums by shuffles: a serial chain of FP64 adds is slow here
     T r = 0;
-    if (threadIdx.x == 0)
-        for (int j = 0; j < nw; ++j) r += sh[j];
+    if (w == 0) {
+        if ((int)threadIdx.x < nw) r = sh[threadIdx.x];
+        for (int o = 1; o < nw; o <<= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    }
     __syncthreads();
     return r;  // valid in thread 0
 }
@@ -844,6 +847,11 @@ __device__ double sample_warp(const DevChain& c, int i, int m, int lane, bool su
     const int lg = K <= 1 ? 0 : 32 - __clz(K - 1), step = lg < 5 ? 32 >> lg : 1;
     const int kk = lg < 5 ? lane & ((1 << lg) - 1) : lane;
     const int ch0 = lg < 5 ? lane >> lg : 0;
+    // what does not depend on the partials, while their loads are in flight
+    const int vt = (int)D.vt[i];
+    Philox ph;
+    ph.init(c.seed, ST_Q | ((uint32_t)m << 4), (uint32_t)i, 0);
+    const float u = ph.uniformf();
     if (ll_tc_at(c, m)) {
         // the tensor-core form's partials: whole numbers of 2^-24
         long long a = 0;
@@ -867,7 +875,6 @@ __device__ double sample_warp(const DevChain& c, int i, int m, int lane, bool su
     int32_t* Mi = c.Mi + (int64_t)i * K;
     if (h0) LL[k0] = v0;
     if (h1) LL[k1] = v1;
-    const int vt = (int)D.vt[i];
     if (vt == 0) {
         if (h0) { Q[k0] = 0.f; Mi[k0] = 0; }
         if (h1) { Q[k1] = 0.f; Mi[k1] = 0; }
@@ -881,8 +888,9 @@ __device__ double sample_warp(const DevChain& c, int i, int m, int lane, bool su
     }
     // the maximum in FP64; the weights exp(LL_k - max), their prefix sums and
     // the draw in FP32 (FP64 arithmetic is slow on this part)
+    // (up to 32 clusters the maximum of a group of 2^lg lanes is that of group 0)
     double mx = fmax(h0 ? w0 : -1.79769313486231570e+308, h1 ? w1 : -1.79769313486231570e+308);
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    for (int o = lg < 5 ? (1 << lg) >> 1 : 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     const float d0 = (float)(w0 - mx), d1 = (float)(w1 - mx);
     const float e0 = h0 ? (d0 < -23.f ? (float)VP_MIN_FREQ : __expf(d0)) : 0.f;
     const float e1 = h1 ? (d1 < -23.f ? (float)VP_MIN_FREQ : __expf(d1)) : 0.f;
@@ -895,9 +903,7 @@ __device__ double sample_warp(const DevChain& c, int i, int m, int lane, bool su
     const float tot0 = __shfl_sync(0xffffffffu, c0, 31);
     c1 += tot0;
     const float s = __shfl_sync(0xffffffffu, c1, 31) + (float)(VP_MIN_FREQ * K);
-    float u = 0.f;
-    if (lane == 0) { Philox ph; ph.init(c.seed, ST_Q | ((uint32_t)m << 4), (uint32_t)i, 0); u = ph.uniformf(); }
-    const float t = __shfl_sync(0xffffffffu, u, 0) * s;
+    const float t = u * s;
     int z = K - 1;
     const unsigned b0 = __ballot_sync(0xffffffffu, h0 && t < c0);
     const unsigned b1 = __ballot_sync(0xffffffffu, h1 && t < c1);
@@ -950,7 +956,11 @@ __global__ void __launch_bounds__(SAMPLE_BLOCK) k_sample_noadmix(const DevChain*
         const int i = vb.x * (SAMPLE_BLOCK / 32) + (threadIdx.x >> 5);
         double lnl = 0;
         if (i < N) lnl = sample_warp(c, i, m, lane, record && record_at(c, m));
-        double t = block_sum(lane == 0 ? lnl : 0.0, sh);
+        // lnl is the same in every lane
+        if (lane == 0) sh[threadIdx.x >> 5] = lnl;
+        __syncthreads();
+        double t = lane < SAMPLE_BLOCK / 32 ? sh[lane] : 0;
+        for (int o = 1; o < SAMPLE_BLOCK / 32; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
         if (threadIdx.x == 0) c.lnlp[vb.x] = t;
         if (!last_block_done(&c.ctl->done, vb.gx)) return;
         const double tot = block_sum_partials(c.lnlp, vb.gx, sh);
@@ -2360,39 +2370,41 @@ __global__ void __launch_bounds__(UF_T) k_update_f(const DevChain* chains, int k
 
 // Record (src/structure.cpp:1941-2045): likelihood trace, running sums of the
 // likelihood and parameters, then m += 1. One block per chain.
-// the scalar part of Record at sweep m, by one block
+// the scalar part of Record at sweep m, by one block of at least 64 threads: an
+// entry of rout a thread, not one thread's chain of loads and stores (the label
+// draw that ends with it, N = 200 x L = 2,000: 13.4 us, 15.6 before)
 __device__ void record_scalars(const DevChain& c, int m, double* sh) {
     const DevData& D = c.D;
     const int K = c.K;
-    if (record_at(c, m)) {
-        double like;
-        if (binaryq_at(c, m)) like = c.ctl->lnl;
-        else {
-            double v = 0;
-            for (int j = threadIdx.x; j < c.nlnlp; j += blockDim.x) v += c.lnlp[j];
-            like = block_sum(v, sh);
-        }
-        if (threadIdx.x == 0) {
-            if (c.writelnl && c.ctl->nlnl < c.ntrace) c.lnlTrace[c.ctl->nlnl++] = like;
-            if (m >= c.nburnin) {
-                c.ctl->nr++;
-                c.rout[0] += like;
-                c.rout[1] += like * like;
-                int nf = c.fmodel ? (c.fsame ? 1 : K) : 0;
-                int na = c.admix ? (c.diffalpha ? K : 1) : 0;
-                int nl = c.difflambda ? K : 1;
-                for (int j = 0; j < nl; ++j) c.rout[4 + j] += c.Lambda[j];
-                if (c.locpriori) {
-                    c.rout[4 + nl] += c.ctl->r;
-                    const double* g = c.admix ? c.Alpha : c.Eta;
-                    for (int j = 0; j < K; ++j) c.rout[4 + nl + 1 + j] += g[j];
-                    const double* gl = c.admix ? c.AlphaLocal : c.Gamma;
-                    for (int j = 0; j < K * D.S; ++j) c.rout[4 + nl + 1 + K + j] += gl[j];
-                } else if (c.admix)
-                    for (int j = 0; j < na; ++j) c.rout[4 + nl + j] += c.Alpha[j];
-                for (int j = 0; j < nf; ++j) c.rout[c.rlen - nf + j] += c.F[j];
-            }
-        }
+    if (!record_at(c, m)) return;
+    __shared__ double s_like;
+    double v = 0;
+    if (!binaryq_at(c, m)) {
+        for (int j = threadIdx.x; j < c.nlnlp; j += blockDim.x) v += c.lnlp[j];
+        v = block_sum(v, sh);
+    } else if (threadIdx.x == 0) v = c.ctl->lnl;
+    if (threadIdx.x == 0) s_like = v;
+    __syncthreads();
+    const double like = s_like;
+    if (threadIdx.x == 0 && c.writelnl && c.ctl->nlnl < c.ntrace) c.lnlTrace[c.ctl->nlnl++] = like;
+    if (m < c.nburnin) return;
+    if (threadIdx.x == 32) c.ctl->nr++;
+    const int nf = c.fmodel ? (c.fsame ? 1 : K) : 0, na = c.admix ? (c.diffalpha ? K : 1) : 0, nl = c.difflambda ? K : 1;
+    for (int j = threadIdx.x; j < c.rlen; j += blockDim.x) {
+        double x;
+        int i = j - 4 - nl;
+        if (j < 2) x = j ? like * like : like;
+        else if (j < 4) continue;
+        else if (i < 0) x = c.Lambda[j - 4];
+        else if (j >= c.rlen - nf) x = c.F[j - (c.rlen - nf)];
+        else if (!c.locpriori) {
+            if (i >= na) continue;
+            x = c.Alpha[i];
+        } else if (i == 0) x = c.ctl->r;
+        else if (--i < K) x = (c.admix ? c.Alpha : c.Eta)[i];
+        else if ((i -= K) < K * D.S) x = (c.admix ? c.AlphaLocal : c.Gamma)[i];
+        else continue;
+        c.rout[j] += x;
     }
 }
 
