@@ -132,7 +132,9 @@ struct TcBatch {
     // cluster rows padded to whole 192-row column groups of the count
     // contraction (BN cluster rows per CTA, piece per MMA)
     int R = 0, Rpad = 0, G = 0, BN = 192, piece = 192, splits = 1;
-    // the count contraction's 128-row A tiles per CTA (compiled in)
+    // the count contraction's 128-row A tiles per CTA: two, or one where two
+    // would leave SMs without a CTA (20,011 loci, 60
+    // rows: 79 CTAs took 17.7 us, 157 take 13.8)
     int mt2 = 2;
     TcChoice cfg;
     int bnc = 192;            // columns per group of the count contraction
@@ -1855,6 +1857,10 @@ int launch_gemm_t(vp_ctx* x, const CUtensorMap& A, const CUtensorMap& B0, const 
     X(128, 1, 2, 1, 128, 128)        \
     X(128, 1, 2, 1, 96, 96)          \
     X(128, 1, 2, 1, 64, 64)          \
+    X(128, 1, 1, 1, 192, 192)        \
+    X(128, 1, 1, 1, 128, 128)        \
+    X(128, 1, 1, 1, 96, 96)          \
+    X(128, 1, 1, 1, 64, 64)          \
     X(64, 2, 1, 2, 288, 144)         \
     X(64, 2, 1, 1, 256, 256)         \
     X(32, 2, 2, 2, 192, 192)
@@ -1972,9 +1978,10 @@ int group_width(int R) {
 // Choice c as it is launched: the (64, 2, 192, 192) tile takes the narrower
 // groups where they cover the rows sooner, with up to twice the stages as
 // they fit. The slices stay c's, so every sum is the same bit for bit.
-// N = 2,003, L = 20,011, 60 rows (K = 1..5 x 4): one 64-row group takes 48 us
-// where the 192-row group took 96 (164 MB of counts: 25 us of HBM reads); the
-// count contraction of the same rows, likewise in 64-row groups, 18 for 30.
+// N = 2,003, L = 20,011, 60 rows (K = 1..5 x 4): one 64-row group takes 36 us
+// where the 192-row group took 96 (164 MB of counts: 25 us of HBM reads; 48 us
+// with the partials stored a float at a time); the count contraction of the
+// same rows, likewise in 64-row groups, 18 for 30.
 TcChoice run_choice(const TcChoice& c, int R) {
     TcChoice r = c;
     if (c.bk1 != 64 || c.mt1 != 2 || c.bn1 != 192) return r;
@@ -2173,6 +2180,7 @@ int make_batch(vp_ctx* x, vp_chain** cs, int n, const TcChoice* force) {
     }
     b->splits = b->cfg.splits > 0 ? b->cfg.splits : tc_splits(gemm1_tiles(x, b->Rpad, b->cfg), x->nsm);
     b->bnc = group_width(b->R);
+    b->mt2 = cdiv(t.packed.shift ? t.Apad / 2 : t.Apad, 256) * cdiv(b->R, b->bnc) < (unsigned)x->nsm ? 1 : 2;
     const int64_t kblocks = t.Apad / b->cfg.bk1;
     b->splits = (int)std::min<int64_t>(b->splits, kblocks);
     b->splits = (int)cdiv(kblocks, cdiv(kblocks, b->splits));   // splits that hold k-blocks
