@@ -74,3 +74,20 @@ def test_loglik_packed2_every_cluster_count(N):
         assert np.isfinite(got).all(), K
         rel = np.abs(got - ref) / np.maximum(np.abs(ref), 1.0)
         assert rel.max() < 1e-5, (K, rel.max())
+
+
+@pytest.mark.parametrize("N,L", [(1, 640), (255, 64), (257, 645), (2049, 13_100), (4100, 9_001)])
+@pytest.mark.parametrize("K", [1, 2])
+def test_loglik_packed2_one_and_two_clusters(N, L, K):
+    """Both splits of the one- and two-cluster forms over threads: 2
+    individuals a thread while the CTAs are few, 16 from there on (the last
+    two sizes)."""
+    rng = np.random.default_rng(N + K)
+    G = rng.integers(0, 2, (L, N, 2), dtype=np.int8)
+    G[rng.random((L, N)) < 0.03] = -1
+    p = np.maximum(rng.dirichlet([0.7, 0.7], size=(K, L)).astype(np.float32), 1e-6)
+    p /= p.sum(axis=2, keepdims=True)
+    freq = np.ascontiguousarray(p.reshape(K, 2 * L))
+    ref = loglik_ref(G, freq)
+    rel = np.abs(_loglik_device(G, freq, N, L, K) - ref) / np.maximum(np.abs(ref), 1.0)
+    assert rel.max() < 1e-5, rel.max()

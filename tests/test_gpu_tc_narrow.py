@@ -29,11 +29,12 @@ def _chains(ctx, ks, **kw):
 
 
 # rows on both sides of every width (64, 96, 128, 192 and two groups), a lone
-# chain, individual tiles of one and of many, K above the 16-cluster draw
+# chain, individual tiles of one and of many, K above the 16-cluster draw, and
+# loci enough for 256-row count tiles
 @pytest.mark.parametrize("N,L,ks", [(33, 70, (1,)), (300, 333, (1, 2, 3, 4, 5) * 4), (257, 200, (32, 32)),
                                     (257, 200, (32, 32, 1)), (700, 150, (16,) * 6), (130, 150, (16,) * 6 + (1,)),
                                     (2003, 90, (16,) * 8), (300, 150, (16,) * 8 + (1,)), (300, 150, (10,) * 20),
-                                    (300, 150, (10,) * 40)])
+                                    (300, 150, (10,) * 40), (33, 39_000, (2, 3)), (40, 39_000, (16,) * 12)])
 def test_narrow_groups(N, L, ks):
     """Exact counts of the labels, the same sweeps bit for bit from 144-row
     groups where those fit (the FP32 sums keep their order), and the chains'

@@ -640,9 +640,10 @@ __global__ void __launch_bounds__(LT_BLOCK, 3) k_loglik(const DevChain* chains, 
 // words are copied to shared memory by cp.async one slice ahead. Sums over 32
 // loci are folded into Kahan-compensated FP32 totals, converted to FP64 once
 // per chunk, as in the table form.
-template <int KC>
+// individuals per thread
+__host__ __device__ constexpr int lf_m(int kc) { return kc <= 2 ? 16 : kc <= 6 ? 4 : 2; }
+template <int KC, int M>
 struct LfShape {
-    static constexpr int M = KC <= 2 ? 16 : KC <= 6 ? 4 : 2;                 // individuals per thread
     static constexpr int SL = M >= 8 ? 32 : 64;                               // loci per staged slice
     static constexpr int GW = LL_BLOCK * M / 16;                              // genotype words per CTA and locus
     static constexpr int KQ = (KC + 3) / 4;                                   // 16-byte chunks of a staged row
@@ -656,12 +657,12 @@ struct LfShape {
 // K > 16. Its columns: K itself for K <= 2, else 6 or 14.
 __host__ __device__ constexpr bool lf_form(int K) { return K <= 2 || K == 5 || K == 6 || K == 13 || K == 14; }
 __host__ __device__ constexpr int lf_kc(int K) { return K <= 2 ? K : K <= 6 ? 6 : 14; }
-__host__ __device__ constexpr int lf_individuals(int kc) { return LL_BLOCK * (kc <= 2 ? 16 : kc <= 6 ? 4 : 2); }
-template <int KC>
+__host__ __device__ constexpr int lf_individuals(int kc) { return LL_BLOCK * lf_m(kc); }
+template <int KC, int M = lf_m(KC)>
 __global__ void __launch_bounds__(LL_BLOCK) k_loglik_fma(const DevChain* chains, int kgroups, int force,
                                                          const int4* map = nullptr) {
-    using S = LfShape<KC>;
-    constexpr int M = S::M, SL = S::SL, GW = S::GW, KQ = S::KQ, GS = SL + 4;
+    using S = LfShape<KC, M>;
+    constexpr int SL = S::SL, GW = S::GW, KQ = S::KQ, GS = SL + 4;
     __shared__ __align__(16) float sT[2][SL][2][4 * KQ];   // rows T0 and T2 of the slice's loci
     __shared__ __align__(16) float2 sAB[SL][KC];            // (a, b)
     __shared__ __align__(16) uint32_t sG[2][GW][GS];        // genotype words, transposed

@@ -368,6 +368,17 @@ void ll_tc_chunks(DevChain& h, int32_t N, int64_t L, int nsm) {
     h.tcchunk = (int32_t)cdiv(nst, per);
 }
 
+// The FMA form of one and two clusters holds 16 individuals a thread, 2,048 a
+// CTA. Where CTAs of two individuals a thread over the same locus chunks (the
+// same sums bit for bit) are at most LF_FEW an SM it runs those: a sweep of N =
+// 200 x L = 2,000, K = 2 takes 27 us with them and 52 without, 500 x 5,000 35
+// and 58, 1,000 x 20,000 (8 an SM) 46 and 48; 2,000 x 20,000 (16 an SM) 57 and
+// 57, and 54 and 52 at K = 1.
+constexpr int LF_FEW = 12;
+bool lf_few(int kc, int32_t N, int64_t nchunk, int nsm) {
+    return kc <= 2 && cdiv(N, 2 * LL_BLOCK) * nchunk <= (int64_t)nsm * LF_FEW;
+}
+
 int launch_loglik(vp_chain* c, int force) {
     vp_ctx* x = c->ctx;
     prof_mark(x, true);
@@ -383,8 +394,11 @@ int launch_loglik(vp_chain* c, int force) {
         }
     }
     if (c->ll_fma) {
-        const dim3 g(cdiv(x->N, lf_individuals(c->kc)), c->h.nchunk, c->kgroups);
-        switch (c->kc) {
+        const bool few = lf_few(c->kc, x->N, c->h.nchunk, x->nsm);
+        const dim3 g(cdiv(x->N, few ? 2 * LL_BLOCK : lf_individuals(c->kc)), c->h.nchunk, c->kgroups);
+        if (few && c->kc == 1) SL(c, (k_loglik_fma<1, 2>), (g), (LL_BLOCK), 0, 2, c->kgroups, force);
+        else if (few) SL(c, (k_loglik_fma<2, 2>), (g), (LL_BLOCK), 0, 2, c->kgroups, force);
+        else switch (c->kc) {
             case 1: SL(c, k_loglik_fma<1>, (g), (LL_BLOCK), 0, 2, c->kgroups, force); break;
             case 2: SL(c, k_loglik_fma<2>, (g), (LL_BLOCK), 0, 2, c->kgroups, force); break;
             case 6: SL(c, k_loglik_fma<6>, (g), (LL_BLOCK), 0, 2, c->kgroups, force); break;
@@ -3041,7 +3055,7 @@ __global__ void k_ll_reduce(const DevChain* chains, double* ll) {
 struct LLPlan {
     DevChain h{};
     size_t scratch = 0;   // bytes: descriptor, table, partials
-    int kc = 16, kgroups = 1;
+    int kc = 16, kgroups = 1, nsm = 1;
     bool fma = false;
 };
 
@@ -3051,6 +3065,7 @@ int ll_plan(int32_t N, int64_t L, int32_t K, int nsm, LLPlan* pl) {
     h.D.N = N; h.D.L = L; h.D.KT = 2 * L; h.D.Nw = (N + 15) / 16; h.D.packed2 = 1; h.D.vmax = 2; h.D.maxK = 2;
     h.K = K;
     h.kp = (K + 3) & ~3;
+    pl->nsm = nsm;
     pl->fma = lf_form(K);
     pl->kc = ll_kc(pl->fma, K);
     pl->kgroups = (K + pl->kc - 1) / pl->kc;
@@ -3077,8 +3092,12 @@ int ll_run(LLPlan& pl, const uint32_t* geno, const float* freq, double* ll, void
     // to outlive the call
     k_set_chain<<<1, 128, 0, s>>>(d, h);
     k_lt_from_freq<<<cdiv((int64_t)h.K * h.D.L, 256), 256, 0, s>>>(freq, h.K, h.D.L, h.kp, h.lt);
-    const dim3 g(cdiv(h.D.N, ll_individuals(pl.fma, pl.kc)), h.nchunk, pl.kgroups);
-    if (pl.fma) {
+    const bool few = pl.fma && lf_few(pl.kc, h.D.N, h.nchunk, pl.nsm);
+    const dim3 g(cdiv(h.D.N, few ? 2 * LL_BLOCK : ll_individuals(pl.fma, pl.kc)), h.nchunk, pl.kgroups);
+    if (few) {
+        if (pl.kc == 1) k_loglik_fma<1, 2><<<g, LL_BLOCK, 0, s>>>(d, pl.kgroups, 1);
+        else k_loglik_fma<2, 2><<<g, LL_BLOCK, 0, s>>>(d, pl.kgroups, 1);
+    } else if (pl.fma) {
         switch (pl.kc) {
             case 1: k_loglik_fma<1><<<g, LL_BLOCK, 0, s>>>(d, pl.kgroups, 1); break;
             case 2: k_loglik_fma<2><<<g, LL_BLOCK, 0, s>>>(d, pl.kgroups, 1); break;
