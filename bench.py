@@ -442,7 +442,7 @@ def bench_single(args):
     peak = peaks.get("hbm_gbs", 6800.0)
     achieved = byts / (dom_ms / 1e3) / 1e9
     l2 = byts < 120e6
-    roof = {"bound": "hbm", "kernel": "k_update_z_admix_ctr (per-copy labels)" if admix else "k_loglik / k_loglik_fma (likelihood stream)",
+    roof = {"bound": "hbm", "kernel": "k_z_admix_pk / k_z_admix_gen (per-copy labels)" if admix else "k_loglik / k_loglik_fma (likelihood stream)",
             "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "peak_source": "MEASURED_PEAKS.json hbm_gbs" if "hbm_gbs" in peaks else "fallback", "traffic": None,
             "avg_launch_ms": dom_ms, "bytes_per_launch": byts,
@@ -546,7 +546,7 @@ def single_compact(name, local, peaks, cpu_budget_s=0.0):
     ctx.close()
     out = {"workload": f"{name}: {SINGLE_DESC[name]}; one step = one sweep", "value": upd / (ms / 1e3),
            "unit": "updates/s", "ms_per_step": ms, "steps": n, "warmup": 3, "gpu_launches": launches,
-           "roofline": {"bound": "hbm", "kernel": "k_update_z_admix_ctr (per-copy labels)" if admix else
+           "roofline": {"bound": "hbm", "kernel": "k_z_admix_pk / k_z_admix_gen (per-copy labels)" if admix else
                         "k_loglik / k_loglik_fma (likelihood stream)", "achieved": achieved, "peak": peak, "unit": "GB/s",
                         "frac": achieved / peak, "avg_launch_ms": dom_ms, "bytes_per_launch": byts},
            "data_seconds": t_data}
@@ -1081,12 +1081,12 @@ def main():
 
     line = {"metric": METRIC, "value": value, "unit": "updates/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak",
-            "vs_baseline": None, "dtype": "likelihood bf16 hi+lo x bf16 counts -> f32; counts e4m3 x e4m3 -> f32 (exact); lnP(D) in f64" if form else "f32",
+            "vs_baseline": None, "dtype": "likelihood bf16 hi+lo x bf16 counts -> f32; counts e5m2 x e5m2 -> f32 (exact); lnP(D) in f64" if form else "f32",
             "data": "synthetic F-model (8 pops, F=0.03, Beta(0.5,0.5) ancestry, 1% missing), seeded",
             "config": {"workload": f"batched K-sweep: N={N_IND}, L={ds.L} biallelic SNPs, K=1..10 x 10 replicates "
                                    f"= 100 no-admixture chains, one sweep of all chains per step",
                        "form": args.form, "chains": len(KS), "sum_K": sumK, "updates_per_step": upd_step,
-                       "l2": "inputs larger than L2 (packed genotypes 0.5 GB; count operands 7.8 GB bf16 + 3.9 GB e4m3)",
+                       "l2": "inputs larger than L2 (packed genotypes 0.5 GB; count operands 7.8 GB bf16 + 1.9 GB e5m2)",
                        "parallelism": f"replicas x{world}" if world > 1 else "1 GPU"},
             "roofline": roof, "cpu_baseline": cpu,
             "e2e": {"value": e2e_value, "unit": "updates/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,

@@ -343,8 +343,8 @@ __global__ void __launch_bounds__(PZ_MAXT, KM <= 6 || INIT ? 3 : 2) k_z_admix_pk
 // roundings of 2^-24 a copy against a rounding at the running sum's size). A
 // call with a product below 2^-100 adds its logarithms singly, so that zeros
 // and infinities come out as they do from the terms.
-// Issue-bound: N = 2,000 x L = 50,000, K = 5 593 -> 149 us a launch, N = 4,999 x
-// L = 40,009, K = 11 1,586 -> 535 us (against k_metro_ratio on the same calls).
+// Issue-bound: N = 2,000 x L = 50,000, K = 5 593 -> 157 us a launch, N = 4,999 x
+// L = 40,009, K = 11 1,586 -> 570 us (against k_metro_ratio on the same calls).
 template <int KM, bool EXACT>
 __global__ void __launch_bounds__(PZ_MAXT, KM <= 11 ? 3 : 2) k_metro_pk(const DevChain* chains, int force, const int4* map = nullptr) {
     constexpr int CH = pz_chunks<KM>();

@@ -5,8 +5,8 @@
 // The reference reads VCF line by line on the host (LoadVCF / AddVCFGenotype,
 // src/load.cpp; GENO_WRITER packs the genotype ids). Here the text is uploaded
 // once and parsed in parallel:
-//   0. upload: through two pinned staging buffers, the host copy of one
-//      overlapping the DMA of the other;
+//   0. upload: the text as it is where the GPU reads pageable memory through
+//      the host's page tables, else through two pinned staging buffers;
 //   1. line index: one warp per 4 KB chunk (coalesced 16-byte loads) counts
 //      its line feeds, an exclusive scan of the counts, then the warp writes
 //      the start offsets of its lines in order;
