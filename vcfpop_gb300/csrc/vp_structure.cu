@@ -604,6 +604,16 @@ bool draw_records(const vp_chain* c) {
     return P.rng == VP_RNG_COUNTER && !P.admix && c->h.nadmburnin == 0 && !P.locpriori && !P.fmodel;
 }
 
+// UpdateP writes the one likelihood table that its own sweep reads (ll_tc_at).
+// A single step may come at another sweep index, or after a batch's sweeps,
+// which write neither: it fills the tables from the frequencies first.
+int refresh_tables(vp_chain* c) {
+    vp_ctx* x = c->ctx;
+    if (!c->h.llnb && !c->plain_lazy) return VP_OK;
+    LAUNCH(x, k_refresh_lt, (cdiv((int64_t)c->P.K * x->L, 256), 256, 0, x->stream), (c->d));
+    return VP_OK;
+}
+
 int launch_step(vp_chain* c, int step, int force, bool sweep = false) {
     vp_ctx* x = c->ctx;
     const vp_params& P = c->P;
@@ -615,9 +625,8 @@ int launch_step(vp_chain* c, int step, int force, bool sweep = false) {
             else SL(c, k_update_p_ctr, (cdiv((int64_t)K * x->L, 256), 1, 1), (256), 0, 1, (int)sweep);
             return VP_OK;
         case VP_STEP_LOGLIK: {
-            // the FP32 stream, whose table UpdateP leaves alone on tensor-core sweeps
-            if (c->h.llnb) LAUNCH(x, k_refresh_lt, (cdiv((int64_t)K * x->L, 256), 256, 0, x->stream), (c->d));
-            int rc = launch_loglik(c, 1);
+            int rc = refresh_tables(c);
+            if (!rc) rc = launch_loglik(c, 1);
             if (rc) return rc;
             SL(c, k_sample_noadmix, (c->h.nsampblk, 1, 1), (SAMPLE_BLOCK), 0, 2, 1, 0);
             return VP_OK;
@@ -625,7 +634,8 @@ int launch_step(vp_chain* c, int step, int force, bool sweep = false) {
         case VP_STEP_UPDATEQ: {
             const unsigned gi = cdiv(x->N, 256);
             if (!P.admix) {
-                int rc = launch_loglik(c, force);
+                int rc = sweep ? VP_OK : refresh_tables(c);
+                if (!rc) rc = launch_loglik(c, force);
                 if (rc) return rc;
                 SL(c, k_sample_noadmix, (ref ? 1 : c->h.nsampblk, 1, 1), (SAMPLE_BLOCK), 0, 2, 0,
                    (int)(sweep && draw_records(c)));
@@ -1503,9 +1513,8 @@ extern "C" int vp_chain_set(vp_chain* c, int32_t field, const void* host, size_t
         }
     }
     CK(cudaMemcpy(p, host, n, cudaMemcpyHostToDevice));
-    if ((field == VP_F_FREQ || (field == VP_F_M && c->h.llnb)) && c->h.lt) {
-        // keep the likelihood tables in step with the frequencies, and both of
-        // them filled whichever the new sweep index reads
+    if (field == VP_F_FREQ && c->h.lt) {
+        // keep the likelihood tables in step with the frequencies
         vp_ctx* x = c->ctx;
         k_refresh_lt<<<cdiv((int64_t)c->P.K * x->L, 256), 256, 0, x->stream>>>(c->d);
         rc = check_launch(x, "k_refresh_lt");
