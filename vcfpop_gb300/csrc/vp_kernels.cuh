@@ -13,7 +13,7 @@ constexpr int KG = 16;          // clusters per thread in the likelihood kernels
 constexpr int LL_BLOCK = 128;   // threads per CTA of the likelihood stream's FMA form
 constexpr int LT_BLOCK = 256;   // threads (= individuals) per CTA of its table form
 constexpr int SUB = 32;         // loci per FP32 sub-sum before folding into FP64
-constexpr double LL_UNIT = 1.0 / 16777216.0;   // the tensor-core likelihood's unit, 2^-24
+constexpr double LL_UNIT = 1.0 / 536870912.0;  // the tensor-core likelihood's unit, 2^-29
 
 struct DevData {
     int32_t N, S, vmax, vstr, maxploidy, maxK, Nw, packed2;
@@ -316,18 +316,67 @@ __device__ __forceinline__ float prior_of(const DevChain& c, int k, int64_t j) {
     if (!c.fmodel) return (float)c.Lambda[k];
     return c.FreqA[j] * (float)c.f[c.fsame ? 0 : k];
 }
-// a logarithm's seven base-32 digits in units of 2^-24 (k_loglik_tc): whole
-// numbers of at most 16 in magnitude, every step exact but the last rounding
-__device__ __forceinline__ void ln_digits(float w, float* d) {
-    float r = w * 16777216.f;
+// ln p as hi + lo in FP32, for k_loglik_tc, whose sums round nothing away: a
+// bias of the logarithm, which the FP32 stream's own roundings cover, would
+// add up over the loci (logf's, near 3e-9, was all of that form's error).
+// p = m 2^e with m in [sqrt(1/2), sqrt(2)); ln m = 2 atanh(s), s = (m - 1) / (m + 1),
+// by the series 2 s (1 + s^2/3 + s^4/5 + ...) with s and its remainder; e ln 2 with
+// an exact head. Within 2^-28.9 of ln p, mean deviation below 3e-11 (against
+// extended precision over 3 million values between 1e-45 and 1). A zero counts
+// as ln_freq's.
+__device__ __forceinline__ void ln_split(float p, float& hi, float& lo) {
+    if (!(p > 0.f)) {
+        hi = ln_freq(p);
+        lo = 0.f;
+        return;
+    }
+    const bool tiny = p < 1.17549435e-38f;
+    const int b = __float_as_int(tiny ? p * 16777216.f : p), e2 = (b - __float_as_int(0.70710678f)) >> 23;
+    const float m = __int_as_float(b - (e2 << 23)), e = (float)(tiny ? e2 - 24 : e2);
+    const float f = m - 1.f, g = m + 1.f, gl = m - (g - 1.f);         // m + 1 = g + gl
+    const float s = __fdividef(f, g), z = s * s;
+    float sl = __fdividef(__fmaf_rn(-s, g, f) - s * gl, g);
+    sl = __fmaf_rn(sl, z, sl);                                        // d atanh(s) = ds (1 + s^2 + ...)
+    float q = 2.f / 13.f;
+    q = __fmaf_rn(q, z, 2.f / 11.f);
+    q = __fmaf_rn(q, z, 2.f / 9.f);
+    q = __fmaf_rn(q, z, 2.f / 7.f);
+    q = __fmaf_rn(q, z, 2.f / 5.f);
+    q = __fmaf_rn(q, z, 2.f / 3.f);
+    constexpr float LN2_H = 0.693145751953125f, LN2_L = (float)(0.69314718055994530942 - 0.693145751953125);
+    const float a = e * LN2_H, t = 2.f * s, h = a + t;
+    const float l = (t - (h - a)) + __fmaf_rn(e, LN2_L, __fmaf_rn(2.f, sl, s * z * q));
+    hi = h + l;
+    lo = l - (hi - h);
+}
+// a logarithm hi + lo in seven digits to base 32 in units of 2^-29
+// (k_loglik_tc), each a value of e4m3. Up to |hi| = 32 they are whole numbers of
+// at most 16 in magnitude. Beyond (frequencies below 1e-14, and zero, whose
+// logarithm counts as -709), a digit above 16 has four significant bits and the
+// next ones take up what it leaves, so they end at the same value. What rounds is
+// the last digit, to a unit, with an offset in (-1/2, 1/2) that runs through
+// the interval evenly from locus to locus: a value that many loci share
+// (1 - j 2^-24 for rare alleles) rounds up at its share of them, and the sums
+// keep what is below the unit.
+__device__ __forceinline__ void ln_digits(float hi, float lo, float offset, float* d) {
+    float r = hi * 536870912.f;
+    const bool wide = fabsf(hi) > 32.f;
 #pragma unroll
     for (int j = 6; j >= 0; --j) {
         const float u = (float)(1u << (5 * j));
-        d[j] = rintf(r * (1.f / u));
+        // (at most 2^9 + 1/2 in all: no digit leaves its range)
+        if (j == 3) r += __fmaf_rn(lo, 536870912.f, offset);
+        const float x = r * (1.f / u);
+        d[j] = rintf(x);
+        if (wide) {
+            // the step of e4m3 at x: an eighth of the power of two below it
+            const float s = __uint_as_float((__float_as_uint(fmaxf(fabsf(x), 8.f)) & 0x7F800000u) - (3u << 23));
+            d[j] = fminf(fmaxf(rintf(x / s) * s, -448.f), 448.f);
+        }
         r = __fmaf_rn(-d[j], u, r);
     }
 }
-// two whole numbers of at most 16 as e4m3 bytes (the second in the low byte)
+// two digits as e4m3 bytes (the second in the low byte)
 __device__ __forceinline__ uint32_t e4m3x2(float hi, float lo) {
     uint16_t r;
     asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(r) : "f"(hi), "f"(lo));
@@ -339,9 +388,12 @@ __device__ __forceinline__ uint32_t e4m3x2(float hi, float lo) {
 // 1 and 16 on for allele 0), the 16-byte chunks of row r exchanged by r / 2 mod
 // 4 (the 64-byte swizzle)
 __device__ __forceinline__ void write_digits(const DevChain& c, int k, int64_t l, const float* p) {
-    float d0[7], d1[7];
-    ln_digits(ln_freq(p[0]), d0);
-    ln_digits(ln_freq(p[1]), d1);
+    float d0[7], d1[7], hi, lo;
+    const float offset = (float)(int32_t)((uint32_t)l * 0x9E3779B9u) * (0.998f / 4294967296.f);   // l / golden ratio, mod 1
+    ln_split(p[0], hi, lo);
+    ln_digits(hi, lo, offset, d0);
+    ln_split(p[1], hi, lo);
+    ln_digits(hi, lo, offset, d1);
     char* t = c.ltd + (l >> 5) * (c.llnb * 64);
     const int j = (int)(l & 15), h = (int)(l >> 4) & 1, in = 4 * (2 * (j >> 3) + (j & 1)) + ((j >> 1) & 3);
 #pragma unroll
@@ -853,24 +905,14 @@ __device__ double sample_warp(const DevChain& c, int i, int m, int lane, bool su
     Philox ph;
     ph.init(c.seed, ST_Q | ((uint32_t)m << 4), (uint32_t)i, 0);
     const float u = ph.uniformf();
-    if (ll_tc_at(c, m)) {
-        // the tensor-core form's partials: whole numbers of 2^-24
-        long long a = 0;
-        const long long* P = reinterpret_cast<const long long*>(c.LLp);
+    const int nch = ll_tc_at(c, m) ? c.tcchunk : c.nchunk;
 #pragma unroll 8
-        for (int ch = ch0; ch < c.tcchunk; ch += step)
-            if (kk < K) a += P[((int64_t)ch * N + i) * K + kk];
-        for (int o = 1 << lg; o < 32; o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        v0 = (double)a * LL_UNIT;
-    } else {
-#pragma unroll 8
-        for (int ch = ch0; ch < c.nchunk; ch += step) {
-            const double* p = c.LLp + ((int64_t)ch * N + i) * K;
-            if (kk < K) v0 += p[kk];
-            if (h1) v1 += p[k1];
-        }
-        for (int o = 1 << lg; o < 32; o <<= 1) v0 += __shfl_xor_sync(0xffffffffu, v0, o);
+    for (int ch = ch0; ch < nch; ch += step) {
+        const double* p = c.LLp + ((int64_t)ch * N + i) * K;
+        if (kk < K) v0 += p[kk];
+        if (h1) v1 += p[k1];
     }
+    for (int o = 1 << lg; o < 32; o <<= 1) v0 += __shfl_xor_sync(0xffffffffu, v0, o);
     double* LL = c.LL + (int64_t)i * K;
     float* Q = c.Q + (int64_t)i * K;
     int32_t* Mi = c.Mi + (int64_t)i * K;

@@ -98,17 +98,19 @@ struct Ring {
 };
 
 // ---- the likelihood, exact ------------------------------------------------
-// ln p is taken as a whole number of 2^-24 units (|ln p| < 2^10, so 34 bits) in
-// seven digits to base 32, each a whole number of at most 16 in magnitude and
-// so exact in e4m3, as the copies 0, 1, 2 are. A call adds at most 2 x 16 to a
-// digit's sum and the FP32 accumulator holds whole numbers up to 2^24, so the
-// sums of up to 2^19 loci are exact whatever the order of the adds, and the
-// digits combine in 64-bit integers. What rounds is the logarithm itself (FP32,
-// as in the FP32 forms) and its unit, an FP32 ulp of 0.5 to 1: against 64 bits
-// LL is 2.5e-9 off, where the FP32 stream is 3.1e-9 to 5.7e-9 off (N = 512 to
-// 2,000, L = 4,096 to 60,000, K = 3 to 16).
+// ln p is taken to about 2^-29 of its value (ln_split) in units of 2^-29, in
+// seven digits to base 32, exact in e4m3 as the copies 0, 1, 2 are (ln_digits).
+// A digit is at most 352 in magnitude (in the logarithm of a zero frequency; at
+// most 64 else, 16 from p = 1e-14 up), so a locus adds at most 2 x 352 to its
+// sum, and the FP32 accumulator holds whole numbers up to 2^24: the sums of 2^14
+// loci are exact whatever the order of the adds, and the digits combine in
+// 64-bit integers. What rounds is a copy's logarithm.
+// LL against float64, rms relative, and the FP32 stream's on the same inputs:
+// frequencies from Beta(1/2, 1/2) 3e-12 to 4e-12 and 1.7e-9 to 4.0e-9, from a 1/x
+// spectrum 1e-11 and 3.3e-9, around 1%, 0.1%, 0.01% and 0.001% 7e-12 to 3.4e-11 and
+// 2.7e-9 to 5.9e-9 (N = 512 and 1,000, L = 32,000 and 100,000, K = 3, 6 and 10).
 constexpr int LL_LOCI = 32;                        // loci of a stage: 64 A bytes (copies of allele 1 and 0 of each)
-constexpr int LL_MAXST = (1 << 19) / LL_LOCI;
+constexpr int LL_MAXST = (1 << 14) / LL_LOCI;
 constexpr int LL_M = 256;                          // individuals per CTA: two 128-row tiles share a B stage
 constexpr int LL_TEAM = 8;                         // builder warps of a stage: one per 32 individuals
 constexpr int LL_BW = 2 * LL_TEAM;                 // two teams take alternate stages
@@ -232,7 +234,7 @@ __global__ void __launch_bounds__(LL_THREADS, NB <= 80 ? 2 : 1) k_loglik_tc(cons
         const bool got = warp_wait(smem_u32(&accum), 0, &s_abort, err, 12) && !*(volatile int*)&s_abort;
         fence_after();
         const int i = ib + (lane >> 1) + 16 * (lane & 1);
-        long long* out = reinterpret_cast<long long*>(c.LLp) + ((int64_t)vb.y * D.N + i) * K;
+        double* out = c.LLp + ((int64_t)vb.y * D.N + i) * K;
 #pragma unroll 1
         for (int k = team; k < K; k += 2) {
             float v[8];
@@ -241,7 +243,7 @@ __global__ void __launch_bounds__(LL_THREADS, NB <= 80 ? 2 : 1) k_loglik_tc(cons
             long long t = 0;
 #pragma unroll
             for (int j = 6; j >= 0; --j) t = t * 32 + __float2int_rn(v[j]);
-            out[k] = t;
+            out[k] = (double)t * LL_UNIT;
         }
     } else if (warp == LL_BW) {
         if (lane == 0) {
