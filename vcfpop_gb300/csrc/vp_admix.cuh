@@ -341,8 +341,8 @@ __global__ void __launch_bounds__(PZ_MAXT, KM <= 6 || INIT ? 3 : 2) k_z_admix_pk
 // in [1, 2) and an integer exponent each, and one logarithm of the mantissas'
 // ratio closes a range, which rounds less than a sum of FP32 logarithms (two
 // roundings of 2^-24 a copy against a rounding at the running sum's size). A
-// call with a product below 2^-100 adds its logarithms singly, so that zeros
-// and infinities come out as they do from the terms.
+// call with a product outside 2^-100 to 2^28 adds its logarithms singly, so that
+// zeros, infinities and NaNs come out as they do from the terms.
 // Issue-bound: N = 2,000 x L = 50,000, K = 5 593 -> 157 us a launch, N = 4,999 x
 // L = 40,009, K = 11 1,586 -> 570 us (against k_metro_ratio on the same calls).
 template <int KM, bool EXACT>
@@ -425,7 +425,9 @@ __global__ void __launch_bounds__(PZ_MAXT, KM <= 11 ? 3 : 2) k_metro_pk(const De
             f2_unpack(x1, a1, b1);
             f2_unpack(x0, a0, b0);
             const float p1 = a1 * b1, p0 = a0 * b0;
-            const bool fine = p1 > 7.888609e-31f && p0 > 7.888609e-31f;   // 2^-100
+            // 2^-100 <= p < 2^28, 128 exponents, by the bits
+            constexpr uint32_t LO = 27u << 23;
+            const bool fine = (((__float_as_uint(p1) - LO) | (__float_as_uint(p0) - LO)) & 0xC0000000u) == 0;
             if (code != 3u) {
                 if (fine) {
                     R1 *= p1;
