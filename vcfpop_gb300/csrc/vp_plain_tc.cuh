@@ -330,7 +330,9 @@ __global__ void __launch_bounds__(CT_IND) k_onehot(const DevChain* chains, int f
     const int i = vb.x * CT_IND + t;
     z[t] = i < N ? c.Z[i] : 0xFFFF;
     __syncthreads();
-    if (i < N) atomicAdd(&nk[z[t]], 1);
+    // a label set from outside may be any number: one without a row is in no
+    // cluster, here and in the rows below (as in k_count_packed)
+    if (z[t] < NB) atomicAdd(&nk[z[t]], 1);
     // thread t: words t & 31 of rows t / 32, t / 32 + 4, ...
     const int w = t & 31, i0 = 16 * (w >> 2) + 8 * ((w >> 1) & 1) + (w & 1);
     uint32_t* B = reinterpret_cast<uint32_t*>(c.oh + (int64_t)vb.x * NB * 128);
