@@ -303,6 +303,11 @@ int vp_debug_gemm_time(int32_t M, int32_t N, int32_t K, int32_t BN, int32_t piec
  * (*status_after: 0) and the largest difference of its result from the exact
  * one (*max_err_after). */
 int vp_debug_gemm_wait_timeout(int32_t* status_timeout, int32_t* status_after, double* max_err_after);
+/* Diagnostic: on != 0 gives a chain's plain-form tensor-core kernels (the
+ * likelihood and the counts of 2-bit data) the same stalled stage barriers, so
+ * their waits run out after a short poll limit and the chain's results are
+ * void; 0 takes it back. */
+int vp_debug_chain_stall(vp_chain* chain, int32_t on);
 
 /* The likelihood accumulation of UpdateQNoAdmix (src/structure.cpp:902-932;
  * the part BAYESIAN<REAL>::UpdateQNoAdmixCUDA offloads, src/structureCUDA.cpp:

@@ -53,6 +53,7 @@ struct DevChain {
     int32_t llnb, tcper, tcchunk;
     int32_t pz_slices, nmetro, nlnlp, kp, nsampblk, zadm_lc;
     int32_t ntrace;       // capacity of lnlTrace in records
+    int32_t stall;        // diagnostics only: bytes the stage barriers of k_loglik_tc and k_count_tc expect beyond their copies'
     double lambda, alpha, stdalpha, maxalpha, alphapriora, alphapriorb, maxr, epsr, epseta, epsgamma;
     double pmeanf, pstdf, stdf;
     uint64_t seed;

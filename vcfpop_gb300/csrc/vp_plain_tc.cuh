@@ -9,8 +9,8 @@
 // tcgen05.mma reads its A operand; the narrow B operand comes through shared
 // memory. A ring of A stages in tensor memory lets the decoding run ahead of
 // the MMAs. Every wait is bounded: on time-out the CTA records an error in its
-// chain's control block (read with the chain's results), waits for what is in
-// flight, frees its tensor memory and returns.
+// chain's control block (read with the chain's results), waits for the copies
+// and MMAs in flight, frees its tensor memory and returns.
 #pragma once
 #include "vp_admix.cuh"
 #include "vp_tc.cuh"
@@ -69,9 +69,11 @@ __device__ __forceinline__ uint32_t bar_done(uint32_t bar, uint32_t parity) {
 // whole warp, which takes one way. The first poll is the common case and all
 // that is inlined: a stage's waits and arrivals are a chain of dependent
 // instructions on few warps, and their length sets the kernels' pace. A wait
-// that runs out, or finds that another warp's has, ends the CTA's work (false).
+// that runs out (abort[1] polls), or finds that another warp's has (abort[0]),
+// ends the CTA's work (false).
 __device__ __noinline__ bool bar_wait_long(uint32_t bar, uint32_t parity, bool warp, volatile int* abort, int* err, int code) {
-    for (uint32_t it = 0; it < tc::SPIN_LIMIT; ++it) {
+    const int limit = abort[1];
+    for (int it = 0; it < limit; ++it) {
         const uint32_t d = bar_done(bar, parity);
         if (warp ? __all_sync(0xffffffffu, d) : d) return true;
         if ((it & 255) == 255 && (warp ? __any_sync(0xffffffffu, *abort) : *abort)) return false;
@@ -86,6 +88,8 @@ __device__ __forceinline__ bool thread_wait(uint32_t bar, uint32_t parity, volat
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort, int* err, int code) {
     return __all_sync(0xffffffffu, bar_done(bar, parity)) || bar_wait_long(bar, parity, true, abort, err, code);
 }
+// polls of a wait; few where a diagnostic has the waits run out (DevChain::stall)
+__device__ __forceinline__ int poll_limit(const DevChain& c) { return c.stall ? 1 << 12 : (int)tc::SPIN_LIMIT; }
 // a place in a ring of ST stages: its index and how often it has come round
 template <int ST>
 struct Ring {
@@ -163,7 +167,7 @@ __global__ void __launch_bounds__(LL_THREADS, NB <= 80 ? 2 : 1) k_loglik_tc(cons
     __shared__ __align__(16) uint32_t sW[LL_BW][LL_PF][LL_LOCI][2];
     __shared__ uint64_t full[ST], fullB[ST], empty[ST], accum;
     __shared__ uint32_t s_tmem;
-    __shared__ int s_abort;
+    __shared__ int s_abort[2];
     const VBlock vb = vblock(map);
     const DevChain& c = chains[vb.z];
     if (map && run_over(c)) return;
@@ -177,7 +181,8 @@ __global__ void __launch_bounds__(LL_THREADS, NB <= 80 ? 2 : 1) k_loglik_tc(cons
     if (threadIdx.x == 0) {
         for (int s = 0; s < ST; ++s) { mbar_init(&full[s], 8); mbar_init(&fullB[s], 1); mbar_init(&empty[s], 1); }
         mbar_init(&accum, 1);
-        s_abort = 0;
+        s_abort[0] = 0;
+        s_abort[1] = poll_limit(c);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == LL_BW) {
@@ -221,7 +226,7 @@ __global__ void __launch_bounds__(LL_THREADS, NB <= 80 ? 2 : 1) k_loglik_tc(cons
             uint32_t r[16];
             calls_to_e4m3(tr.codes(w0), r);
             calls_to_e4m3(tr.codes(w1), r + 8);
-            if (r_.round && !warp_wait(empty0 + 8 * s, (r_.round & 1) ^ 1, &s_abort, err, 11)) break;
+            if (r_.round && !warp_wait(empty0 + 8 * s, (r_.round & 1) ^ 1, s_abort, err, 11)) break;
             fence_after();
             tmem_st16(ring + lanes + (uint32_t)(s * 32 + tile * 16), r);
             wait_st();
@@ -231,7 +236,7 @@ __global__ void __launch_bounds__(LL_THREADS, NB <= 80 ? 2 : 1) k_loglik_tc(cons
         }
         cp_async_wait<0>();
         // the digits' sums of this lane's individual
-        const bool got = warp_wait(smem_u32(&accum), 0, &s_abort, err, 12) && !*(volatile int*)&s_abort;
+        const bool got = warp_wait(smem_u32(&accum), 0, s_abort, err, 12) && !*(volatile int*)s_abort;
         fence_after();
         const int i = ib + (lane >> 1) + 16 * (lane & 1);
         double* out = c.LLp + ((int64_t)vb.y * D.N + i) * K;
@@ -251,7 +256,7 @@ __global__ void __launch_bounds__(LL_THREADS, NB <= 80 ? 2 : 1) k_loglik_tc(cons
             Ring<ST> r_;
             for (int it = 0; it < n; ++it, r_.step()) {
                 const int s = r_.s;
-                if (!thread_wait(fullB0 + 8 * s, r_.round & 1, &s_abort, err, 15) || !thread_wait(full0 + 8 * s, r_.round & 1, &s_abort, err, 13)) break;
+                if (!thread_wait(fullB0 + 8 * s, r_.round & 1, s_abort, err, 15) || !thread_wait(full0 + 8 * s, r_.round & 1, s_abort, err, 13)) break;
                 fence_after();
                 const uint64_t bd = d0 + (uint64_t)((s * NB * 64) >> 4);
 #pragma unroll
@@ -262,21 +267,25 @@ __global__ void __launch_bounds__(LL_THREADS, NB <= 80 ? 2 : 1) k_loglik_tc(cons
                                    IDESC, (it | kk) ? 1u : 0u);
                 mma_commit(&empty[s]);
             }
+            // also when a wait has run out: it arrives once the MMAs issued are done,
+            // and tensor memory is not given back before
             mma_commit(&accum);
+            mbar_wait(&accum, 0);
         }
     } else if (lane == 0) {
+        const uint32_t tx = NB * 64 + c.stall;
         const char* src = reinterpret_cast<const char*>(c.ltd) + (int64_t)st0 * (NB * 64);
         int issued = 0;
         Ring<ST> r_;
         for (int it = 0; it < n; ++it, r_.step()) {
             const int s = r_.s;
-            if (r_.round && !thread_wait(empty0 + 8 * s, (r_.round & 1) ^ 1, &s_abort, err, 14)) break;
-            mbar_expect_tx(&fullB[s], NB * 64);
+            if (r_.round && !thread_wait(empty0 + 8 * s, (r_.round & 1) ^ 1, s_abort, err, 14)) break;
+            mbar_expect_tx(&fullB[s], tx);
             bulk_load(&sB[s][0], src + (int64_t)it * (NB * 64), NB * 64, &fullB[s]);
             issued = it + 1;
         }
         // every copy issued has landed before the CTA may exit
-        for (int it = issued > ST ? issued - ST : 0; it < issued; ++it) mbar_wait(&fullB[it % ST], (it / ST) & 1);
+        for (int it = issued > ST ? issued - ST : 0; it < issued; ++it) mbar_wait(&fullB[it % ST], (it / ST) & 1, s_abort[1]);
     }
     fence_before();
     __syncthreads();
@@ -354,10 +363,10 @@ __global__ void __launch_bounds__(CT_THREADS, NB == 16 ? 2 : 1) k_count_tc(const
     constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NB >> 3) << 17) | (8u << 24);
     __shared__ __align__(1024) unsigned char sB[ST][NB * 128];
     __shared__ __align__(16) unsigned char sG[CT_BW][PF][32 * CT_PITCH];
-    __shared__ uint64_t full[ST], fullB[ST], empty[ST], dfull[2], dempty[2];
+    __shared__ uint64_t full[ST], fullB[ST], empty[ST], dfull[2], dempty[2], drained;
     __shared__ int s_nk[NB];
     __shared__ uint32_t s_tmem;
-    __shared__ int s_abort;
+    __shared__ int s_abort[2];
     const VBlock vb = vblock(map);
     const DevChain& c = chains[vb.z];
     if (map && counts_over(c)) return;
@@ -369,7 +378,9 @@ __global__ void __launch_bounds__(CT_THREADS, NB == 16 ? 2 : 1) k_count_tc(const
     if (threadIdx.x == 0) {
         for (int s = 0; s < ST; ++s) { mbar_init(&full[s], 4); mbar_init(&fullB[s], 1); mbar_init(&empty[s], 1); }
         for (int d = 0; d < 2; ++d) { mbar_init(&dfull[d], 1); mbar_init(&dempty[d], 4); }
-        s_abort = 0;
+        mbar_init(&drained, 1);
+        s_abort[0] = 0;
+        s_abort[1] = poll_limit(c);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == CT_BW) {
@@ -407,7 +418,7 @@ __global__ void __launch_bounds__(CT_THREADS, NB == 16 ? 2 : 1) k_count_tc(const
             cp_async_commit();
         };
         auto drain = [&](int g) {
-            if (!warp_wait(dfull0 + 8 * (g & 1), (g >> 1) & 1, &s_abort, err, 22)) return false;
+            if (!warp_wait(dfull0 + 8 * (g & 1), (g >> 1) & 1, s_abort, err, 22)) return false;
             fence_after();
 #pragma unroll
             for (int b = 0; b < NB; b += 16) {
@@ -439,7 +450,7 @@ __global__ void __launch_bounds__(CT_THREADS, NB == 16 ? 2 : 1) k_count_tc(const
             const uint4 x = *reinterpret_cast<const uint4*>(my), y = *reinterpret_cast<const uint4*>(my + 16);
             __syncwarp();
             const uint32_t wd[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
-            if (r_.round && !warp_wait(empty0 + 8 * s, (r_.round & 1) ^ 1, &s_abort, err, 21)) { run = false; break; }
+            if (r_.round && !warp_wait(empty0 + 8 * s, (r_.round & 1) ^ 1, s_abort, err, 21)) { run = false; break; }
             fence_after();
             const uint32_t a = ring + lanes + (uint32_t)(s * 32);
 #pragma unroll
@@ -471,26 +482,18 @@ __global__ void __launch_bounds__(CT_THREADS, NB == 16 ? 2 : 1) k_count_tc(const
             const int last = ((n - 1) & ~1), g = last / CT_GROUP, r = last - g * CT_GROUP;    // the team's last stage
             for (int d = max(0, r >= DRAIN_AT ? g : g - 1); d < ngr && run; ++d) run = drain(d);
         }
-        if (!run) {
-            // an abort: the MMAs issued must have ended before tensor memory goes
-            // (the MMA warp commits to both barriers when it gives up)
-            mbar_wait(&dfull[(ngr - 1) & 1], ((ngr - 1) >> 1) & 1);
-            a1[0] = -1;
-        }
+        if (!run) a1[0] = -1;                // nothing is written
     } else if (warp == CT_BW) {
         if (lane == 0) {
             const uint64_t d0 = tc::sw_desc(smem_u32(&sB[0][0]), 128);
-            bool run = true;
             Ring<ST> r_;
             Ring<CT_GROUP> g_;
-            for (int it = 0; it < n && run; ++it, r_.step(), g_.step()) {
+            for (int it = 0; it < n; ++it, r_.step(), g_.step()) {
                 const int s = r_.s, g = (int)g_.round;
                 const bool first = g_.s == 0;
-                if ((first && g >= 2 && !thread_wait(dempty0 + 8 * (g & 1), ((g >> 1) & 1) ^ 1, &s_abort, err, 25)) ||
-                    !thread_wait(fullB0 + 8 * s, r_.round & 1, &s_abort, err, 26) || !thread_wait(full0 + 8 * s, r_.round & 1, &s_abort, err, 23)) {
-                    run = false;
+                if ((first && g >= 2 && !thread_wait(dempty0 + 8 * (g & 1), ((g >> 1) & 1) ^ 1, s_abort, err, 25)) ||
+                    !thread_wait(fullB0 + 8 * s, r_.round & 1, s_abort, err, 26) || !thread_wait(full0 + 8 * s, r_.round & 1, s_abort, err, 23))
                     break;
-                }
                 fence_after();
                 const uint64_t bd = d0 + (uint64_t)((s * NB * 128) >> 4);
 #pragma unroll
@@ -500,24 +503,24 @@ __global__ void __launch_bounds__(CT_THREADS, NB == 16 ? 2 : 1) k_count_tc(const
                 mma_commit(&empty[s]);
                 if (g_.s == CT_GROUP - 1 || it == n - 1) mma_commit(&dfull[g & 1]);
             }
-            if (!run) {
-                mma_commit(&dfull[0]);
-                mma_commit(&dfull[1]);
-            }
+            // as the likelihood's accum: the MMAs issued are done before tensor memory goes
+            mma_commit(&drained);
+            mbar_wait(&drained, 0);
         }
     } else if (warp == CT_BW + 1) {
         if (lane == 0) {
+            const uint32_t tx = NB * 128 + c.stall;
             int issued = 0;
             Ring<ST> r_;
             for (int it = 0; it < n; ++it, r_.step()) {
                 const int s = r_.s;
-                if (r_.round && !thread_wait(empty0 + 8 * s, (r_.round & 1) ^ 1, &s_abort, err, 24)) break;
-                mbar_expect_tx(&fullB[s], NB * 128);
+                if (r_.round && !thread_wait(empty0 + 8 * s, (r_.round & 1) ^ 1, s_abort, err, 24)) break;
+                mbar_expect_tx(&fullB[s], tx);
                 bulk_load(&sB[s][0], c.oh + (int64_t)it * (NB * 128), NB * 128, &fullB[s]);
                 issued = it + 1;
             }
             // every copy issued has landed before the CTA may exit
-            for (int it = issued > ST ? issued - ST : 0; it < issued; ++it) mbar_wait(&fullB[it % ST], (it / ST) & 1);
+            for (int it = issued > ST ? issued - ST : 0; it < issued; ++it) mbar_wait(&fullB[it % ST], (it / ST) & 1, s_abort[1]);
         }
     } else if (lane < NB) {
         const int* nk = reinterpret_cast<const int*>(c.oh + (int64_t)n * NB * 128);

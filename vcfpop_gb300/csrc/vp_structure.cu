@@ -2865,6 +2865,17 @@ extern "C" int vp_debug_gemm_wait_timeout(int32_t* status_timeout, int32_t* stat
     return rc;
 }
 
+// the same for a chain's own tensor-core kernels (k_loglik_tc, k_count_tc)
+extern "C" int vp_debug_chain_stall(vp_chain* c, int32_t on) {
+    if (!c) { vp_set_error("null chain"); return VP_E_ARG; }
+    vp_ctx* x = c->ctx;
+    cudaSetDevice(x->device);
+    c->h.stall = on ? 16 : 0;
+    CK(cudaStreamSynchronize(x->stream));
+    CK(cudaMemcpy(&c->d->stall, &c->h.stall, sizeof c->h.stall, cudaMemcpyHostToDevice));
+    return VP_OK;
+}
+
 extern "C" int vp_debug_gemm_e4m3(const uint8_t* A, const uint8_t* B, int32_t M, int32_t N, int32_t K, int32_t BN,
                                   int32_t piece, int32_t stages, int32_t mt, float* D) {
     if (!A || !B || !D || M <= 0 || N <= 0 || K <= 0 || K % 128 || N % BN || BN % piece || piece % 16 || piece > 256 ||
