@@ -38,3 +38,60 @@ def test_a_run_ends_and_the_next_chain_is_right(N, L, K):
     for x in (got, want):
         x.close()
     ctx.close()
+
+
+def _raises(f, *a):
+    with pytest.raises(B.VpError, match="timed out"):
+        f(*a)
+
+
+# the counts of 600 individuals run on the tensor cores, with 6 clusters the
+# likelihood too
+@pytest.mark.parametrize("L,K", [(6000, 4), (8200, 6)])
+def test_every_way_to_the_state_reports(L, K):
+    c, ctx, ch = _chain(_calls(600, L, K), K)
+    other = S.Chain(ctx, _params(K, 5))
+    _stall(ch, 1)
+    ch.run(2)
+    for f in ("FREQ", "Q", "Z", "NI", "MI", "LL", "ALPHA", "M", "FF", "LOCP"):
+        _raises(ch.get, f)
+    _raises(ch.result)
+    _raises(ch.step, "UPDATEP")
+    _raises(S.finish, [ch])
+    _raises(ch.result, True)
+    _raises(ch.divergence)
+    S.finish([other])                        # the context's other chain is well
+    other.divergence()
+    assert other.result()["nr"] == 1
+    ch.close()
+    other.close()
+    ctx.close()
+
+
+def test_steps_report():
+    c, ctx, ch = _chain(_calls(600, 8200, 1), 6)
+    ch.step("UPDATEP")
+    _stall(ch, 1)
+    _raises(ch.step, "UPDATEQ")
+    ch.close()
+    ch = S.Chain(ctx, _params(6, 5))
+    _stall(ch, 1)
+    _raises(ch.step, "UPDATEZ")
+    ch.close()
+    ctx.close()
+
+
+def test_a_cohort_reports():
+    c, ctx, ch = _chain(_calls(600, 8200, 2), 6)
+    other = S.Chain(ctx, _params(6, 5))
+    _stall(ch, 1)
+    co = S.Cohort()
+    co.set([ch, other])
+    co.run(3)
+    _raises(co.sync)
+    _raises(ch.get, "Z")
+    assert other.get("M")[0] == 3
+    co.close()
+    for x in (ch, other):
+        x.close()
+    ctx.close()

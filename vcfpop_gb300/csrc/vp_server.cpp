@@ -194,6 +194,11 @@ bool advance(vp_server* s, Req* r, bool* finished) {
     }
     if (r->finishing) {
         if (r->inflight == 0) {
+            if (int rc = vp_chain_check(r->chain)) {
+                fail(s, r, rc, "run failed");
+                *finished = true;
+                return true;
+            }
             std::lock_guard<std::mutex> lk(s->mu);
             r->state = VP_REQ_DONE;
             r->t_done = s->now();

@@ -555,6 +555,15 @@ bool count_tc_form(const vp_ctx* x, int K) {
     return x->packed2 && K <= 32 && (x->N < 512 ? calls >= 1 << 21 : x->N <= 1024 || calls >= 1 << 22);
 }
 
+// Chains whose plain form may end a launch with an error in their control block
+// instead of a result (a wait of k_loglik_tc or k_count_tc that ran out): state
+// is handed out, and steps and runs end, only after a look at it.
+bool may_time_out(const vp_chain* c) { return c->h.llnb || (!c->P.admix && count_tc_form(c->ctx, c->P.K)); }
+int timed_out(int code) {
+    if (!code) return VP_OK;
+    vp_set_error("a tensor-core kernel of this chain timed out (code %d): its results are void", code);
+    return VP_E_CUDA;
+}
 // the no-admixture counts: from bit planes on 2-bit packed data with at
 // least 32 words per locus (N >= 512) when the masks of a cluster group fit in
 // shared memory, else the per-individual pass
@@ -843,6 +852,14 @@ int ensure_plain(vp_chain* c) {
     LAUNCH(x, k_set_plain, (1, 1, 0, x->stream), (c->d, h.lt, h.ltd, h.LLp));
     LAUNCH(x, k_refresh_lt, (cdiv((int64_t)c->P.K * x->L, 256), 256, 0, x->stream), (c->d));
     return VP_OK;
+}
+
+int vp_chain_check(const vp_chain* c) {
+    if (!may_time_out(c)) return VP_OK;
+    int code = 0;
+    CK(cudaMemcpyAsync(&code, &c->h.ctl->err, sizeof code, cudaMemcpyDeviceToHost, c->ctx->stream));
+    CK(cudaStreamSynchronize(c->ctx->stream));
+    return timed_out(code);
 }
 
 cudaError_t vp_pool_alloc(void** p, size_t bytes, int device, cudaStream_t s) { return dev_alloc(p, bytes, device, s); }
@@ -1329,7 +1346,9 @@ int vp_finish_issue(vp_chain** cs, int32_t n) {
 
 extern "C" int vp_finish(vp_chain** cs, int32_t n) {
     int rc = vp_finish_issue(cs, n);
-    return rc ? rc : vp_sync(cs[0]->ctx);
+    if (!rc) rc = vp_sync(cs[0]->ctx);
+    for (int i = 0; i < n && !rc; ++i) rc = vp_chain_check(cs[i]);
+    return rc;
 }
 
 const vp_dataset* vp_chain_dataset(const vp_chain* c) { return c->ctx->hold; }
@@ -1345,6 +1364,7 @@ extern "C" int vp_chain_divergence(vp_chain* c, double* H, double* D, double* Hl
     if (!c->arranged) { vp_set_error("the chain is not finished (vp_finish arranges the mean frequencies)"); return VP_E_STATE; }
     vp_ctx* x = c->ctx;
     cudaSetDevice(x->device);
+    if (int rc0 = vp_chain_check(c)) return rc0;
     const int K = c->P.K;
     const int npairs = K * (K + 1) / 2;
     const int nch = (int)std::min<int64_t>(DIV_CHUNKS, std::max<int64_t>(1, x->L / 256));
@@ -1391,7 +1411,7 @@ extern "C" int vp_chain_sizes(vp_chain* c, vp_result* r) {
     CK(cudaStreamSynchronize(c->ctx->stream));
     Ctl ctl;
     CK(cudaMemcpy(&ctl, c->h.ctl, sizeof ctl, cudaMemcpyDeviceToHost));
-    if (ctl.err) { vp_set_error("a tensor-core kernel of this chain timed out (code %d): its results are void", ctl.err); return VP_E_CUDA; }
+    if (int rc = timed_out(ctl.err)) return rc;
     r->nr = ctl.nr; r->nlnl = ctl.nlnl;
     return VP_OK;
 }
@@ -1468,7 +1488,10 @@ extern "C" int vp_chain_get(vp_chain* c, int32_t field, void* host, size_t bytes
     cudaSetDevice(c->ctx->device);
     if (int rc0 = ensure_counts(c)) return rc0;
     // (a single array's copy below is ordered after the stream's work)
-    if (field == VP_F_FF || field == VP_F_LOCP) CK(cudaStreamSynchronize(c->ctx->stream));
+    if (field == VP_F_FF || field == VP_F_LOCP) {
+        CK(cudaStreamSynchronize(c->ctx->stream));
+        if (int rc0 = vp_chain_check(c)) return rc0;
+    }
     if (field == VP_F_FF) {
         size_t K = c->P.K;
         if (bytes != 2 * K * 8) { vp_set_error("field %d holds %zu bytes", field, 2 * K * 8); return VP_E_ARG; }
@@ -1483,6 +1506,7 @@ extern "C" int vp_chain_get(vp_chain* c, int32_t field, void* host, size_t bytes
     if (bytes != n) { vp_set_error("field %d holds %zu bytes, not %zu", field, n, bytes); return VP_E_ARG; }
     vp_touch_pages(host, n);
     CK(cudaMemcpyAsync(host, p, n, cudaMemcpyDeviceToHost, c->ctx->stream));
+    if (int rc0 = vp_chain_check(c)) return rc0;
     CK(cudaStreamSynchronize(c->ctx->stream));
     return VP_OK;
 }
@@ -1540,8 +1564,8 @@ extern "C" int vp_chain_step(vp_chain* c, int32_t step) {
         return VP_E_STATE;
     }
     rc = launch_step(c, step, 0);
-    if (rc) return rc;
-    return vp_sync(c->ctx);
+    if (!rc) rc = vp_sync(c->ctx);
+    return rc ? rc : vp_chain_check(c);
 }
 
 // ===================== cohorts: runs of different datasets in shared launches =====================
@@ -1788,6 +1812,8 @@ extern "C" int vp_cohort_sync(vp_cohort* h) {
     cudaSetDevice(h->device);
     CK(cudaStreamSynchronize(h->stream));
     cohort_reap(h, true);
+    for (const vp_chain* c : h->chains)
+        if (int rc = vp_chain_check(c)) return rc;
     return VP_OK;
 }
 
