@@ -339,8 +339,10 @@ int vp_loglik_packed2_noalloc(const uint32_t* geno, int32_t n_ind, int64_t n_loc
 
 /* Contexts, chains and batches take device memory from a stream-ordered
  * pool per device that keeps freed blocks for the next run (no map/unmap
- * between runs, frees do not wait for the device). This gives the kept
- * blocks back to the device (after a device synchronisation). */
+ * between runs, frees do not wait for the device); the ingest and filter calls
+ * take theirs from a second one, which keeps at most 256 MiB after a call. This
+ * gives the kept blocks of both back to the device (after a device
+ * synchronisation). */
 int vp_release_memory(int device);
 
 /* The CUDA stream (cudaStream_t) every launch of this context goes to. */

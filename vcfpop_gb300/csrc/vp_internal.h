@@ -55,9 +55,11 @@ int64_t vp_request_bytes(const vp_dataset* ds, const vp_params* P, int nsm);
 // vp_open with the context's stream at a CUDA stream priority (lower numbers
 // run first; 0 is the default)
 int vp_open_ex(const vp_dataset* ds, int device, int priority, vp_ctx** out);
-// device memory from the library's pool, which keeps freed blocks for the next
-// call (freed with cudaFreeAsync; vp_release_memory gives the kept blocks back)
+// device memory for one call, from a pool that keeps up to 256 MiB of freed
+// blocks for the next (freed with cudaFreeAsync before the call's last wait;
+// vp_pool_trim and vp_release_memory give the kept blocks back)
 cudaError_t vp_pool_alloc(void** p, size_t bytes, int device, cudaStream_t s);
+cudaError_t vp_pool_trim(int device);
 // maps the pages of a caller's buffer before the device writes all of it
 void vp_touch_pages(void* host, size_t bytes);
 // one more reference to a dataset; vp_dataset_free drops one

@@ -458,6 +458,7 @@ extern "C" int vp_server_open(int device, int64_t mem_budget, int32_t max_active
         s->prio_least = s->prio_greatest = 0;
     if (mem_budget == 0) {
         size_t fr = 0, tot = 0;
+        vp_pool_trim(device);                // what ingest kept is free memory too
         if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) { delete s; vp_set_error("cudaMemGetInfo failed"); return VP_E_CUDA; }
         mem_budget = (int64_t)(fr * 0.9);
     }

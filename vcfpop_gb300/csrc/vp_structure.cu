@@ -217,30 +217,41 @@ int sweep_launch(vp_chain* c, const void* fn, const char* name, dim3 g, dim3 b, 
         if (rc_) return rc_;                                                                       \
     } while (0)
 
-// The library's device memory: one stream-ordered pool per device that keeps
-// freed blocks for the next context, chain or batch, so repeated runs do not
-// pay to map and unmap memory (and a free does not wait for the device);
-// vp_release_memory gives the kept blocks back.
-cudaMemPool_t lib_pool(int device) {
+// The library's device memory: stream-ordered pools that keep freed blocks for
+// the next call, so repeated runs do not pay to map and unmap memory (and a free
+// does not wait for the device). Two per device: POOL_RUN for contexts, chains
+// and batches, which keeps every block until vp_release_memory, and POOL_CALL for
+// the buffers of one ingest or filter call, whose text may be as large as all of
+// a run's data: it keeps CALL_KEPT bytes between calls (an 80 MB text and its
+// results stay mapped) and gives the rest back as a call ends.
+enum { POOL_RUN, POOL_CALL, POOLS };
+constexpr uint64_t CALL_KEPT = 256ull << 20;
+cudaMemPool_t lib_pool(int device, int which) {
     static std::mutex mu;
     static std::vector<cudaMemPool_t> pools;
     std::lock_guard<std::mutex> lk(mu);
-    if ((int)pools.size() <= device) pools.resize(device + 1, nullptr);
-    if (!pools[device]) {
+    if ((int)pools.size() <= device * POOLS + which) pools.resize((device + 1) * POOLS, nullptr);
+    cudaMemPool_t& pool = pools[device * POOLS + which];
+    if (!pool) {
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = device;
-        if (cudaMemPoolCreate(&pools[device], &props) != cudaSuccess) return nullptr;
-        uint64_t keep = UINT64_MAX;
-        cudaMemPoolSetAttribute(pools[device], cudaMemPoolAttrReleaseThreshold, &keep);
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) return pool = nullptr;
+        uint64_t keep = which == POOL_RUN ? UINT64_MAX : CALL_KEPT;
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
     }
-    return pools[device];
+    return pool;
 }
 cudaError_t dev_alloc(void** p, size_t bytes, int device, cudaStream_t s) {
-    cudaMemPool_t pool = lib_pool(device);
+    cudaMemPool_t pool = lib_pool(device, POOL_RUN);
     if (!pool) return cudaErrorMemoryAllocation;
-    return cudaMallocFromPoolAsync(p, bytes, pool, s);
+    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+    if (e == cudaErrorMemoryAllocation && vp_pool_trim(device) == cudaSuccess) {
+        cudaGetLastError();
+        e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+    }
+    return e;
 }
 void dev_free(void* p, cudaStream_t s) {
     if (p) cudaFreeAsync(p, s);
@@ -862,7 +873,14 @@ int vp_chain_check(const vp_chain* c) {
     return timed_out(code);
 }
 
-cudaError_t vp_pool_alloc(void** p, size_t bytes, int device, cudaStream_t s) { return dev_alloc(p, bytes, device, s); }
+cudaError_t vp_pool_alloc(void** p, size_t bytes, int device, cudaStream_t s) {
+    cudaMemPool_t pool = lib_pool(device, POOL_CALL);
+    return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaErrorMemoryAllocation;
+}
+cudaError_t vp_pool_trim(int device) {
+    cudaMemPool_t pool = lib_pool(device, POOL_CALL);
+    return pool ? cudaMemPoolTrimTo(pool, 0) : cudaErrorMemoryAllocation;
+}
 
 #ifndef MADV_POPULATE_WRITE
 #define MADV_POPULATE_WRITE 23
@@ -3027,11 +3045,13 @@ extern "C" int vp_release_memory(int device) {
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) { vp_set_error("no CUDA device"); return VP_E_NODEV; }
     if (device < 0 || device >= ndev) { vp_set_error("device %d out of range", device); return VP_E_ARG; }
-    cudaMemPool_t pool = lib_pool(device);
-    if (!pool) { vp_set_error("no memory pool on device %d", device); return VP_E_CUDA; }
     CK(cudaSetDevice(device));
     CK(cudaDeviceSynchronize());
-    CK(cudaMemPoolTrimTo(pool, 0));
+    for (int which = 0; which < POOLS; ++which) {
+        cudaMemPool_t pool = lib_pool(device, which);
+        if (!pool) { vp_set_error("no memory pool on device %d", device); return VP_E_CUDA; }
+        CK(cudaMemPoolTrimTo(pool, 0));
+    }
     return VP_OK;
 }
 
