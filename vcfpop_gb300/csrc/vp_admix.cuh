@@ -448,7 +448,7 @@ __global__ void __launch_bounds__(PZ_MAXT, KM <= 11 ? 3 : 2) k_metro_pk(const De
 // Label draws per copy of the byte layout (any ploidy and allele count), up to
 // 16 clusters, on the same streams and with the same operations a copy as
 // k_update_z_admix_ctr: one lane per individual (in ascending ploidy with mixed
-// ploidy), 256 individuals per CTA. A call is one aligned load; the staged
+// ploidy), 256 individuals per CTA. A call is one to three aligned loads; the staged
 // frequencies of an allele are whole 16-byte chunks, an odd count, so that a
 // copy's weights take a quarter of the loads; the label is the number of
 // thresholds that the uniform reaches, its count goes to the lane's own column
@@ -490,25 +490,31 @@ __global__ void __launch_bounds__(ZG_T, KM <= 8 ? 3 : 2) k_z_admix_gen(const Dev
     const float minf = (float)VP_MIN_FREQ, kmin = (float)(VP_MIN_FREQ * K);
     const uint2 key = make_uint2((uint32_t)c.seed, (uint32_t)(c.seed >> 32));
     const uint32_t ca = ST_ZSLICE | ((uint32_t)m << 4);
-    // a call's bytes: copy a in byte a, 0xFF past the last one (WIDE: 16 bytes)
-    const uint8_t* gp = D.gb + (size_t)i * D.vstr;
-    const size_t row = (size_t)D.N * D.vstr;
+    // a call's bytes: copy a in byte a, 0xFF past the last one, anything from byte
+    // vmax on (WIDE: 16 bytes). Calls of 1, 2, 4 and 8 bytes are one load; others
+    // start anywhere and are put together from the aligned words they touch (the
+    // array is longer than its calls by GB_PAD bytes for the last one's).
+    const bool split = WIDE || (vmax & (vmax - 1));
+    const uint8_t* gp = D.gb + (size_t)i * vmax;
+    const size_t row = (size_t)D.N * vmax;
     auto call = [&](int64_t l, uint64_t& lo, uint64_t& hi) {
         lo = hi = ~0ull;
         if (!live || l >= lb1) return;
         const uint8_t* g = gp + l * row;
-        if constexpr (WIDE) {
-            const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2*>(g));
-            lo = v.x;
-            hi = v.y;
-        } else if (D.vstr == 8) {
+        if (split) {
+            // 3, 5 and 6 bytes are within two words, 7, 9 and 10 within three
+            const uint32_t* w = reinterpret_cast<const uint32_t*>((uintptr_t)g & ~(uintptr_t)3);
+            const uint32_t sh = 8 * ((uint32_t)(uintptr_t)g & 3u), w1 = __ldg(w + 1), w2 = vmax >= 7 ? __ldg(w + 2) : 0u;
+            lo = __funnelshift_r(__ldg(w), w1, sh) | ((uint64_t)__funnelshift_r(w1, w2, sh) << 32);
+            if constexpr (WIDE) hi = w2 >> sh;
+        } else if (vmax == 8) {
             lo = __ldg(reinterpret_cast<const unsigned long long*>(g));
-        } else if (D.vstr == 4) {
-            lo = 0xFFFFFFFF00000000ull | __ldg(reinterpret_cast<const uint32_t*>(g));
-        } else if (D.vstr == 2) {
-            lo = 0xFFFFFFFFFFFF0000ull | __ldg(reinterpret_cast<const uint16_t*>(g));
+        } else if (vmax == 4) {
+            lo = __ldg(reinterpret_cast<const uint32_t*>(g));
+        } else if (vmax == 2) {
+            lo = __ldg(reinterpret_cast<const uint16_t*>(g));
         } else {
-            lo = 0xFFFFFFFFFFFFFF00ull | __ldg(g);
+            lo = __ldg(g);
         }
     };
     // the calls of ZG_G loci are loaded while the ones before are drawn

@@ -233,24 +233,20 @@ extern "C" int vp_dataset_prepare(const vp_input* in, vp_dataset** out) {
         d->maxploidy = 0;
         for (int i = 0; i < N; ++i) if (typed[i]) d->maxploidy = 2;
     } else {
-        // calls of 1, 2, 4, 8 or 16 bytes, so that a call is one aligned load
-        int vstr = 1;
-        while (vstr < vmax) vstr <<= 1;
-        d->vstr = vstr;
-        d->gb.assign((size_t)L * N * vstr, 0xFF);
+        d->gb.assign((size_t)L * N * vmax + GB_PAD, 0xFF);
         parallel_for(L, [&](int64_t l) {
             const int8_t* G = in->alleles + (size_t)d->order[l] * N * vmax;
-            uint8_t* o = &d->gb[(size_t)l * N * vstr];
+            uint8_t* o = &d->gb[(size_t)l * N * vmax];
             for (int i = 0; i < N; ++i) {
                 const int8_t* g = G + (size_t)i * vmax;
                 if (g[0] < 0) continue;
-                for (int c = 0; c < in->ploidy[i]; ++c) o[(size_t)i * vstr + c] = (uint8_t)g[c];
+                for (int c = 0; c < in->ploidy[i]; ++c) o[(size_t)i * vmax + c] = (uint8_t)g[c];
             }
         });
         for (int64_t l = 0; l < L; ++l) {
-            const uint8_t* o = &d->gb[(size_t)l * N * vstr];
+            const uint8_t* o = &d->gb[(size_t)l * N * vmax];
             for (int i = 0; i < N; ++i)
-                if (o[(size_t)i * vstr] != 0xFF) {
+                if (o[(size_t)i * vmax] != 0xFF) {
                     d->vt[i] += in->ploidy[i];
                     d->maxploidy = std::max(d->maxploidy, in->ploidy[i]);
                 }

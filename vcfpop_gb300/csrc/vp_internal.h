@@ -29,13 +29,16 @@ struct HostBuf {
     const T& operator[](size_t i) const { return p[i]; }
 };
 
+// bytes behind the last call of the byte layout: words that hold its end may be read whole
+constexpr int GB_PAD = 16;
+
 struct vp_dataset {
     std::atomic<int> refs{1};      // the caller's handle plus each server request holding it
-    int32_t N = 0, S = 0, vmax = 0, vstr = 0, maxploidy = 0, maxK = 0, Nw = 0;
+    int32_t N = 0, S = 0, vmax = 0, maxploidy = 0, maxK = 0, Nw = 0;
     int64_t L = 0, KT = 0, coprime = 1;
     bool packed2 = false;
     HostBuf<uint32_t> g2;          // packed2: [L][Nw] 2-bit codes, sorted locus order; Nw a multiple of 4
-    std::vector<uint8_t> gb;       // general: [L][N][vstr] allele per copy, 0xFF none; vstr: vmax up to a power of two
+    std::vector<uint8_t> gb;       // general: [L][N][vmax] allele per copy, 0xFF none, then GB_PAD bytes
     std::vector<int32_t> k;        // [L] alleles
     std::vector<int64_t> off;      // [L] allele offsets
     std::vector<int64_t> vt;       // [N] typed copies per individual

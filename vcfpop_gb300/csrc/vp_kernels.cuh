@@ -16,11 +16,11 @@ constexpr int SUB = 32;         // loci per FP32 sub-sum before folding into FP6
 constexpr double LL_UNIT = 1.0 / 536870912.0;  // the tensor-core likelihood's unit, 2^-29
 
 struct DevData {
-    int32_t N, S, vmax, vstr, maxploidy, maxK, Nw, packed2;
+    int32_t N, S, vmax, maxploidy, maxK, Nw, packed2;
     int32_t popcontig;    // every population's individuals are consecutive
     int64_t L, KT, coprime;
     const uint32_t* g2;   // [L][Nw]
-    const uint8_t* gb;    // [L][N][vstr], vstr a power of two
+    const uint8_t* gb;    // [L][N][vmax]
     const int32_t* k;
     const int64_t* off;
     const int64_t* vt;
@@ -223,7 +223,7 @@ __device__ __forceinline__ void load_copies(const DevData& D, int64_t l, int i, 
         cp.a[1] = code == 0 ? 0 : 1;
         return;
     }
-    const uint8_t* g = D.gb + ((size_t)l * D.N + i) * D.vstr;
+    const uint8_t* g = D.gb + ((size_t)l * D.N + i) * D.vmax;
     int n = 0;
     if (g[0] != 0xFF)
         for (; n < D.vmax && g[n] != 0xFF; ++n) cp.a[n] = g[n];

@@ -476,7 +476,7 @@ int launch_zadm_ctr(vp_chain* c, int force) {
     prof_mark(x, true);
     struct End { vp_ctx* x; ~End() { prof_mark(x, false); } } end_{x};
     const int K = c->P.K;
-    if (K <= PZ_MAXK && x->D.vstr == 16) {
+    if (K <= PZ_MAXK && x->D.vmax > 8) {
         SL(c, (k_z_admix_gen<PZ_MAXK, false, true>), (g), (ZG_T), zgen_smem(c, PZ_MAXK), 1, force);
         return VP_OK;
     }
@@ -919,7 +919,7 @@ int vp_open_ex(const vp_dataset* ds, int device, int priority, vp_ctx** out) {
     x->N = ds->N; x->S = ds->S; x->L = ds->L; x->KT = ds->KT; x->maxK = ds->maxK; x->maxploidy = ds->maxploidy;
     x->packed2 = ds->packed2;
     DevData& D = x->D;
-    D.N = ds->N; D.S = ds->S; D.vmax = ds->vmax; D.vstr = ds->vstr; D.maxploidy = ds->maxploidy; D.maxK = ds->maxK; D.Nw = ds->Nw;
+    D.N = ds->N; D.S = ds->S; D.vmax = ds->vmax; D.maxploidy = ds->maxploidy; D.maxK = ds->maxK; D.Nw = ds->Nw;
     D.packed2 = ds->packed2; D.L = ds->L; D.KT = ds->KT; D.coprime = ds->coprime;
     D.popcontig = 1;
     for (int32_t sp = 0; sp < ds->S; ++sp)
