@@ -448,13 +448,14 @@ __global__ void __launch_bounds__(PZ_MAXT, KM <= 11 ? 3 : 2) k_metro_pk(const De
 // Label draws per copy of the byte layout (any ploidy and allele count), up to
 // 16 clusters, on the same streams and with the same operations a copy as
 // k_update_z_admix_ctr: one lane per individual (in ascending ploidy with mixed
-// ploidy), 256 individuals per CTA. A call is one to three aligned loads; the staged
+// ploidy), 256 individuals per CTA. A call is two or three aligned loads; the staged
 // frequencies of an allele are whole 16-byte chunks, an odd count, so that a
 // copy's weights take a quarter of the loads; the label is the number of
 // thresholds that the uniform reaches, its count goes to the lane's own column
 // of a shared array and to the slice's shared histogram. The Philox block is
 // formed when the warp's draw index enters it (mixed ploidy skips some).
-// N = 1,500 x L = 8,000, ploidy 2, 4 and 6, 2-8 alleles, K = 8: 295 -> 254 us.
+// N = 1,500 x L = 8,000, ploidy 2, 4 and 6, 2-8 alleles, K = 8: 295 -> 278 us
+// (256 with calls padded to 8 bytes, a third more device memory).
 // Issue-bound (64% active, about 140 instructions a warp and copy); loading the
 // calls four loci ahead or taking 16 to 64 CTAs per SM made no difference.
 constexpr int ZG_T = 256, ZG_G = 4;
@@ -491,31 +492,20 @@ __global__ void __launch_bounds__(ZG_T, KM <= 8 ? 3 : 2) k_z_admix_gen(const Dev
     const uint2 key = make_uint2((uint32_t)c.seed, (uint32_t)(c.seed >> 32));
     const uint32_t ca = ST_ZSLICE | ((uint32_t)m << 4);
     // a call's bytes: copy a in byte a, 0xFF past the last one, anything from byte
-    // vmax on (WIDE: 16 bytes). Calls of 1, 2, 4 and 8 bytes are one load; others
-    // start anywhere and are put together from the aligned words they touch (the
+    // vmax on (WIDE: 16 bytes). Calls start anywhere: a call is put together from
+    // the aligned words that hold it, two up to 6 bytes and at 8, else three (the
     // array is longer than its calls by GB_PAD bytes for the last one's).
-    const bool split = WIDE || (vmax & (vmax - 1));
     const uint8_t* gp = D.gb + (size_t)i * vmax;
     const size_t row = (size_t)D.N * vmax;
+    const bool third = WIDE || vmax == 7;
     auto call = [&](int64_t l, uint64_t& lo, uint64_t& hi) {
         lo = hi = ~0ull;
         if (!live || l >= lb1) return;
-        const uint8_t* g = gp + l * row;
-        if (split) {
-            // 3, 5 and 6 bytes are within two words, 7, 9 and 10 within three
-            const uint32_t* w = reinterpret_cast<const uint32_t*>((uintptr_t)g & ~(uintptr_t)3);
-            const uint32_t sh = 8 * ((uint32_t)(uintptr_t)g & 3u), w1 = __ldg(w + 1), w2 = vmax >= 7 ? __ldg(w + 2) : 0u;
-            lo = __funnelshift_r(__ldg(w), w1, sh) | ((uint64_t)__funnelshift_r(w1, w2, sh) << 32);
-            if constexpr (WIDE) hi = w2 >> sh;
-        } else if (vmax == 8) {
-            lo = __ldg(reinterpret_cast<const unsigned long long*>(g));
-        } else if (vmax == 4) {
-            lo = __ldg(reinterpret_cast<const uint32_t*>(g));
-        } else if (vmax == 2) {
-            lo = __ldg(reinterpret_cast<const uint16_t*>(g));
-        } else {
-            lo = __ldg(g);
-        }
+        const uintptr_t g = (uintptr_t)(gp + l * row);
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(g & ~(uintptr_t)3);
+        const uint32_t sh = 8 * (uint32_t)g, w1 = __ldg(w + 1), w2 = third ? __ldg(w + 2) : 0u;   // shifts by sh mod 32
+        lo = __funnelshift_r(__ldg(w), w1, sh) | ((uint64_t)__funnelshift_r(w1, w2, sh) << 32);
+        if constexpr (WIDE) hi = w2 >> (sh & 31);
     };
     // the calls of ZG_G loci are loaded while the ones before are drawn
     uint64_t nlo[ZG_G], nhi[ZG_G];
