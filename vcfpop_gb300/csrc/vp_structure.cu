@@ -134,8 +134,8 @@ struct TcBatch {
     double* lnlrec = nullptr;       // [chain][block] sums of a recorded sweep's lnP(D)
     int32_t *rowchain = nullptr, *rowk = nullptr, *row0 = nullptr;
     // cluster rows padded to whole 192-row column groups of the count
-    // contraction (BN cluster rows per CTA, piece per MMA)
-    int R = 0, Rpad = 0, G = 0, BN = 192, piece = 192, splits = 1;
+    // contraction
+    int R = 0, Rpad = 0, splits = 1;
     // the count contraction's 128-row A tiles per CTA: two, or one where two
     // would leave SMs without a CTA (20,011 loci, 60
     // rows: 79 CTAs took 17.7 us, 157 take 13.8)
@@ -1706,7 +1706,7 @@ int cohort_build(vp_cohort* h) {
     for (int i = 0; i < n; ++i) hc[i] = h->chains[i]->h;
     DevChain* dchains = (DevChain*)h->mem;
     int4* dmaps = (int4*)((char*)h->mem + hb);
-    // (from pageable memory: the copies are staged before the calls return)
+    // (from pageable memory: each call returns once the source has been read)
     CK(cudaMemcpyAsync(dchains, hc.data(), (size_t)n * sizeof(DevChain), cudaMemcpyHostToDevice, h->stream));
     CK(cudaMemcpyAsync(dmaps, maps.data(), maps.size() * sizeof(int4), cudaMemcpyHostToDevice, h->stream));
     // 4. capture one sweep
@@ -2239,8 +2239,7 @@ int make_batch(vp_ctx* x, vp_chain** cs, int n, const TcChoice* force) {
     }
     b->nsgrp = (int)sgrp.size();
     for (const int4& gr : sgrp) b->sgrp_rows = std::max(b->sgrp_rows, gr.w);
-    b->G = (b->R + b->BN - 1) / b->BN;
-    b->Rpad = b->G * b->BN;
+    b->Rpad = (b->R + 191) / 192 * 192;
     const TcOperands& t = x->tc;
     b->cfg = force ? *force : tuned_choice(x, b->R);
     if (choice_error(x, b->Rpad, b->cfg)) {
@@ -2368,8 +2367,6 @@ unsigned updatep_blocks(const vp_ctx* x, int64_t nloci, int R) {
     }
     return upx;
 }
-
-// branch streams and events for a sweep's fork and join
 
 // dynamic shared memory of an UpdateP block that lets at most `share` of
 // them sit on an SM beside one CTA of the likelihood contraction (the
@@ -2514,7 +2511,8 @@ int set_node_priorities(vp_ctx* x, cudaGraph_t g, const void* hi_fn) {
 }
 
 // the count contraction of the batch: Ni[row, a] = sum_i OH[row, i] C[i, a]
-// into every chain's Ni (e4m3 operands, exact), or into `out` ([Rpad][KT])
+// into every chain's Ni (e5m2 operands, e4m3 past the packed form's range; exact),
+// or into `out` ([Rpad][KT])
 int launch_counts_gemm(vp_ctx* x, int32_t* out) {
     TcBatch* b = x->batch;
     const TcOperands& t = x->tc;

@@ -572,8 +572,6 @@ __global__ void __launch_bounds__(256) k_update_p_tc(BatchDev b, int64_t l0, int
     }
 }
 
-// one-hot rows of every chain's current labels (the initial counts of a
-// batch: the count contraction of these rows is the no-admixture UpdateZ)
 // adds the individuals of each cluster among the warp's labels z (-1: none) to nk
 __device__ __forceinline__ void add_sizes(int32_t* nk, int K, int z) {
     const int lane = threadIdx.x & 31;
@@ -586,6 +584,8 @@ __device__ __forceinline__ void add_sizes(int32_t* nk, int K, int z) {
         if (mine) atomicAdd(nk + k0 + lane, mine);
     }
 }
+// one-hot rows of every chain's current labels (the initial counts of a
+// batch: the count contraction of these rows is the no-admixture UpdateZ)
 __global__ void k_onehot_from_z(BatchDev b) {
     const int ci = blockIdx.y;
     const DevChain& c = b.chains[ci];
