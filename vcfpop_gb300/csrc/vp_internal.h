@@ -71,7 +71,7 @@ void vp_dataset_retain(const vp_dataset* ds);
 int vp_finish_issue(vp_chain** cs, int32_t n);
 // after the work queued on the chain's stream: VP_E_CUDA where a kernel's wait
 // ran out and left the chain's state void
-int vp_chain_check(const vp_chain* c);
+int vp_chain_check(vp_chain* c);
 // sweeps issued so far and in total for one chain
 void vp_chain_progress(const vp_chain* c, int64_t* issued, int64_t* total);
 // the dataset a chain's context holds, and the chain's parameters

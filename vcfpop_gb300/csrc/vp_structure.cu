@@ -110,6 +110,10 @@ struct vp_chain {
     void* plain_mem = nullptr;
     // the cohort whose shared launches sweep this chain (vp_cohort_set)
     struct vp_cohort* cohort = nullptr;
+    // k_loglik_tc or k_count_tc is among the chain's launches, whose waits may
+    // run out and leave an error in the control block instead of a result; and
+    // work was queued since the last look at it (vp_chain_check)
+    bool may_time_out = false, unchecked = false;
 };
 
 // launch configuration of a batch's two contractions: the likelihood
@@ -399,6 +403,7 @@ int launch_loglik(vp_chain* c, int force) {
     prof_mark(x, true);
     struct End { vp_ctx* x; ~End() { prof_mark(x, false); } } end_{x};
     if (c->h.llnb && !force) {
+        c->may_time_out = c->unchecked = true;
         const dim3 g(cdiv(x->N, ptc::LL_M), c->h.tcchunk, 1);
         switch (c->h.llnb) {
             case 32: SL(c, ptc::k_loglik_tc<32>, (g), (ptc::LL_THREADS), 0, 0); break;
@@ -566,10 +571,6 @@ bool count_tc_form(const vp_ctx* x, int K) {
     return x->packed2 && K <= 32 && (x->N < 512 ? calls >= 1 << 21 : x->N <= 1024 || calls >= 1 << 22);
 }
 
-// Chains whose plain form may end a launch with an error in their control block
-// instead of a result (a wait of k_loglik_tc or k_count_tc that ran out): state
-// is handed out, and steps and runs end, only after a look at it.
-bool may_time_out(const vp_chain* c) { return c->h.llnb || (!c->P.admix && count_tc_form(c->ctx, c->P.K)); }
 int timed_out(int code) {
     if (!code) return VP_OK;
     vp_set_error("a tensor-core kernel of this chain timed out (code %d): its results are void", code);
@@ -582,6 +583,7 @@ int launch_count(vp_chain* c, int force) {
     vp_ctx* x = c->ctx;
     const int K = c->P.K;
     if (count_tc_form(x, K)) {
+        c->may_time_out = c->unchecked = true;
         SL(c, ptc::k_onehot, (cdiv(x->N, ptc::CT_IND), 1, 1), (ptc::CT_IND), 0, 1, force);
         const dim3 g(cdiv(x->L, ptc::CT_M), 1, 1);
         if (ptc::ct_rows(K) == 16) SL(c, ptc::k_count_tc<16>, (g), (ptc::CT_THREADS), 0, 1, force);
@@ -865,11 +867,14 @@ int ensure_plain(vp_chain* c) {
     return VP_OK;
 }
 
-int vp_chain_check(const vp_chain* c) {
-    if (!may_time_out(c)) return VP_OK;
+// State is handed out, and steps and runs end, only after a look at the error of
+// the work before: one copy of four bytes for any number of reads after it.
+int vp_chain_check(vp_chain* c) {
+    if (!c->may_time_out || !c->unchecked) return VP_OK;
     int code = 0;
     CK(cudaMemcpyAsync(&code, &c->h.ctl->err, sizeof code, cudaMemcpyDeviceToHost, c->ctx->stream));
     CK(cudaStreamSynchronize(c->ctx->stream));
+    c->unchecked = code != 0;
     return timed_out(code);
 }
 
@@ -1272,6 +1277,7 @@ static int run_plain(vp_ctx* x, vp_chain** cs, int n, int nsweeps) {
             if (rc) return rc;
             x->pg_chains = act;
         }
+        for (vp_chain* c : act) c->unchecked = true;
         for (int s = 0; s < step; ++s) {
             CK(cudaGraphLaunch(x->pg, x->stream));
             x->launches += x->pg_nodes;
@@ -1813,6 +1819,7 @@ extern "C" int vp_cohort_run(vp_cohort* h, int32_t nsweeps) {
     if (!h || nsweeps < 0) { vp_set_error("bad arguments"); return VP_E_ARG; }
     if (h->chains.empty() || nsweeps == 0) return VP_OK;
     cudaSetDevice(h->device);
+    for (vp_chain* c : h->chains) c->unchecked = true;
     for (int s = 0; s < nsweeps; ++s) CK(cudaGraphLaunch(h->graph, h->stream));
     h->launches += (int64_t)h->nodes * nsweeps;
     // members' own streams (results, Arrange, later single steps) follow
@@ -1830,7 +1837,7 @@ extern "C" int vp_cohort_sync(vp_cohort* h) {
     cudaSetDevice(h->device);
     CK(cudaStreamSynchronize(h->stream));
     cohort_reap(h, true);
-    for (const vp_chain* c : h->chains)
+    for (vp_chain* c : h->chains)
         if (int rc = vp_chain_check(c)) return rc;
     return VP_OK;
 }
