@@ -128,8 +128,8 @@ __host__ __device__ constexpr int pz_chunks() { return ((KM + 1) / 2) | 1; }
 //
 // Measured, us a launch against k_update_z_admix_ctr on the same calls: N = 2,000 x
 // L = 50,000, K = 5 1,030 -> 375; N = 4,999 x L = 40,009, K = 11 3,700 -> 1,160;
-// N = 300 x L = 3,000, K = 4 32 -> 17. At K = 5 issue is 75% active, the ALU
-// pipe 61%, the multiplier pipe (Philox) 64%. Round keys read from shared
+// N = 300 x L = 3,000, K = 4 32 -> 17. At K = 5 issue is 76% active, the ALU
+// pipe 62%, the multiplier pipe (Philox) 55%. Round keys read from shared
 // memory instead of added up gave 1.7%, 2 or 4 CTAs per SM instead of 3 lost 1%.
 constexpr int PZ_MAXK = 16;
 constexpr int PZ_MAXT = 256;
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(PZ_MAXT, KM <= 11 ? 3 : 2) k_metro_pk(const De
 // formed when the warp's draw index enters it (mixed ploidy skips some).
 // N = 1,500 x L = 8,000, ploidy 2, 4 and 6, 2-8 alleles, K = 8: 295 -> 278 us
 // (256 with calls padded to 8 bytes, a third more device memory).
-// Issue-bound (64% active, about 140 instructions a warp and copy); loading the
+// Issue-bound (59% active, 131 instructions a warp's copy); loading the
 // calls four loci ahead or taking 16 to 64 CTAs per SM made no difference.
 constexpr int ZG_T = 256, ZG_G = 4;
 static_assert(ZA_LC % ZG_G == 0, "whole groups a slice");

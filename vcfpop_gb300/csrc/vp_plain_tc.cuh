@@ -153,9 +153,9 @@ __device__ __forceinline__ void calls_to_e4m3(uint32_t w, uint32_t* r) {
 // instructions of a stage (copies, shuffles, byte permutes, waits, a store) set
 // the pace: halving the MMAs or the ring changed nothing, so two teams of
 // builders take alternate stages and a wait's first poll is all that is inlined.
-// N = 10,000 x L = 60,000, K = 10: 141 us (667 for the FP32 stream; 271 with f16
+// N = 10,000 x L = 60,000, K = 10: 149 us (680 for the FP32 stream; 271 with f16
 // digits and a team, 232 with one-byte digits, 180 with the words copied
-// ahead); ALU pipe 60%, issue 66%, DRAM 0.9 TB/s. Lane n of a
+// ahead, in shorter runs); ALU pipe 60%, issue 66%, tensor pipe 29%, DRAM 1.1 TB/s. Lane n of a
 // builder warp is individual n / 2 of the warp's first genotype word or of its
 // second, by n's last bit (the in-register transpose's order).
 template <int NB>
@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(LL_THREADS, NB <= 80 ? 2 : 1) k_loglik_tc(cons
 // kernel's pace: 172 us against 125), with the clusters' sizes: copies of
 // allele 0 are 2 (size - missing) - copies of allele 1.
 // Bound, as the likelihood, by the builders' and waits' dependent instructions.
-// N = 10,000 x L = 60,000, K = 10: 84 us against 307 for the bit-plane kernel's
+// N = 10,000 x L = 60,000, K = 10: 93 us against 307 for the bit-plane kernel's
 // population counts (125 with one team of builders and longer waits).
 constexpr int CT_IND = 128, CT_M = 128, CT_BW = 8;   // two teams of four builder warps take alternate stages
 constexpr int CT_THREADS = (CT_BW + 3) * 32;         // the builders, MMA, B producer, cluster sizes
