@@ -42,6 +42,7 @@ struct Ctl {
     double fprop;         // UpdateF's proposal for the next cluster
     int32_t err;          // a tensor-core kernel's wait ran out (0: none)
     int32_t drawn;        // the label draw recorded this sweep and advanced m; its counts follow
+    int32_t infinite;     // 1 + the last sweep with an infinite frequency, where the chain has digits
 };
 
 struct DevChain {
@@ -423,7 +424,18 @@ __device__ __forceinline__ void write_lt(const DevChain& c, int k, int64_t l, co
 // form, but on sweeps that Record reads: their lnP(D) keeps the FP32 stream, so
 // that what a run reports does not change with the form (the two differ by a
 // few 1e-9, the FP32 stream's own rounding); label draws do not tell.
-__device__ __forceinline__ bool ll_tc_at(const DevChain& c, int m) { return c.llnb && binaryq_at(c, m) && !record_at(c, m); }
+// An infinite frequency (the quotient of two gamma draws below the normal
+// numbers: clusters without a copy at a locus, lambda below about 0.05) has no
+// digits, and in the FP32 stream it reaches only the individuals that read it:
+// such a sweep keeps that stream too, its table filled by the kernel that
+// would have run.
+__device__ __forceinline__ bool ll_tc_turn(const DevChain& c, int m) { return c.llnb && binaryq_at(c, m) && !record_at(c, m); }
+__device__ __forceinline__ bool ll_tc_at(const DevChain& c, int m) { return ll_tc_turn(c, m) && c.ctl->infinite != m + 1; }
+// digits of locus l's frequencies p in cluster k, at sweep m
+__device__ __forceinline__ void set_digits(const DevChain& c, int k, int64_t l, const float* p, int m) {
+    write_digits(c, k, l, p);
+    if (fmaxf(p[0], p[1]) > 3.402823466e38f) c.ctl->infinite = m + 1;
+}
 
 // rebuild the lookup table from Freq (after a host-side state import)
 __global__ void k_refresh_lt(const DevChain* chains) {
@@ -435,7 +447,7 @@ __global__ void k_refresh_lt(const DevChain* chains) {
     int64_t l = kl % D.L;
     const float* p = c.Freq + k * D.KT + D.off[l];
     write_lt(c, k, l, p, D.k[l]);
-    if (c.llnb) write_digits(c, k, l, p);
+    if (c.llnb) set_digits(c, k, l, p, c.ctl->m);
 }
 
 // UpdateP. With `mean` (a sweep; a single step leaves that to Record) the new
@@ -510,7 +522,7 @@ __global__ void k_update_p_ctr(const DevChain* chains, int mean, const int4* map
     for (int a = 0; a < k2; ++a) c.Freq[j + a] = p[a];
     if (mean && mean_at(c, m))
         for (int a = 0; a < k2; ++a) c.FreqM[j + a] += p[a];
-    if (ll_tc_at(c, m)) write_digits(c, k, l, p);
+    if (ll_tc_turn(c, m)) set_digits(c, k, l, p, m);
     else write_lt(c, k, l, p, k2);
 }
 

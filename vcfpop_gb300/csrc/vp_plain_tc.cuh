@@ -149,6 +149,16 @@ __device__ __forceinline__ void calls_to_e4m3(uint32_t w, uint32_t* r) {
     }
 }
 
+// the FP32 stream's table from the frequencies, by thread t of nt
+__device__ __noinline__ void fill_lt(const DevChain& c, int64_t t, int64_t nt) {
+    const int64_t L = c.D.L;
+    for (; t < (int64_t)c.K * L; t += nt) {
+        const int k = (int)(t / L);
+        const int64_t l = t - k * L;
+        write_lt(c, k, l, c.Freq + (int64_t)k * c.D.KT + 2 * l, 2);
+    }
+}
+
 // CTA: LL_M individuals x the stages of its chunk (grid.y). The dependent
 // instructions of a stage (copies, shuffles, byte permutes, waits, a store) set
 // the pace: halving the MMAs or the ring changed nothing, so two teams of
@@ -171,7 +181,12 @@ __global__ void __launch_bounds__(LL_THREADS, NB <= 80 ? 2 : 1) k_loglik_tc(cons
     const VBlock vb = vblock(map);
     const DevChain& c = chains[vb.z];
     if (map && run_over(c)) return;
-    if (!ll_tc_at(c, c.ctl->m)) return;
+    const int m = c.ctl->m;
+    if (!ll_tc_at(c, m)) {
+        if (ll_tc_turn(c, m))
+            fill_lt(c, ((int64_t)vb.y * vb.gx + vb.x) * LL_THREADS + threadIdx.x, (int64_t)vb.gx * c.tcchunk * LL_THREADS);
+        return;
+    }
     const DevData& D = c.D;
     const int K = c.K;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

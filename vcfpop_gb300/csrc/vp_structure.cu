@@ -629,12 +629,13 @@ bool draw_records(const vp_chain* c) {
 // UpdateP writes the one likelihood table that its own sweep reads (ll_tc_at).
 // A single step may come at another sweep index, or after a batch's sweeps,
 // which write neither: it fills the tables from the frequencies first.
-int refresh_tables(vp_chain* c) {
+int fill_tables(vp_chain* c) {
     vp_ctx* x = c->ctx;
-    if (!c->h.llnb && !c->plain_lazy) return VP_OK;
+    CK(cudaMemsetAsync(&c->h.ctl->infinite, 0, sizeof c->h.ctl->infinite, x->stream));
     LAUNCH(x, k_refresh_lt, (cdiv((int64_t)c->P.K * x->L, 256), 256, 0, x->stream), (c->d));
     return VP_OK;
 }
+int refresh_tables(vp_chain* c) { return c->h.llnb || c->plain_lazy ? fill_tables(c) : VP_OK; }
 
 int launch_step(vp_chain* c, int step, int force, bool sweep = false) {
     vp_ctx* x = c->ctx;
@@ -863,8 +864,7 @@ int ensure_plain(vp_chain* c) {
     h.ltd = (char*)c->plain_mem + lt_bytes;
     h.LLp = (double*)((char*)c->plain_mem + lt_bytes + ltd_bytes);
     LAUNCH(x, k_set_plain, (1, 1, 0, x->stream), (c->d, h.lt, h.ltd, h.LLp));
-    LAUNCH(x, k_refresh_lt, (cdiv((int64_t)c->P.K * x->L, 256), 256, 0, x->stream), (c->d));
-    return VP_OK;
+    return fill_tables(c);
 }
 
 // State is handed out, and steps and runs end, only after a look at the error of
@@ -1563,11 +1563,8 @@ extern "C" int vp_chain_set(vp_chain* c, int32_t field, const void* host, size_t
     CK(cudaMemcpy(p, host, n, cudaMemcpyHostToDevice));
     if (field == VP_F_FREQ && c->h.lt) {
         // keep the likelihood tables in step with the frequencies
-        vp_ctx* x = c->ctx;
-        k_refresh_lt<<<cdiv((int64_t)c->P.K * x->L, 256), 256, 0, x->stream>>>(c->d);
-        rc = check_launch(x, "k_refresh_lt");
-        if (rc) return rc;
-        CK(cudaStreamSynchronize(x->stream));
+        if ((rc = fill_tables(c))) return rc;
+        CK(cudaStreamSynchronize(c->ctx->stream));
     }
     return VP_OK;
 }
